@@ -14,6 +14,7 @@
 // row stores is one coalesced 512-byte (patches) segment.  Per-source constants
 // (frames, the REAL*4-rounded DC3D inputs, the Nikkhoo-Walter records) are built
 // once on the host and read through the read-only path.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include "ucg_internal.cuh"
@@ -184,24 +185,149 @@ __global__ void __launch_bounds__(128) k_assemble_rect(double *__restrict__ K, l
 }
 
 // ---- triangles (Nikkhoo & Walter 2015) -----------------------------------------
+//
+// Two kernels per batch of receivers.  k_tri_edges forms the free-surface term
+// of every mesh edge for unit slip along east, north and up (9 or 18 values per
+// receiver) into a scratch small enough to stay in L2; k_assemble_tri adds, for
+// every triangle, its main and image dislocations and its three edges times its
+// slip directions, and writes K once.  A mesh of N triangles has about 1.5 N
+// edges against 3 N sides.
+//
+// Bound by the FP64 pipe: 74 % active in k_tri_edges (254 registers, 8 warps an
+// SM), 58 % in k_assemble_tri (164 registers, 12 warps; the rest waits on record
+// loads and the scratch).  FP64 instructions per pair: 970 for the triangle's own
+// dislocations and 1,150 per edge, against 12,050 for the free-surface term of a
+// pair on single-direction duals, one side at a time.  N = 5,000: 68 -> 8.5 ms,
+// N = 20,000: 893 -> 132 ms (3 % of it the HBM writes of K).  Triangles in one
+// pass instead of three also drops the two re-reads of K.
 
-template <int PART>
-__global__ void __launch_bounds__(128) k_assemble_tri(double *__restrict__ K, long n, long col0,
-        const double *__restrict__ rcv, int nrcv, int np, const double *__restrict__ rec, int ns,
-        NwConst cst)
+// position and unit vectors of a receiver, NED -> ENU
+__device__ __forceinline__ void enu_receiver(const double *rc, double X[3], double vs[3], double vd[3], double vn[3])
+{
+    const double *v[4] = {rc + RC_X, rc + RC_S, rc + RC_D, rc + RC_N};
+    double *o[4] = {X, vs, vd, vn};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        o[k][0] = __ldg(v[k] + 1);
+        o[k][1] = __ldg(v[k]);
+        o[k][2] = -__ldg(v[k] + 2);
+    }
+}
+
+__device__ __forceinline__ void load_edge(const TriTables &t, int j, double e[NE_SIZE])
+{
+#pragma unroll
+    for (int f = 0; f < NE_SIZE; f++) e[f] = __ldg(t.ed + (long)f * t.ne + j);
+}
+
+template <int NR>
+__global__ void __launch_bounds__(128) k_tri_edges(double *__restrict__ sc, const double *__restrict__ rcv, int r0,
+        int r1, TriTables tab, NwConst cst)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= tab.ne) return;
+    double ed[NE_SIZE];
+    load_edge(tab, j, ed);
+    for (int e = r0 + blockIdx.y; e < r1; e += gridDim.y) {
+        double X[3], vs[3], vd[3], vn[3], o[NR][3];
+        enu_receiver(rcv + (long)e * RC_SIZE, X, vs, vd, vn);
+        nw_edge_rows<NR>(X, vs, vd, vn, ed, cst, o);
+        double *p = sc + (long)(e - r0) * (3 * NR) * tab.ne + j;
+#pragma unroll
+        for (int q = 0; q < NR; q++)
+#pragma unroll
+            for (int x = 0; x < 3; x++) p[(long)(3 * q + x) * tab.ne] = o[q][x];
+    }
+}
+
+// slip of the strike and dip modes (ENU): the strike axis and minus the dip
+// axis of the TD frame (nikkhoo15.f90:140)
+__device__ __forceinline__ void tri_slip(const NwRec &R, double bS[3], double bD[3])
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        bS[k] = R[NW_MAIN + TD_S + k];
+        bD[k] = -R[NW_MAIN + TD_D + k];
+    }
+}
+
+// main and image dislocation of triangle j (R), summed into oS, oD
+template <int NR>
+__device__ __forceinline__ void tri_rows(const double X[3], const double vs[3], const double vd[3],
+                                         const double vn[3], const NwRec &R, const NwConst &cst, double oS[NR],
+                                         double oD[NR])
+{
+#pragma unroll
+    for (int q = 0; q < NR; q++) oS[q] = oD[q] = 0.0;
+#pragma unroll 1
+    for (int part = 0; part < 2; part++) {
+        const bool flip = part && R[NW_SURF] != 0.0;
+        if (!nw_td_rows<NR>(X, vs, vd, vn, R, part ? NW_IMG : NW_MAIN, flip, cst, oS, oD)) {
+#pragma unroll
+            for (int q = 0; q < NR; q++) oS[q] = oD[q] = nan("");
+        }
+    }
+}
+
+template <int NR>
+__global__ void __launch_bounds__(128) k_assemble_tri(double *__restrict__ K, long n, long col0, long row0,
+        const double *__restrict__ sc, const double *__restrict__ rcv, int r0, int r1, TriTables tab, NwConst cst)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= tab.ns) return;
+    const NwRec R{tab.rec + j, (long)tab.ns};
+    for (int e = r0 + blockIdx.y; e < r1; e += gridDim.y) {
+        double X[3], vs[3], vd[3], vn[3], oS[NR], oD[NR], bS[3], bD[3];
+        enu_receiver(rcv + (long)e * RC_SIZE, X, vs, vd, vn);
+        tri_rows<NR>(X, vs, vd, vn, R, cst, oS, oD);
+        tri_slip(R, bS, bD);
+#pragma unroll
+        for (int side = 0; side < 3; side++) {
+            const int id = __ldg(tab.edge + (long)side * tab.ns + j);
+            const double sg = (id & 1) ? -1.0 : 1.0;
+            const double *p = sc + (long)(e - r0) * (3 * NR) * tab.ne + (id >> 1);
+#pragma unroll
+            for (int q = 0; q < NR; q++) {
+                const double a = p[(long)(3 * q) * tab.ne], b = p[(long)(3 * q + 1) * tab.ne],
+                             c = p[(long)(3 * q + 2) * tab.ne];
+                oS[q] += sg * (a * bS[0] + b * bS[1] + c * bS[2]);
+                oD[q] += sg * (a * bD[0] + b * bD[1] + c * bD[2]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < NR; q++)
+            *reinterpret_cast<double2 *>(K + (row0 + (long)NR * (e - r0) + q) * n + col0 + 2L * j) =
+                make_double2(oS[q], oD[q]);
+    }
+}
+
+// source records from the vertices (north, east, down): one thread per triangle
+// and per edge
+__global__ void k_tri_prepare(const double *__restrict__ vert, const int *__restrict__ id, int ns,
+                              double *__restrict__ rec)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= ns) return;
-    NwRec R{rec + j, (long)ns};
-    for (int e = blockIdx.y; e < nrcv; e += gridDim.y) {
-        const double *rc = rcv + (long)e * RC_SIZE;
-        double rloc[RC_SIZE];
-#pragma unroll
-        for (int f = 0; f < RC_SIZE; f++) rloc[f] = __ldg(rc + f);
-        double sS[6], sD[6];
-        nw_part_stress<PART>(rloc, R, cst, sS, sD);
-        store_patch_source<PART != 0>(K, n, col0 + 2L * j, rloc, rcv_info(e, np), sS, sD);
+    double P[3][3], r[NW_SIZE];
+    for (int k = 0; k < 3; k++) {
+        // NED -> ENU (nikkhoo15.f90:143-146)
+        const double *v = vert + 3L * id[(long)k * ns + j];
+        P[k][0] = v[1]; P[k][1] = v[0]; P[k][2] = -v[2];
     }
+    nw_prepare(P[0], P[1], P[2], r);
+    for (int f = 0; f < NW_SIZE; f++) rec[(long)f * ns + j] = r[f];
+}
+
+__global__ void k_edge_prepare(const double *__restrict__ vert, const int2 *__restrict__ ends, int ne,
+                               double *__restrict__ ed)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= ne) return;
+    const double *a = vert + 3L * ends[j].x, *b = vert + 3L * ends[j].y;
+    const double PA[3] = {a[1], a[0], -a[2]}, PB[3] = {b[1], b[0], -b[2]};
+    double r[NE_SIZE];
+    nw_prepare_edge(PA, PB, r);
+    for (int f = 0; f < NE_SIZE; f++) ed[(long)f * ne + j] = r[f];
 }
 
 // ---- strain volumes (Barbot, Moore & Lambert 2017) -------------------------------
@@ -281,34 +407,35 @@ __global__ void __launch_bounds__(128) k_block_rect(double *__restrict__ out, co
     }
 }
 
-template <int PART>
 __global__ void __launch_bounds__(128) k_block_tri(double *__restrict__ out, const int *__restrict__ ridx, int nrb,
-        const int *__restrict__ sidx, int nsb, const double *__restrict__ rcv, const double *__restrict__ rec,
-        int ns, NwConst cst)
+        const int *__restrict__ sidx, int nsb, const double *__restrict__ rcv, TriTables tab, NwConst cst)
 {
     const int jj = blockIdx.x * blockDim.x + threadIdx.x;
     if (jj >= nsb) return;
-    NwRec R{rec + __ldg(sidx + jj), (long)ns};
+    const int j = __ldg(sidx + jj);
+    const NwRec R{tab.rec + j, (long)tab.ns};
     const long ld = 2L * nsb;
     for (int ii = blockIdx.y; ii < nrb; ii += gridDim.y) {
-        const double *rc = rcv + (long)__ldg(ridx + ii) * RC_SIZE;
-        double rloc[RC_SIZE];
+        double X[3], vs[3], vd[3], vn[3], oS[3], oD[3], bS[3], bD[3];
+        enu_receiver(rcv + (long)__ldg(ridx + ii) * RC_SIZE, X, vs, vd, vn);
+        tri_rows<3>(X, vs, vd, vn, R, cst, oS, oD);
+        tri_slip(R, bS, bD);
+#pragma unroll 1
+        for (int side = 0; side < 3; side++) {
+            const int id = __ldg(tab.edge + (long)side * tab.ns + j);
+            const double sg = (id & 1) ? -1.0 : 1.0;
+            double ed[NE_SIZE], o[3][3];
+            load_edge(tab, id >> 1, ed);
+            nw_edge_rows<3>(X, vs, vd, vn, ed, cst, o);
 #pragma unroll
-        for (int f = 0; f < RC_SIZE; f++) rloc[f] = __ldg(rc + f);
-        double sS[6], sD[6], tS[3], tD[3];
-        nw_part_stress<PART>(rloc, R, cst, sS, sD);
-        traction3(rloc, sS, tS);
-        traction3(rloc, sD, tD);
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            double2 *p = reinterpret_cast<double2 *>(out + (3L * ii + c) * ld + 2L * jj);
-            if (PART == 0) {
-                *p = make_double2(tS[c], tD[c]);
-            } else {
-                const double2 o = *p;
-                *p = make_double2(o.x + tS[c], o.y + tD[c]);
+            for (int q = 0; q < 3; q++) {
+                oS[q] += sg * (o[q][0] * bS[0] + o[q][1] * bS[1] + o[q][2] * bS[2]);
+                oD[q] += sg * (o[q][0] * bD[0] + o[q][1] * bD[1] + o[q][2] * bD[2]);
             }
         }
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            *reinterpret_cast<double2 *>(out + (3L * ii + c) * ld + 2L * jj) = make_double2(oS[c], oD[c]);
     }
 }
 
@@ -470,20 +597,107 @@ static void build_rect_sources(ucg_ctx *c, int mode, std::vector<double> &s)
     }
 }
 
-static void build_tri_sources(ucg_ctx *c, std::vector<double> &s)
+// a context workspace of at least `bytes` (its earlier contents are lost)
+template <class T>
+static int workspace(ucg_ctx *c, int which, size_t bytes, T **out)
 {
-    const int ns = c->nt;
-    s.assign((size_t)ns * NW_SIZE, 0.0);
-    std::vector<double> r(NW_SIZE);
-    for (int j = 0; j < ns; j++) {
-        const double *A = &c->tvert[3L * (c->ti1[j] - 1)];
-        const double *B = &c->tvert[3L * (c->ti2[j] - 1)];
-        const double *C = &c->tvert[3L * (c->ti3[j] - 1)];
-        // NED -> ENU (nikkhoo15.f90:143-146)
-        double P1[3] = {A[1], A[0], -A[2]}, P2[3] = {B[1], B[0], -B[2]}, P3[3] = {C[1], C[0], -C[2]};
-        nw_prepare(P1, P2, P3, r.data());
-        for (int f = 0; f < NW_SIZE; f++) s[(size_t)f * ns + j] = r[f];
+    if (c->ws_bytes[which] < bytes) {
+        UCG_CUDA(cudaStreamSynchronize(c->stream));
+        if (c->ws[which]) cudaFree(c->ws[which]);
+        c->ws[which] = nullptr;
+        c->ws_bytes[which] = 0;
+        const cudaError_t e = cudaMalloc(&c->ws[which], bytes);
+        if (e != cudaSuccess) {
+            c->ws[which] = nullptr;
+            return cuda_fail(c, e, "cudaMalloc(assembly workspace)");
+        }
+        c->ws_bytes[which] = bytes;
     }
+    *out = static_cast<T *>(c->ws[which]);
+    return UCG_OK;
+}
+
+// a host table into a workspace
+template <class T, class H>
+static int upload(ucg_ctx *c, int which, const std::vector<H> &h, T **out)
+{
+    const int rc = workspace(c, which, sizeof(H) * h.size(), out);
+    if (rc) return rc;
+    UCG_CUDA(cudaMemcpyAsync(*out, h.data(), sizeof(H) * h.size(), cudaMemcpyHostToDevice, c->stream));
+    return UCG_OK;
+}
+
+// the receiver table of every element
+static int upload_receivers(ucg_ctx *c)
+{
+    std::vector<double> r;
+    build_receivers(c, r);
+    if (c->rcv_len != r.size()) {
+        if (c->rcv) cudaFree(c->rcv);
+        c->rcv = nullptr;
+        c->rcv_len = 0;
+        UCG_CUDA(cudaMalloc(&c->rcv, sizeof(double) * r.size()));
+        c->rcv_len = r.size();
+    }
+    UCG_CUDA(cudaMemcpyAsync(c->rcv, r.data(), sizeof(double) * r.size(), cudaMemcpyHostToDevice, c->stream));
+    return UCG_OK;
+}
+
+// device tables of the triangles; with edges, the
+// unique edges of the mesh by vertex pair, oriented as their first triangle
+// runs along them, numbered in triangle order so that neighbours stay close
+static int tri_tables_build(ucg_ctx *c, bool edges, TriTables *t)
+{
+    const int ns = c->nt, nve = c->nve;
+    *t = TriTables{};
+    t->ns = ns;
+    std::vector<int> id((size_t)3 * ns);
+    const std::vector<int> *ti[3] = {&c->ti1, &c->ti2, &c->ti3};
+    for (int k = 0; k < 3; k++)
+        for (int j = 0; j < ns; j++) id[(size_t)k * ns + j] = (*ti[k])[j] - 1;
+    std::vector<int> side((size_t)3 * ns);
+    std::vector<int2> ends;
+    if (edges) {
+        std::vector<int> head(nve, -1), next;   // edges chained by their smaller vertex
+        ends.reserve((size_t)ns * 2);
+        next.reserve((size_t)ns * 2);
+        for (int j = 0; j < ns; j++)
+            for (int k = 0; k < 3; k++) {
+                const int a = id[(size_t)k * ns + j], b = id[(size_t)((k + 1) % 3) * ns + j];
+                const int lo = a < b ? a : b;
+                int e = head[lo];
+                while (e >= 0 && !((ends[e].x == a && ends[e].y == b) || (ends[e].x == b && ends[e].y == a))) e = next[e];
+                if (e < 0) {
+                    e = (int)ends.size();
+                    ends.push_back(make_int2(a, b));
+                    next.push_back(head[lo]);
+                    head[lo] = e;
+                }
+                side[(size_t)k * ns + j] = 2 * e + (ends[e].x == a ? 0 : 1);
+            }
+    }
+    t->ne = (int)ends.size();
+    double *vert, *rec, *ed;
+    int *idd, *sd;
+    int2 *endd;
+    int rc;
+    if ((rc = upload(c, WS_VERT, c->tvert, &vert)) || (rc = upload(c, WS_ID, id, &idd)) ||
+        (rc = workspace(c, WS_SRC, sizeof(double) * (size_t)NW_SIZE * ns, &rec)))
+        return rc;
+    t->rec = rec;
+    k_tri_prepare<<<(ns + 127) / 128, 128, 0, c->stream>>>(vert, idd, ns, rec);
+    c->launches.count++;
+    if (edges) {
+        if ((rc = upload(c, WS_SIDE, side, &sd)) || (rc = upload(c, WS_ENDS, ends, &endd)) ||
+            (rc = workspace(c, WS_EDGE, sizeof(double) * (size_t)NE_SIZE * t->ne, &ed)))
+            return rc;
+        t->edge = sd;
+        t->ed = ed;
+        k_edge_prepare<<<(t->ne + 127) / 128, 128, 0, c->stream>>>(vert, endd, t->ne, ed);
+        c->launches.count++;
+    }
+    UCG_CUDA(cudaGetLastError());
+    return UCG_OK;
 }
 
 static void build_vol_sources(ucg_ctx *c, std::vector<double> &s)
@@ -495,6 +709,40 @@ static void build_vol_sources(ucg_ctx *c, std::vector<double> &s)
         sv_prepare(&c->vx[3 * j], c->vL[j], c->vT[j], c->vW[j], c->vstrike[j], r.data());
         for (int f = 0; f < SV_SIZE; f++) s[(size_t)f * ns + j] = r[f];
     }
+}
+
+// gridDim.y of a pair kernel: up to 8 receivers per thread, so that a thread's
+// source record is read from L1 after the first, while about 16 CTAs per SM are left
+static int receiver_grid(const ucg_ctx *c, int xblocks, int receivers)
+{
+    long per = (long)xblocks * receivers / (16L * c->sms);
+    per = per < 1 ? 1 : per > 8 ? 8 : per;
+    const long gy = (receivers + per - 1) / per;
+    return (int)(gy < 65535 ? gy : 65535);
+}
+
+// rows of receivers [e0, e1) (NR each, the first at row0) against all triangles,
+// in batches whose edge scratch stays in L2
+template <int NR>
+static int assemble_tri_rows(ucg_ctx *c, long n, int e0, int e1, long row0, const TriTables &tab, const NwConst &cst)
+{
+    if (e1 <= e0) return UCG_OK;
+    const size_t SCRATCH = (size_t)96 << 20;
+    const size_t per = sizeof(double) * 3 * NR * (size_t)tab.ne;
+    const int batch = (int)std::max<size_t>(1, std::min<size_t>(SCRATCH / per, (size_t)(e1 - e0)));
+    double *sc;
+    const int rc = workspace(c, WS_SCRATCH, per * batch, &sc);
+    if (rc) return rc;
+    const int TPB = 128, xe = (tab.ne + TPB - 1) / TPB, xt = (tab.ns + TPB - 1) / TPB;
+    for (int r0 = e0; r0 < e1; r0 += batch) {
+        const int r1 = std::min(e1, r0 + batch);
+        k_tri_edges<NR><<<dim3(xe, receiver_grid(c, xe, r1 - r0)), TPB, 0, c->stream>>>(sc, c->rcv, r0, r1, tab, cst);
+        k_assemble_tri<NR><<<dim3(xt, receiver_grid(c, xt, r1 - r0)), TPB, 0, c->stream>>>(
+            c->K, n, 2L * c->nr, row0 + (long)NR * (r0 - e0), sc, c->rcv, r0, r1, tab, cst);
+        c->launches.count += 2;
+    }
+    UCG_CUDA(cudaGetLastError());
+    return UCG_OK;
 }
 
 int assemble_matrix(ucg_ctx *c, int okada_mode)
@@ -519,22 +767,12 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     }
     c->n = n;
     c->m = m;
-    std::vector<double> rh;
-    build_receivers(c, rh);
-    if (c->rcv) cudaFree(c->rcv);
-    UCG_CUDA(cudaMalloc(&c->rcv, sizeof(double) * rh.size()));
-    UCG_CUDA(cudaMemcpyAsync(c->rcv, rh.data(), sizeof(double) * rh.size(), cudaMemcpyHostToDevice, c->stream));
+    int rc = upload_receivers(c);
+    if (rc) return rc;
 
     const int TPB = 128;
     const int gy = ne < 65535 ? ne : 65535;
     double *dsrc = nullptr;
-    auto upload = [&](const std::vector<double> &h) -> int {
-        if (dsrc) { cudaStreamSynchronize(c->stream); cudaFree(dsrc); dsrc = nullptr; }
-        UCG_CUDA(cudaMalloc(&dsrc, sizeof(double) * h.size()));
-        UCG_CUDA(cudaMemcpyAsync(dsrc, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, c->stream));
-        return UCG_OK;
-    };
-    int rc;
     // device time of each family's launches (ucg_assembly_times)
     cudaEvent_t ev[6];
     for (cudaEvent_t &e : ev) UCG_CUDA(cudaEventCreate(&e));
@@ -545,15 +783,18 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     if (c->nr) UCG_CUDA(okada_mode == UCG_OKADA_REF32IO ? cudaFuncGetAttributes(&fa, k_assemble_rect<true>)
                                                         : cudaFuncGetAttributes(&fa, k_assemble_rect<false>));
     if (c->nt) {
-        UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<0>));
-        UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<1>));
-        UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<2>));
+        UCG_CUDA(cudaFuncGetAttributes(&fa, k_tri_edges<3>));
+        UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<3>));
+        if (c->nv) {
+            UCG_CUDA(cudaFuncGetAttributes(&fa, k_tri_edges<6>));
+            UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<6>));
+        }
     }
     if (c->nv) UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_vol));
     if (c->nr) {
         std::vector<double> s;
         build_rect_sources(c, okada_mode, s);
-        if ((rc = upload(s))) return rc;
+        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
         UCG_CUDA(cudaEventRecord(ev[0], c->stream));
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         const double alpha = okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d;
@@ -569,24 +810,19 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
         UCG_CUDA(cudaEventRecord(ev[1], c->stream));
     }
     if (c->nt) {
-        std::vector<double> s;
-        build_tri_sources(c, s);
-        if ((rc = upload(s))) return rc;
+        TriTables tab;
+        if ((rc = tri_tables_build(c, true, &tab))) return rc;
         UCG_CUDA(cudaEventRecord(ev[2], c->stream));
-        NwConst cst{c->lambda / (c->lambda + c->mu) / 2.0, c->mu, c->lambda};
-        dim3 grid((c->nt + TPB - 1) / TPB, gy);
-        // main TD, image TD and free-surface term in three accumulating passes
-        k_assemble_tri<0><<<grid, TPB, 0, c->stream>>>(c->K, n, 2L * c->nr, c->rcv, ne, np, dsrc, c->nt, cst);
-        k_assemble_tri<1><<<grid, TPB, 0, c->stream>>>(c->K, n, 2L * c->nr, c->rcv, ne, np, dsrc, c->nt, cst);
-        k_assemble_tri<2><<<grid, TPB, 0, c->stream>>>(c->K, n, 2L * c->nr, c->rcv, ne, np, dsrc, c->nt, cst);
-        c->launches.count += 3;
-        UCG_CUDA(cudaGetLastError());
+        const NwConst cst{c->lambda / (c->lambda + c->mu) / 2.0, c->mu, c->lambda};
+        rc = assemble_tri_rows<3>(c, n, 0, np, 0, tab, cst);
+        if (!rc && c->nv) rc = assemble_tri_rows<6>(c, n, np, ne, 3L * np, tab, cst);
+        if (rc) return rc;
         UCG_CUDA(cudaEventRecord(ev[3], c->stream));
     }
     if (c->nv) {
         std::vector<double> s;
         build_vol_sources(c, s);
-        if ((rc = upload(s))) return rc;
+        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
         UCG_CUDA(cudaEventRecord(ev[4], c->stream));
         const double nu = c->lambda / (c->lambda + c->mu) / 2.0;
         dim3 grid((c->nv + TPB - 1) / TPB, gy);
@@ -602,7 +838,6 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
         if (have[f] && cudaEventElapsedTime(&ms, ev[2 * f], ev[2 * f + 1]) == cudaSuccess) c->asm_ms[f] = ms;
     }
     for (cudaEvent_t &e : ev) cudaEventDestroy(e);
-    if (dsrc) cudaFree(dsrc);
     c->okada_mode = okada_mode;
     c->assembled = true;
     return UCG_OK;
@@ -636,12 +871,6 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     const int TPB = 128;
     const int gy = nobs < 65535 ? nobs : 65535;
     double *dsrc = nullptr;
-    auto upload = [&](const std::vector<double> &h) -> int {
-        if (dsrc) { cudaStreamSynchronize(c->stream); cudaFree(dsrc); dsrc = nullptr; }
-        UCG_CUDA(cudaMalloc(&dsrc, sizeof(double) * h.size()));
-        UCG_CUDA(cudaMemcpyAsync(dsrc, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, c->stream));
-        return UCG_OK;
-    };
     int rc;
     cudaEvent_t ev[2];
     for (cudaEvent_t &e : ev) UCG_CUDA(cudaEventCreate(&e));
@@ -649,7 +878,7 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     if (c->nr) {
         std::vector<double> s;
         build_rect_sources(c, okada_mode, s);
-        if ((rc = upload(s))) return rc;
+        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         const double alpha = okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d;
         dim3 grid((c->nr + TPB - 1) / TPB, gy);
@@ -661,11 +890,10 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
         UCG_CUDA(cudaGetLastError());
     }
     if (c->nt) {
-        std::vector<double> s;
-        build_tri_sources(c, s);
-        if ((rc = upload(s))) return rc;
+        TriTables tab;
+        if ((rc = tri_tables_build(c, false, &tab))) return rc;
         dim3 grid((c->nt + TPB - 1) / TPB, gy);
-        k_observe_tri<<<grid, TPB, 0, c->stream>>>(c->O, n, 2L * c->nr, c->obs_dev, nobs, dsrc, c->nt,
+        k_observe_tri<<<grid, TPB, 0, c->stream>>>(c->O, n, 2L * c->nr, c->obs_dev, nobs, tab.rec, c->nt,
                                                    c->lambda / (c->lambda + c->mu) / 2.0);
         c->launches.count++;
         UCG_CUDA(cudaGetLastError());
@@ -673,7 +901,7 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     if (c->nv) {
         std::vector<double> s;
         build_vol_sources(c, s);
-        if ((rc = upload(s))) return rc;
+        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
         dim3 grid((c->nv + TPB - 1) / TPB, gy);
         k_observe_vol<<<grid, TPB, 0, c->stream>>>(c->O, n, 2L * np, c->obs_dev, nobs, dsrc, c->nv, c->mu,
                                                    c->lambda / (c->lambda + c->mu) / 2.0);
@@ -685,7 +913,6 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     float ms = 0.0f;
     if (cudaEventElapsedTime(&ms, ev[0], ev[1]) == cudaSuccess) c->obs_ms = ms;
     for (cudaEvent_t &e : ev) cudaEventDestroy(e);
-    if (dsrc) cudaFree(dsrc);
     c->O_ready = true;
     return UCG_OK;
 }
@@ -696,12 +923,8 @@ int block_sources_build(ucg_ctx *c, int okada_mode, BlockSources *bs)
 {
     if ((c->nr > 0) == (c->nt > 0) || c->nv > 0) return UCG_E_UNSUPPORTED;   // one patch family
     UCG_CUDA(cudaSetDevice(c->device));
-    std::vector<double> rh;
-    build_receivers(c, rh);
-    if (c->rcv) cudaFree(c->rcv);
-    c->rcv = nullptr;
-    UCG_CUDA(cudaMalloc(&c->rcv, sizeof(double) * rh.size()));
-    UCG_CUDA(cudaMemcpy(c->rcv, rh.data(), sizeof(double) * rh.size(), cudaMemcpyHostToDevice));
+    int rc = upload_receivers(c);
+    if (rc) return rc;
     std::vector<double> s;
     bs->family = c->nr > 0 ? 0 : 1;
     bs->okada_mode = okada_mode;
@@ -711,19 +934,14 @@ int block_sources_build(ucg_ctx *c, int okada_mode, BlockSources *bs)
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         bs->med = ok_med(okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d);
     } else {
-        build_tri_sources(c, s);
         bs->ns = c->nt;
         bs->cst = NwConst{c->lambda / (c->lambda + c->mu) / 2.0, c->mu, c->lambda};
+        return tri_tables_build(c, true, &bs->tri);
     }
-    UCG_CUDA(cudaMalloc(&bs->src, sizeof(double) * s.size()));
-    UCG_CUDA(cudaMemcpy(bs->src, s.data(), sizeof(double) * s.size(), cudaMemcpyHostToDevice));
+    double *src;
+    if ((rc = upload(c, WS_SRC, s, &src))) return rc;
+    bs->src = src;
     return UCG_OK;
-}
-
-void block_sources_free(BlockSources *bs)
-{
-    if (bs->src) cudaFree(bs->src);
-    bs->src = nullptr;
 }
 
 void assemble_block(ucg_ctx *c, const BlockSources &bs, const int *ridx, int nrb, const int *sidx, int nsb,
@@ -740,10 +958,8 @@ void assemble_block(ucg_ctx *c, const BlockSources &bs, const int *ridx, int nrb
                                                             bs.med, c->mu, c->lambda);
         c->launches.count++;
     } else {
-        k_block_tri<0><<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.src, bs.ns, bs.cst);
-        k_block_tri<1><<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.src, bs.ns, bs.cst);
-        k_block_tri<2><<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.src, bs.ns, bs.cst);
-        c->launches.count += 3;
+        k_block_tri<<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.tri, bs.cst);
+        c->launches.count++;
     }
 }
 

@@ -102,65 +102,6 @@ __device__ __forceinline__ Dd dlog_gi(Dd a, Dd ia) { return Dd{0.0, ia.v * a.x, 
 // gradient-only arctangent of n / d: (d n' - n d') / (n^2 + d^2), one division
 __device__ __forceinline__ Dd datan_q_g(Dd n, Dd d) { return datan2_g(n, d); }
 
-// Single-direction dual: a value and one directional derivative.  Evaluating a
-// field once per coordinate direction with these keeps half the live state of
-// the three-direction type, which matters for the longest expressions.
-struct Dd1 {
-    double v, d;
-    Dd1() = default;
-    __host__ __device__ constexpr Dd1(double c) : v(c), d(0.0) {}
-    __host__ __device__ constexpr Dd1(double c, double e) : v(c), d(e) {}
-};
-__device__ __forceinline__ Dd1 operator+(Dd1 a, Dd1 b) { return Dd1{a.v + b.v, a.d + b.d}; }
-__device__ __forceinline__ Dd1 operator-(Dd1 a, Dd1 b) { return Dd1{a.v - b.v, a.d - b.d}; }
-__device__ __forceinline__ Dd1 operator-(Dd1 a) { return Dd1{-a.v, -a.d}; }
-__device__ __forceinline__ Dd1 operator*(Dd1 a, Dd1 b) { return Dd1{a.v * b.v, a.d * b.v + a.v * b.d}; }
-__device__ __forceinline__ Dd1 operator+(Dd1 a, double c) { return Dd1{a.v + c, a.d}; }
-__device__ __forceinline__ Dd1 operator+(double c, Dd1 a) { return Dd1{a.v + c, a.d}; }
-__device__ __forceinline__ Dd1 operator-(Dd1 a, double c) { return Dd1{a.v - c, a.d}; }
-__device__ __forceinline__ Dd1 operator-(double c, Dd1 a) { return Dd1{c - a.v, -a.d}; }
-__device__ __forceinline__ Dd1 operator*(Dd1 a, double c) { return Dd1{a.v * c, a.d * c}; }
-__device__ __forceinline__ Dd1 operator*(double c, Dd1 a) { return Dd1{a.v * c, a.d * c}; }
-__device__ __forceinline__ Dd1 rcp(Dd1 a)
-{
-    double r = 1.0 / a.v;
-    return Dd1{r, -r * r * a.d};
-}
-__device__ __forceinline__ Dd1 operator/(Dd1 a, Dd1 b)
-{
-    double r = 1.0 / b.v, q = a.v * r;
-    return Dd1{q, (a.d - q * b.d) * r};
-}
-__device__ __forceinline__ Dd1 operator/(Dd1 a, double c)
-{
-    double r = 1.0 / c;
-    return Dd1{a.v * r, a.d * r};
-}
-__device__ __forceinline__ Dd1 operator/(double c, Dd1 a)
-{
-    double r = 1.0 / a.v, q = c * r;
-    return Dd1{q, -q * r * a.d};
-}
-__device__ __forceinline__ Dd1 dsqrt(Dd1 a)
-{
-    double s = sqrt(a.v);
-    return Dd1{s, 0.5 / s * a.d};
-}
-__device__ __forceinline__ Dd1 dlog_g(Dd1 a) { return Dd1{0.0, a.d / a.v}; }
-__device__ __forceinline__ Dd1 datan_g(Dd1 a) { return Dd1{0.0, a.d / (1.0 + a.v * a.v)}; }
-
-__device__ __forceinline__ void dsqrt_inv(Dd1 a, Dd1 &s, Dd1 &is)
-{
-    const double q = sqrt(a.v), r = 1.0 / q, h = 0.5 * r * a.d;
-    s = Dd1{q, h};
-    is = Dd1{r, -r * r * h};
-}
-__device__ __forceinline__ Dd1 dlog_gi(Dd1 a, Dd1 ia) { return Dd1{0.0, ia.v * a.d}; }
-__device__ __forceinline__ Dd1 datan_q_g(Dd1 n, Dd1 d)
-{
-    return Dd1{0.0, (d.v * n.d - n.v * d.d) / (n.v * n.v + d.v * d.v)};
-}
-
 // Plain value: the same closed forms evaluated for the displacement itself
 // (observation-point displacements).  The "gradient-only" forms of the dual
 // types above skip the value of a logarithm or arctangent; for this type the

@@ -798,7 +798,6 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         cudaFree(jobs_d);
         cudaFree(ranks_d);
         cudaFree(errs_d);
-        block_sources_free(&bs);
     };
 
     // the blocks in batches that fit the scratch

@@ -5,16 +5,18 @@
 // The reference evaluates TD strain with straininhalfspace_
 // (fortran/3d/src/StrainInHalfSpace.c:42-177), whose expressions are the
 // analytic derivatives of the TD displacement field of the same paper
-// (fortran/3d/src/DispInHalfSpace.c:153-617).  Here the displacement field is
-// evaluated on dual numbers seeded with the observation point, which gives the
-// exact displacement gradient, and the three parts are assembled as
-// straininhalfspace_ does: main TD + image TD (vertices mirrored in z) +
-// harmonic free-surface correction; the image's yz and zz stresses change sign
-// when all vertices lie at z = 0 (StrainInHalfSpace.c:162-165); configuration I
-// of the free-surface angular-dislocation pairs is taken in the mirrored frame
-// (StrainInHalfSpace.c:644-652).  Because only the gradient is formed, the
-// logarithms and arctangents of the displacement field contribute through their
-// derivatives alone and are never evaluated.
+// (fortran/3d/src/DispInHalfSpace.c:153-617): main TD + image TD (vertices
+// mirrored in z) + harmonic free-surface correction; the image's yz and zz
+// stresses change sign when all vertices lie at z = 0 (StrainInHalfSpace.c:
+// 162-165); configuration I of the free-surface angular-dislocation pairs is
+// taken in the mirrored frame (StrainInHalfSpace.c:644-652).  The same three
+// parts are summed here, but the strain is formed from shorter expressions of
+// the same field (derived below from the displacement's), and the free-surface
+// term is formed per mesh edge: it depends on the edge alone and is linear in
+// the slip, so the two triangles of an edge share it.  Only the gradient is
+// formed, so the logarithms and arctangents contribute through their
+// derivatives alone.  The displacement itself (observation points) is
+// evaluated from the displacement expressions with plain values.
 //
 // Per-source geometry (frames, vertex coordinates in the TD frame, angular-
 // dislocation angles, free-surface side frames, slip vectors) is computed once
@@ -464,67 +466,346 @@ __device__ inline void nw_side(const Dd X[3], const NwRec &R, int o, double nu, 
     uD[2] = uD[2] - vD2;
 }
 
-// gradient -> stress, C order xx, xy, xz, yy, yz, zz (ENU)
-__device__ __forceinline__ void nw_stress(const Dd u[3], double mu, double lambda, double s[6])
-{
-    const double exx = u[0].x, eyy = u[1].y, ezz = u[2].z;
-    const double exy = 0.5 * (u[0].y + u[1].x);
-    const double exz = 0.5 * (u[0].z + u[2].x);
-    const double eyz = 0.5 * (u[1].z + u[2].y);
-    const double kk = exx + eyy + ezz;
-    s[0] = 2.0 * mu * exx + lambda * kk;
-    s[1] = 2.0 * mu * exy;
-    s[2] = 2.0 * mu * exz;
-    s[3] = 2.0 * mu * eyy + lambda * kk;
-    s[4] = 2.0 * mu * eyz;
-    s[5] = 2.0 * mu * ezz + lambda * kk;
-}
+// ---- stress of a pair ----------------------------------------------------------
 
-// ENU stress (C order) -> NED s11,s12,s13,s22,s23,s33 (nikkhoo15.f90:156-161)
-__device__ __forceinline__ void nw_to_ned(const double e[6], double s[6])
+// Receiver rows.  r: the receiver's record (NED: centre, strike, dip, normal);
+// rows are the 3 tractions (ts, td, tn) of a patch or the 6 stresses (s11, s12,
+// s13, s22, s23, s33 in the element's frame) of a volume, formed from a stress
+// given in a frame where the receiver's unit vectors are vs, vd, vn.
+template <int NR>
+__device__ __forceinline__ void nw_rows(const double vs[3], const double vd[3], const double vn[3], double sxx,
+                                        double sxy, double sxz, double syy, double syz, double szz, double o[NR])
 {
-    s[0] = e[3]; s[1] = e[1]; s[2] = -e[4]; s[3] = e[0]; s[4] = -e[2]; s[5] = e[5];
-}
-
-// One part of the TD stress at receiver xr (NED) for unit strike slip (sS) and
-// unit dip slip (sD): PART 0 main TD, 1 image TD (with the surface sign flip),
-// 2 harmonic free-surface term.  The three parts sum to straininhalfspace_'s
-// stress; evaluating them in separate passes keeps the live state of each pass
-// small enough for the register file.
-template <int PART>
-__device__ inline void nw_part_stress(const double xr[3], const NwRec &R, const NwConst &c, double sS[6],
-                                      double sD[6])
-{
-    Dd X[3] = {Dd{xr[1], 1.0, 0.0, 0.0}, Dd{xr[0], 0.0, 1.0, 0.0}, Dd{-xr[2], 0.0, 0.0, 1.0}};
-    Dd uS[3] = {dd(0), dd(0), dd(0)}, uD[3] = {dd(0), dd(0), dd(0)};
-    if (PART == 2) {
-        // one pass per derivative direction with single-direction duals
-        double gS[3][3], gD[3][3];
-#pragma unroll 1
-        for (int dir = 0; dir < 3; dir++) {
-            Dd1 X1[3] = {Dd1{xr[1], dir == 0 ? 1.0 : 0.0}, Dd1{xr[0], dir == 1 ? 1.0 : 0.0},
-                         Dd1{-xr[2], dir == 2 ? 1.0 : 0.0}};
-            Dd1 vS[3] = {Dd1(0.0), Dd1(0.0), Dd1(0.0)}, vD[3] = {Dd1(0.0), Dd1(0.0), Dd1(0.0)};
-#pragma unroll 1
-            for (int side = 0; side < 3; side++) nw_side<Dd1>(X1, R, NW_FS + side * FS_SIZE, c.nu, vS, vD);
-            for (int k = 0; k < 3; k++) { gS[k][dir] = vS[k].d; gD[k][dir] = vD[k].d; }
-        }
-        for (int k = 0; k < 3; k++) {
-            uS[k] = Dd{0.0, gS[k][0], gS[k][1], gS[k][2]};
-            uD[k] = Dd{0.0, gD[k][0], gD[k][1], gD[k][2]};
-        }
+    const double t0 = sxx * vn[0] + sxy * vn[1] + sxz * vn[2];
+    const double t1 = sxy * vn[0] + syy * vn[1] + syz * vn[2];
+    const double t2 = sxz * vn[0] + syz * vn[1] + szz * vn[2];
+    if (NR == 3) {
+        // okada92.f90:390-398
+        o[0] = t0 * vs[0] + t1 * vs[1] + t2 * vs[2];
+        o[1] = t0 * vd[0] + t1 * vd[1] + t2 * vd[2];
+        o[2] = t0 * vn[0] + t1 * vn[1] + t2 * vn[2];
     } else {
-        if (!nw_td_fs(X, R, PART == 0 ? NW_MAIN : NW_IMG, c.nu, uS, uD)) {
-            for (int k = 0; k < 6; k++) { sS[k] = nan(""); sD[k] = nan(""); }
-            return;
-        }
+        // okada92.f90:445-462 (the third axis is the dip vector negated)
+        const double a0 = sxx * vs[0] + sxy * vs[1] + sxz * vs[2];
+        const double a1 = sxy * vs[0] + syy * vs[1] + syz * vs[2];
+        const double a2 = sxz * vs[0] + syz * vs[1] + szz * vs[2];
+        const double b0 = sxx * vd[0] + sxy * vd[1] + sxz * vd[2];
+        const double b1 = sxy * vd[0] + syy * vd[1] + syz * vd[2];
+        const double b2 = sxz * vd[0] + syz * vd[1] + szz * vd[2];
+        o[0] = a0 * vs[0] + a1 * vs[1] + a2 * vs[2];
+        o[1] = t0 * vs[0] + t1 * vs[1] + t2 * vs[2];
+        o[2 % NR] = -(b0 * vs[0] + b1 * vs[1] + b2 * vs[2]);
+        o[3 % NR] = t0 * vn[0] + t1 * vn[1] + t2 * vn[2];
+        o[4 % NR] = -(t0 * vd[0] + t1 * vd[1] + t2 * vd[2]);
+        o[5 % NR] = b0 * vd[0] + b1 * vd[1] + b2 * vd[2];
     }
-    double eS[6], eD[6];
-    nw_stress(uS, c.mu, c.lambda, eS);
-    nw_stress(uD, c.mu, c.lambda, eD);
-    if (PART == 1 && R[NW_SURF] != 0.0) { eS[4] = -eS[4]; eS[5] = -eS[5]; eD[4] = -eD[4]; eD[5] = -eD[5]; }
-    nw_to_ned(eS, sS);
-    nw_to_ned(eD, sD);
+}
+
+// Strain of the angular dislocation of one TD corner, added to the TD-frame
+// strain (xx, 2xy, 2xz, yy, 2yz, zz) of the strike (by = 1) and dip (bz = -1)
+// modes, all over k = 1 / (8 pi (1 - nu)).  (ga, de) are the cosine and sine
+// that take (y, z) into the corner's frame; s, c the corner's sine and cosine;
+// m = 1 - 2 nu; r receives the distance to the corner.
+//
+// With zeta = y1 s + z1 c, p = 1 / (r - zeta), q = 1 / (r - z1), rho = 1 / r,
+// D = c p - q, the displacement of DispInHalfSpace.c:541-575 is, over k,
+//   by: u = x^2 rho D - m (c ln(r - zeta) - ln(r - z1)),
+//       v = x (y1 rho D - s c p),  w = x (rho - c (c p - z1 rho p))
+//   bz: s (m ln(r - zeta) - x^2 rho p),  s x (s p - y1 rho p),  s x (c p - z1 rho p)
+// so that the whole gradient needs only those of rho D and rho p, and the
+// gradient of p is -p times that of ln(r - zeta).
+__device__ __forceinline__ void nw_corner_strain(double x, double y, double z, double ga, double de, double s,
+                                                 double c, double m, double &r, double eS[6], double eD[6])
+{
+    const double y1 = ga * y - de * z, z1 = de * y + ga * z;
+    const double zeta = y1 * s + z1 * c;
+    r = sqrt(x * x + y1 * y1 + z1 * z1);
+    const double rho = 1.0 / r, p = 1.0 / (r - zeta), q = 1.0 / (r - z1);
+    const double nx = x * rho, ny = y1 * rho, nz = z1 * rho, rr = rho * rho;
+    const Dd R{rho, -rr * nx, -rr * ny, -rr * nz};
+    const Dd Lp{0.0, p * nx, p * (ny - s), p * (nz - c)};
+    const Dd Lq{0.0, q * nx, q * ny, q * (nz - 1.0)};
+    const Dd P{p, -p * Lp.x, -p * Lp.y, -p * Lp.z};
+    const Dd D{c * p - q, c * P.x + q * Lq.x, c * P.y + q * Lq.y, c * P.z + q * Lq.z};
+    const Dd RD = R * D, RP = R * P;
+    const double x2 = x * x, sc = s * c;
+    const Dd uy{0.0, x2 * RD.x + 2.0 * x * RD.v - m * (c * Lp.x - Lq.x), x2 * RD.y - m * (c * Lp.y - Lq.y),
+                x2 * RD.z - m * (c * Lp.z - Lq.z)};
+    const Dd uz{0.0, m * Lp.x - x2 * RP.x - 2.0 * x * RP.v, m * Lp.y - x2 * RP.y, m * Lp.z - x2 * RP.z};
+    // v and w over x
+    const Dd v0{y1 * RD.v - sc * p, y1 * RD.x - sc * P.x, y1 * RD.y + RD.v - sc * P.y, y1 * RD.z - sc * P.z};
+    const Dd w1{c * p - z1 * RP.v, c * P.x - z1 * RP.x, c * P.y - z1 * RP.y, c * P.z - z1 * RP.z - RP.v};
+    const Dd w0{rho - c * w1.v, R.x - c * w1.x, R.y - c * w1.y, R.z - c * w1.z};
+    const Dd v1{s * p - y1 * RP.v, s * P.x - y1 * RP.x, s * P.y - y1 * RP.y - RP.v, s * P.z - y1 * RP.z};
+    const double B[6] = {uy.x, uy.y + x * v0.x + v0.v, uy.z + x * w0.x + w0.v, x * v0.y, x * (v0.z + w0.y), x * w0.z};
+    const double G[6] = {s * uz.x, s * (uz.y + x * v1.x + v1.v), s * (uz.z + x * w1.x + w1.v), s * x * v1.y,
+                         s * x * (v1.z + w1.y), s * x * w1.z};
+    // the modes' slip in the corner's frame, and the strain back to the TD frame
+    const double g2 = ga * ga, d2 = de * de, gd = ga * de;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        double e[6];
+        double *o = t ? eD : eS;
+#pragma unroll
+        for (int k = 0; k < 6; k++) e[k] = t ? de * B[k] - ga * G[k] : ga * B[k] + de * G[k];
+        o[0] += e[0];
+        o[1] += ga * e[1] + de * e[2];
+        o[2] += ga * e[2] - de * e[1];
+        o[3] += g2 * e[3] + gd * e[4] + d2 * e[5];
+        o[4] += 2.0 * gd * (e[5] - e[3]) + (g2 - d2) * e[4];
+        o[5] += d2 * e[3] - gd * e[4] + g2 * e[5];
+    }
+}
+
+// gradient of the solid angle over one side of the TD: a and b the vectors from
+// the receiver to its ends (x component -x), ra and rb their lengths
+__device__ __forceinline__ void nw_side_angle(double x, double ay, double az, double ra, double by, double bz,
+                                              double rb, double f[3])
+{
+    const double ab = ra * rb;
+    const double w = (ra + rb) / (ab * (ab + x * x + ay * by + az * bz));
+    f[0] += w * (ay * bz - az * by);
+    f[1] += w * (x * (bz - az));
+    f[2] += w * (x * (ay - by));
+}
+
+// Rows of a receiver at (X0, X1, X2) (ENU) with unit vectors vs, vd, vn (ENU)
+// for unit strike and dip slip of one TD (o: NW_MAIN, or NW_IMG with flip when
+// the image's yz and zz stresses change sign), added to oS and oD.
+// Returns false when the point lies on a TD side (reference result: NaN).
+template <int NR>
+__device__ __forceinline__ bool nw_td_rows(const double X[3], const double vs[3], const double vd[3],
+                                           const double vn[3], const NwRec &R, int o, bool flip, const NwConst &cst,
+                                           double oS[NR], double oD[NR])
+{
+    const double d0 = X[0] - R[o + TD_P2], d1 = X[1] - R[o + TD_P2 + 1], d2 = X[2] - R[o + TD_P2 + 2];
+    const double x = R[o + TD_N] * d0 + R[o + TD_N + 1] * d1 + R[o + TD_N + 2] * d2;
+    const double y = R[o + TD_S] * d0 + R[o + TD_S + 1] * d1 + R[o + TD_S + 2] * d2;
+    const double z = R[o + TD_D] * d0 + R[o + TD_D + 1] * d1 + R[o + TD_D + 2] * d2;
+    const double p1y = R[o + TD_P1], p1z = R[o + TD_P1 + 1], p3y = R[o + TD_P3], p3z = R[o + TD_P3 + 1];
+    const int mode = nw_trimode(y, z, x, p1y, p1z, p3y, p3z);
+    if (mode == 0) return false;
+    const double sg = (mode == 1) ? 1.0 : -1.0;   // sign on e12, e23 (corners 2, 3), opposite on e13
+    const double m = 1.0 - 2.0 * cst.nu;
+    double eS[6] = {0, 0, 0, 0, 0, 0}, eD[6] = {0, 0, 0, 0, 0, 0}, r1, r2, r3;
+    nw_corner_strain(x, y - p1y, z - p1z, -sg * R[o + TD_E13 + 1], -sg * R[o + TD_E13], R[o + TD_CS + 1],
+                     R[o + TD_CS], m, r1, eS, eD);
+    nw_corner_strain(x, y, z, sg * R[o + TD_E12 + 1], sg * R[o + TD_E12], R[o + TD_CS + 3], R[o + TD_CS + 2], m, r2,
+                     eS, eD);
+    nw_corner_strain(x, y - p3y, z - p3z, sg * R[o + TD_E23 + 1], sg * R[o + TD_E23], R[o + TD_CS + 5],
+                     R[o + TD_CS + 4], m, r3, eS, eD);
+    // Burgers function: minus the solid angle over 4 pi, times the slip
+    const double ay = p1y - y, az = p1z - z, cy = p3y - y, cz = p3z - z;
+    double f[3] = {0.0, 0.0, 0.0};
+    nw_side_angle(x, ay, az, r1, -y, -z, r2, f);
+    nw_side_angle(x, -y, -z, r2, cy, cz, r3, f);
+    nw_side_angle(x, cy, cz, r3, ay, az, r1, f);
+    const double h = -2.0 * (1.0 - cst.nu);
+    eS[1] += h * f[0]; eS[3] += h * f[1]; eS[4] += h * f[2];
+    eD[2] -= h * f[0]; eD[4] -= h * f[1]; eD[5] -= h * f[2];
+    // the receiver's unit vectors in the TD frame
+    double w[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const double n0 = R[o + TD_N + 3 * a], n1 = R[o + TD_N + 3 * a + 1], n2 = R[o + TD_N + 3 * a + 2];
+        w[0][a] = n0 * vs[0] + n1 * vs[1] + n2 * vs[2];
+        w[1][a] = n0 * vd[0] + n1 * vd[1] + n2 * vd[2];
+        w[2][a] = n0 * vn[0] + n1 * vn[1] + n2 * vn[2];
+    }
+    const double k = 1.0 / 8.0 / 3.141592653589793 / (1.0 - cst.nu);
+    const double mu = k * cst.mu, la = k * cst.lambda;
+    // a TD with all vertices at z = 0 lies flat: ENU's yz and zz are its xy and xx
+    const double fl = flip ? -1.0 : 1.0;
+#pragma unroll
+    for (int t = 0; t < 2; t++) {
+        const double *e = t ? eD : eS;
+        double *out = t ? oD : oS;
+        const double tr = la * (e[0] + e[3] + e[5]);
+        double v[NR];
+        nw_rows<NR>(w[0], w[1], w[2], fl * (2.0 * mu * e[0] + tr), fl * mu * e[1], mu * e[2], 2.0 * mu * e[3] + tr,
+                    mu * e[4], 2.0 * mu * e[5] + tr, v);
+#pragma unroll
+        for (int q = 0; q < NR; q++) out[q] += v[q];
+    }
+    return true;
+}
+
+// ---- free-surface term of an edge -------------------------------------------------
+
+// record of the edge PA -> PB (ENU)
+enum : int {
+    NE_PA = 0,   // 3
+    NE_E1 = 3,   // 2: horizontal direction of the edge
+    NE_H = 5,    // horizontal length
+    NE_PBZ = 6,  // up coordinate of PB
+    NE_S = 7,    // sine and cosine of the angle between the edge and the vertical; the sine is 0
+    NE_C = 8,    // on a vertical edge, whose pair contributes nothing (DispInHalfSpace.c:474-479)
+    NE_SIZE = 9
+};
+
+__host__ __device__ inline void nw_prepare_edge(const double PA[3], const double PB[3], double *r)
+{
+    const double s0 = PB[0] - PA[0], s1 = PB[1] - PA[1], s2 = PB[2] - PA[2];
+    const double h = sqrt(s0 * s0 + s1 * s1), l = sqrt(s0 * s0 + s1 * s1 + s2 * s2);
+    const double beta = acos(-s2 / l);
+    const bool vertical = fabs(beta) < 2.220446049250313e-16 || fabs(3.141592653589793 - beta) < 2.220446049250313e-16;
+    r[NE_PA] = PA[0]; r[NE_PA + 1] = PA[1]; r[NE_PA + 2] = PA[2];
+    r[NE_E1] = vertical ? 1.0 : s0 / h;
+    r[NE_E1 + 1] = vertical ? 0.0 : s1 / h;
+    r[NE_H] = h;
+    r[NE_PBZ] = PB[2];
+    r[NE_S] = vertical ? 0.0 : sin(beta);
+    r[NE_C] = cos(beta);
+}
+
+// Strain (11, 2 12, 2 13, 22, 2 23, 33) of the free-surface field of one
+// angular dislocation for unit slip along each axis of its frame, times sgn,
+// added to E (over 1 / (4 pi (1 - nu))).  S, C, T, iS: sine, cosine, cotangent
+// and reciprocal sine of the dislocation's angle.
+//
+// The displacement is AngDisDispFSC's (DispInHalfSpace.c:577-617).  Written
+// with rho = 1 / r, A = a rho, q = 1 / (r + y3b), p = 1 / (r + z3b), X = y1 q,
+// Z = z1b p, c3 = y3b rho, g = (y3b - a) rho, L = ln(r + y3b), M = ln(r + z3b),
+// N = L - C M, m = 1 - 2 nu, w = 1 - nu, and using
+//   (r + y3b)(r - y3b) = y1^2 + y2^2,   (r + z3b)(r - z3b) = z1b^2 + y2^2,
+//   p (r C + y3b) = C + S Z,   p (r S - y1) = S - C Z,   (C + c3) p = rho (C + S Z),
+// its nine components become (u_i of slip b_j; y2 divided out where it is a factor)
+//   u1(b1) = -2 w m T^2 F + y2 (G + C^2 H + 2 w C^2 S p g)
+//   u2(b2) =  2 w m T^2 F - y2 (G + H)
+//     G = m (T q (m - A) - q X (nu + A)) + g (T (A rho - m q) + X (q (2 nu + A) + A rho))
+//     H = m p (T + A/S) + p g (m C T - Z (C + A) - T A - A c3 / S)
+//   u2(b1) = m (2 w T^2 N - nu L - m M C) - m (T X (m - A) + (nu + A) B - A)
+//            + g (m T X - 2 nu + (2 nu + A) B - A c3 - A y1 rho (X + T))
+//            - m T Z (C + A) - (y3b - a) C p (C + A)
+//            + g (C^2 + C Z^2 (C + A) - m T Z + T K),  B = r q - X^2, K = A Z (C + c3)
+//   u1(b2) = u2(b1) + 2 nu (m N + g S (S - C Z))    (up to a constant)
+//   u3(b1) = 2 w m T F + y2 (2 w (q (2 nu + A) - C p (C + A)) + g (2 nu q + A rho) + C p g (m - W))
+//   u1(b3) = y2 (m (q (1 + A) - C p (C + A)) - g (A rho + q) + C p g W)
+//   u3(b3) = 2 w F + y2 S (2 w p (C + A) + p g (1 + W)),  W = (C + S Z)(C + A) + A c3
+//   u3(b2) = -2 w m T N - 2 w (X (2 nu + A) - Z (C + A)) - (y3b - a) S p (C + A)
+//            + g (m C S - 2 nu (X - C^2 Z) + J),  J = S Z^2 (C + A) + K - A y1 rho
+//   u2(b3) = m (-S M - X (1 + A) + Z (C + A)) + (y3b - a) S p (C + A) + g (X - Z - C S - J)
+// with F the angle of DispInHalfSpace.c:585, whose gradient is that of the
+// solid angle of its two half-lines.  The gradient of each factor is short, so
+// one evaluation with three-direction duals costs about 500 FP64 instructions
+// per endpoint, against about 3 x 1,300 for the expressions as published on
+// single-direction duals.
+__device__ __forceinline__ void nw_fsc_strain(double y1, double y2, double y3, double a, double S, double C, double T,
+                                              double iS, double nu, double sgn, double E[3][6])
+{
+    const double y3b = y3 + 2.0 * a, ya = y3 + a;
+    const double z1 = y1 * C + y3b * S, z3 = y3b * C - y1 * S;
+    const double r = sqrt(y1 * y1 + y2 * y2 + y3b * y3b);
+    const double rho = 1.0 / r, q = 1.0 / (r + y3b), p = 1.0 / (r + z3);
+    const double n1 = y1 * rho, n2 = y2 * rho, n3 = y3b * rho, rr = rho * rho;
+    const double m = 1.0 - 2.0 * nu, w = 1.0 - nu, nu2 = 2.0 * nu;
+    const Dd R{rho, -rr * n1, -rr * n2, -rr * n3};
+    const Dd L{0.0, n1 * q, n2 * q, rho};
+    const Dd M{0.0, p * (n1 - S), p * n2, p * (n3 + C)};
+    const Dd N{0.0, L.x - C * M.x, L.y - C * M.y, L.z - C * M.z};
+    const Dd Q{q, -q * L.x, -q * L.y, -q * L.z};
+    const Dd P{p, -p * M.x, -p * M.y, -p * M.z};
+    const Dd X{y1 * q, y1 * Q.x + q, y1 * Q.y, y1 * Q.z};
+    const Dd Z{z1 * p, z1 * P.x + C * p, z1 * P.y, z1 * P.z + S * p};
+    const Dd F{0.0, n2 * (q - C * p), rho * (Z.v - X.v), -S * n2 * p};
+    const Dd g{ya * rho, ya * R.x, ya * R.y, ya * R.z + rho};
+    const Dd c3{n3, y3b * R.x, y3b * R.y, y3b * R.z + rho};
+    const Dd V{1.0 - y3b * q, -y3b * Q.x, -y3b * Q.y, -y3b * Q.z - q};   // r q
+    const Dd A = a * R;
+    const Dd Ar = A * R, QA = Q * A, PA = P * A, XA = X * A, ZA = Z * A, cA = c3 * A;
+    const Dd yAr{y1 * Ar.v, y1 * Ar.x + Ar.v, y1 * Ar.y, y1 * Ar.z};
+    const Dd Pc = C * P + PA, Zc = C * Z + ZA;
+    const Dd yPc{0.0, ya * Pc.x, ya * Pc.y, ya * Pc.z + Pc.v};
+    const Dd Pg = P * g, gQ = g * Q, gA = g * Ar;
+    const Dd ZZc = Z * Zc, K = C * ZA + Z * cA;
+    const Dd B = V - X * X;
+    const Dd AB = A * B;
+    // b1 -> u2 and b2 -> u1
+    const Dd e12 = m * ((2.0 * w * T * T + m) * N - (nu + m) * L) - m * (T * (m * X - XA) + nu * B + AB - A)
+                 - m * T * Zc - C * yPc
+                 + g * (m * T * (X - Z) - nu2 + nu2 * B + AB - cA - yAr * (X + T) + C * C + C * ZZc + T * K);
+    const Dd e21 = e12 + nu2 * (m * N + S * (S * g - C * (g * Z)));
+    // b1 -> u1 and b2 -> u2
+    const Dd QA2 = nu2 * Q + QA;
+    const Dd G = m * (T * (m * Q - QA) - X * (nu * Q + QA)) + g * (T * (Ar - m * Q) + X * (QA2 + Ar));
+    const Dd H = m * (T * P + iS * PA) + Pg * (m * C * T - Zc - T * A - iS * cA);
+    const double cF = 2.0 * w * m * T * T;
+    const Dd i22 = G + H, i11 = G + C * C * H + (2.0 * w * C * C * S) * Pg;
+    const Dd e11{0.0, y2 * i11.x - cF * F.x, y2 * i11.y + i11.v - cF * F.y, y2 * i11.z - cF * F.z};
+    const Dd e22{0.0, cF * F.x - y2 * i22.x, cF * F.y - y2 * i22.y - i22.v, cF * F.z - y2 * i22.z};
+    // b1 -> u3, b3 -> u1 and u3
+    const Dd W = C * A + S * Zc + cA + C * C;
+    const Dd PW = Pg * W;
+    const Dd i13 = 2.0 * w * (QA2 - C * Pc) + nu2 * gQ + gA + C * (m * Pg - PW);
+    const Dd i31 = m * (Q + QA - C * Pc) - gA - gQ + C * PW;
+    const Dd i33 = S * (2.0 * w * Pc + Pg + PW);
+    const double c13 = 2.0 * w * m * T, c33 = 2.0 * w;
+    const Dd e13{0.0, c13 * F.x + y2 * i13.x, c13 * F.y + y2 * i13.y + i13.v, c13 * F.z + y2 * i13.z};
+    const Dd e31{0.0, y2 * i31.x, y2 * i31.y + i31.v, y2 * i31.z};
+    const Dd e33{0.0, c33 * F.x + y2 * i33.x, c33 * F.y + y2 * i33.y + i33.v, c33 * F.z + y2 * i33.z};
+    // b2 -> u3, b3 -> u2
+    const Dd J = S * ZZc + K - yAr;
+    const Dd e23 = -c13 * N - 2.0 * w * (nu2 * X + XA - Zc) - S * yPc + g * (m * C * S - nu2 * (X - C * C * Z) + J);
+    const Dd e32 = m * (Zc - S * M - X - XA) + S * yPc + g * (X - Z - C * S - J);
+    const Dd u[3][3] = {{e11, e12, e13}, {e21, e22, e23}, {e31, e32, e33}};
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        E[b][0] += sgn * u[b][0].x;
+        E[b][1] += sgn * (u[b][0].y + u[b][1].x);
+        E[b][2] += sgn * (u[b][0].z + u[b][2].x);
+        E[b][3] += sgn * u[b][1].y;
+        E[b][4] += sgn * (u[b][1].z + u[b][2].y);
+        E[b][5] += sgn * u[b][2].z;
+    }
+}
+
+// Rows of a receiver (ENU, as in nw_td_rows) for unit slip along east, north
+// and up carried by the edge PA -> PB: out[q][axis] (AngSetupFSC).
+template <int NR>
+__device__ __forceinline__ void nw_edge_rows(const double X[3], const double vs[3], const double vd[3],
+                                             const double vn[3], const double ed[NE_SIZE], const NwConst &cst,
+                                             double out[NR][3])
+{
+    const double S = ed[NE_S];
+    if (S == 0.0) {
+#pragma unroll
+        for (int q = 0; q < NR; q++) out[q][0] = out[q][1] = out[q][2] = 0.0;
+        return;
+    }
+    // side frame: along the edge, across it, down; mirrored with the angle
+    // pi - beta (configuration I) where the receiver lies on PB's side of PA
+    double e1x = ed[NE_E1], e1y = ed[NE_E1 + 1], C = ed[NE_C], h = ed[NE_H];
+    const double d0 = X[0] - ed[NE_PA], d1 = X[1] - ed[NE_PA + 1];
+    double y1 = e1x * d0 + e1y * d1, y2 = e1y * d0 - e1x * d1;
+    if (y1 >= 0.0) {
+        e1x = -e1x; e1y = -e1y; C = -C; h = -h; y1 = -y1; y2 = -y2;
+    }
+    const double iS = 1.0 / S, T = C * iS;
+    const double aA = -ed[NE_PA + 2], aB = -ed[NE_PBZ];
+    double E[3][6] = {{0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0}};
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const double a = k ? aB : aA;
+        nw_fsc_strain(k ? y1 - h : y1, y2, -X[2] - a, a, S, C, T, iS, cst.nu, k ? 1.0 : -1.0, E);
+    }
+    const double w0[3] = {e1x * vs[0] + e1y * vs[1], e1y * vs[0] - e1x * vs[1], -vs[2]};
+    const double w1[3] = {e1x * vd[0] + e1y * vd[1], e1y * vd[0] - e1x * vd[1], -vd[2]};
+    const double w2[3] = {e1x * vn[0] + e1y * vn[1], e1y * vn[0] - e1x * vn[1], -vn[2]};
+    const double k = 1.0 / 4.0 / 3.141592653589793 / (1.0 - cst.nu);
+    const double mu = k * cst.mu, la = k * cst.lambda;
+    double o[3][NR];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const double tr = la * (E[b][0] + E[b][3] + E[b][5]);
+        nw_rows<NR>(w0, w1, w2, 2.0 * mu * E[b][0] + tr, mu * E[b][1], mu * E[b][2], 2.0 * mu * E[b][3] + tr,
+                    mu * E[b][4], 2.0 * mu * E[b][5] + tr, o[b]);
+    }
+#pragma unroll
+    for (int q = 0; q < NR; q++) {
+        out[q][0] = e1x * o[0][q] + e1y * o[1][q];
+        out[q][1] = e1y * o[0][q] - e1x * o[1][q];
+        out[q][2] = -o[2][q];
+    }
 }
 
 // Displacement (north, east, down) at xr (NED) for unit strike slip (uS) and

@@ -115,6 +115,8 @@ void ucg_destroy(ucg_ctx *c)
     hmatrix_free(c);
     if (c->K) cudaFree(c->K);
     if (c->rcv) cudaFree(c->rcv);
+    for (void *w : c->ws)
+        if (w) cudaFree(w);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }

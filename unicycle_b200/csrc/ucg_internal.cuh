@@ -115,6 +115,9 @@ struct Launches {
     long count = 0;
 };
 
+// the assembly workspaces of a context
+enum { WS_SRC = 0, WS_VERT, WS_ID, WS_SIDE, WS_ENDS, WS_EDGE, WS_SCRATCH, WS_COUNT };
+
 }  // namespace ucg
 
 struct ucg_ctx {
@@ -146,6 +149,13 @@ struct ucg_ctx {
 
     // receivers: 12 doubles per element (xc, sv, dv, nv)
     double *rcv = nullptr;
+    size_t rcv_len = 0;
+
+    // assembly workspaces (assemble.cu), kept between calls and freed with the
+    // context: source records, mesh tables and the edge scratch (about 1.2 KB per
+    // triangle and at most 96 MB)
+    void *ws[ucg::WS_COUNT] = {};
+    size_t ws_bytes[ucg::WS_COUNT] = {};
 
     // constitutive parameters (host copies for the state initialisation)
     std::vector<double> hVpl, hrake, hmu0, hsig, ha, hb, hL, hVo, hdamp;
