@@ -376,48 +376,54 @@ __global__ void __launch_bounds__(128) k_assemble_vol(double *__restrict__ K, lo
 
 // ---- dense blocks of K for the hierarchical approximation -------------------------
 //
-// Rows of receivers ridx[0..nrb) (element ids, patches only: 3 traction rows
-// each) against the columns of sources sidx[0..nsb) of one family (2 slip
-// columns each); out is row-major (3 nrb) x (2 nsb).  The same pair kernels as
-// K; the grid's y dimension strides over the receivers.
+// Many blocks in one launch.  A CTA takes one tile, BLOCK_TILE consecutive
+// (receiver, source) pairs of one block in row-major order, so that its threads
+// read the same few source records (kept in the permuted order) from L1 and write
+// consecutive columns.  Patches only: 3 traction rows a receiver, 2 slip columns
+// a source.  One launch per block and pass, as before, left the device waiting
+// for launches: 7,500 blocks at N = 7,200 (build 223 -> 70 ms, 26 ms of it these kernels;
+// N = 20,000: 3.6 s with the old pair kernels -> 0.47 s).
+
+constexpr int BLOCK_TILE = 512;
 
 template <bool R32>
-__global__ void __launch_bounds__(128) k_block_rect(double *__restrict__ out, const int *__restrict__ ridx, int nrb,
-        const int *__restrict__ sidx, int nsb, const double *__restrict__ rcv, const double *__restrict__ src,
-        int ns, OkMed med, double mu, double lambda)
+__global__ void __launch_bounds__(128) k_blocks_rect(const BlockJob *__restrict__ jobs, const int2 *__restrict__ tiles,
+        const int *__restrict__ perm, const double *__restrict__ rcv, const double *__restrict__ src, int ns,
+        OkMed med, double mu, double lambda)
 {
-    const int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jj >= nsb) return;
-    double sr[RS_SIZE];
-    OkDip dp;
-    rect_record(src, ns, __ldg(sidx + jj), sr, dp);
-    const long ld = 2L * nsb;
-    for (int ii = blockIdx.y; ii < nrb; ii += gridDim.y) {
-        const double *rc = rcv + (long)__ldg(ridx + ii) * RC_SIZE;
-        double rloc[RC_SIZE];
+    const int2 tile = tiles[blockIdx.x];
+    const BlockJob J = jobs[tile.x];
+    const int pairs = J.nr * J.ns, last = min(pairs, tile.y + BLOCK_TILE);
+    const long ld = 2L * J.ns;
+    for (int p = tile.y + threadIdx.x; p < last; p += blockDim.x) {
+        const int ii = p / J.ns, jj = p - ii * J.ns;
+        double sr[RS_SIZE], rloc[RC_SIZE], sig[2][6], tS[3], tD[3];
+        OkDip dp;
+        rect_record(src, ns, J.s0 + jj, sr, dp);
+        const double *rc = rcv + (long)__ldg(perm + J.r0 + ii) * RC_SIZE;
 #pragma unroll
         for (int f = 0; f < RC_SIZE; f++) rloc[f] = __ldg(rc + f);
-        double sig[2][6], tS[3], tD[3];
         rect_pair_sig<R32>(sr, dp, rloc[0], rloc[1], rloc[2], med, mu, lambda, sig);
         traction3(rloc, sig[0], tS);
         traction3(rloc, sig[1], tD);
 #pragma unroll
         for (int c = 0; c < 3; c++)
-            *reinterpret_cast<double2 *>(out + (3L * ii + c) * ld + 2L * jj) = make_double2(tS[c], tD[c]);
+            *reinterpret_cast<double2 *>(J.out + (3L * ii + c) * ld + 2L * jj) = make_double2(tS[c], tD[c]);
     }
 }
 
-__global__ void __launch_bounds__(128) k_block_tri(double *__restrict__ out, const int *__restrict__ ridx, int nrb,
-        const int *__restrict__ sidx, int nsb, const double *__restrict__ rcv, TriTables tab, NwConst cst)
+__global__ void __launch_bounds__(128) k_blocks_tri(const BlockJob *__restrict__ jobs, const int2 *__restrict__ tiles,
+        const int *__restrict__ perm, const double *__restrict__ rcv, TriTables tab, NwConst cst)
 {
-    const int jj = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jj >= nsb) return;
-    const int j = __ldg(sidx + jj);
-    const NwRec R{tab.rec + j, (long)tab.ns};
-    const long ld = 2L * nsb;
-    for (int ii = blockIdx.y; ii < nrb; ii += gridDim.y) {
+    const int2 tile = tiles[blockIdx.x];
+    const BlockJob J = jobs[tile.x];
+    const int pairs = J.nr * J.ns, last = min(pairs, tile.y + BLOCK_TILE);
+    const long ld = 2L * J.ns;
+    for (int p = tile.y + threadIdx.x; p < last; p += blockDim.x) {
+        const int ii = p / J.ns, jj = p - ii * J.ns, j = J.s0 + jj;
+        const NwRec R{tab.rec + j, (long)tab.ns};
         double X[3], vs[3], vd[3], vn[3], oS[3], oD[3], bS[3], bD[3];
-        enu_receiver(rcv + (long)__ldg(ridx + ii) * RC_SIZE, X, vs, vd, vn);
+        enu_receiver(rcv + (long)__ldg(perm + J.r0 + ii) * RC_SIZE, X, vs, vd, vn);
         tri_rows<3>(X, vs, vd, vn, R, cst, oS, oD);
         tri_slip(R, bS, bD);
 #pragma unroll 1
@@ -435,7 +441,7 @@ __global__ void __launch_bounds__(128) k_block_tri(double *__restrict__ out, con
         }
 #pragma unroll
         for (int c = 0; c < 3; c++)
-            *reinterpret_cast<double2 *>(out + (3L * ii + c) * ld + 2L * jj) = make_double2(oS[c], oD[c]);
+            *reinterpret_cast<double2 *>(J.out + (3L * ii + c) * ld + 2L * jj) = make_double2(oS[c], oD[c]);
     }
 }
 
@@ -597,36 +603,6 @@ static void build_rect_sources(ucg_ctx *c, int mode, std::vector<double> &s)
     }
 }
 
-// a context workspace of at least `bytes` (its earlier contents are lost)
-template <class T>
-static int workspace(ucg_ctx *c, int which, size_t bytes, T **out)
-{
-    if (c->ws_bytes[which] < bytes) {
-        UCG_CUDA(cudaStreamSynchronize(c->stream));
-        if (c->ws[which]) cudaFree(c->ws[which]);
-        c->ws[which] = nullptr;
-        c->ws_bytes[which] = 0;
-        const cudaError_t e = cudaMalloc(&c->ws[which], bytes);
-        if (e != cudaSuccess) {
-            c->ws[which] = nullptr;
-            return cuda_fail(c, e, "cudaMalloc(assembly workspace)");
-        }
-        c->ws_bytes[which] = bytes;
-    }
-    *out = static_cast<T *>(c->ws[which]);
-    return UCG_OK;
-}
-
-// a host table into a workspace
-template <class T, class H>
-static int upload(ucg_ctx *c, int which, const std::vector<H> &h, T **out)
-{
-    const int rc = workspace(c, which, sizeof(H) * h.size(), out);
-    if (rc) return rc;
-    UCG_CUDA(cudaMemcpyAsync(*out, h.data(), sizeof(H) * h.size(), cudaMemcpyHostToDevice, c->stream));
-    return UCG_OK;
-}
-
 // the receiver table of every element
 static int upload_receivers(ucg_ctx *c)
 {
@@ -643,10 +619,10 @@ static int upload_receivers(ucg_ctx *c)
     return UCG_OK;
 }
 
-// device tables of the triangles; with edges, the
-// unique edges of the mesh by vertex pair, oriented as their first triangle
+// device tables of the triangles (in the order perm, or the mesh's); with edges,
+// the unique edges of the mesh by vertex pair, oriented as their first triangle
 // runs along them, numbered in triangle order so that neighbours stay close
-static int tri_tables_build(ucg_ctx *c, bool edges, TriTables *t)
+static int tri_tables_build(ucg_ctx *c, bool edges, const int *perm, TriTables *t)
 {
     const int ns = c->nt, nve = c->nve;
     *t = TriTables{};
@@ -654,7 +630,7 @@ static int tri_tables_build(ucg_ctx *c, bool edges, TriTables *t)
     std::vector<int> id((size_t)3 * ns);
     const std::vector<int> *ti[3] = {&c->ti1, &c->ti2, &c->ti3};
     for (int k = 0; k < 3; k++)
-        for (int j = 0; j < ns; j++) id[(size_t)k * ns + j] = (*ti[k])[j] - 1;
+        for (int j = 0; j < ns; j++) id[(size_t)k * ns + j] = (*ti[k])[perm ? perm[j] : j] - 1;
     std::vector<int> side((size_t)3 * ns);
     std::vector<int2> ends;
     if (edges) {
@@ -681,14 +657,14 @@ static int tri_tables_build(ucg_ctx *c, bool edges, TriTables *t)
     int *idd, *sd;
     int2 *endd;
     int rc;
-    if ((rc = upload(c, WS_VERT, c->tvert, &vert)) || (rc = upload(c, WS_ID, id, &idd)) ||
+    if ((rc = workspace_upload(c, WS_VERT, c->tvert, &vert)) || (rc = workspace_upload(c, WS_ID, id, &idd)) ||
         (rc = workspace(c, WS_SRC, sizeof(double) * (size_t)NW_SIZE * ns, &rec)))
         return rc;
     t->rec = rec;
     k_tri_prepare<<<(ns + 127) / 128, 128, 0, c->stream>>>(vert, idd, ns, rec);
     c->launches.count++;
     if (edges) {
-        if ((rc = upload(c, WS_SIDE, side, &sd)) || (rc = upload(c, WS_ENDS, ends, &endd)) ||
+        if ((rc = workspace_upload(c, WS_SIDE, side, &sd)) || (rc = workspace_upload(c, WS_ENDS, ends, &endd)) ||
             (rc = workspace(c, WS_EDGE, sizeof(double) * (size_t)NE_SIZE * t->ne, &ed)))
             return rc;
         t->edge = sd;
@@ -794,7 +770,7 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     if (c->nr) {
         std::vector<double> s;
         build_rect_sources(c, okada_mode, s);
-        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
+        if ((rc = workspace_upload(c, WS_SRC, s, &dsrc))) return rc;
         UCG_CUDA(cudaEventRecord(ev[0], c->stream));
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         const double alpha = okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d;
@@ -811,7 +787,7 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     }
     if (c->nt) {
         TriTables tab;
-        if ((rc = tri_tables_build(c, true, &tab))) return rc;
+        if ((rc = tri_tables_build(c, true, nullptr, &tab))) return rc;
         UCG_CUDA(cudaEventRecord(ev[2], c->stream));
         const NwConst cst{c->lambda / (c->lambda + c->mu) / 2.0, c->mu, c->lambda};
         rc = assemble_tri_rows<3>(c, n, 0, np, 0, tab, cst);
@@ -822,7 +798,7 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     if (c->nv) {
         std::vector<double> s;
         build_vol_sources(c, s);
-        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
+        if ((rc = workspace_upload(c, WS_SRC, s, &dsrc))) return rc;
         UCG_CUDA(cudaEventRecord(ev[4], c->stream));
         const double nu = c->lambda / (c->lambda + c->mu) / 2.0;
         dim3 grid((c->nv + TPB - 1) / TPB, gy);
@@ -878,7 +854,7 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     if (c->nr) {
         std::vector<double> s;
         build_rect_sources(c, okada_mode, s);
-        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
+        if ((rc = workspace_upload(c, WS_SRC, s, &dsrc))) return rc;
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         const double alpha = okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d;
         dim3 grid((c->nr + TPB - 1) / TPB, gy);
@@ -891,7 +867,7 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     }
     if (c->nt) {
         TriTables tab;
-        if ((rc = tri_tables_build(c, false, &tab))) return rc;
+        if ((rc = tri_tables_build(c, false, nullptr, &tab))) return rc;
         dim3 grid((c->nt + TPB - 1) / TPB, gy);
         k_observe_tri<<<grid, TPB, 0, c->stream>>>(c->O, n, 2L * c->nr, c->obs_dev, nobs, tab.rec, c->nt,
                                                    c->lambda / (c->lambda + c->mu) / 2.0);
@@ -901,7 +877,7 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
     if (c->nv) {
         std::vector<double> s;
         build_vol_sources(c, s);
-        if ((rc = upload(c, WS_SRC, s, &dsrc))) return rc;
+        if ((rc = workspace_upload(c, WS_SRC, s, &dsrc))) return rc;
         dim3 grid((c->nv + TPB - 1) / TPB, gy);
         k_observe_vol<<<grid, TPB, 0, c->stream>>>(c->O, n, 2L * np, c->obs_dev, nobs, dsrc, c->nv, c->mu,
                                                    c->lambda / (c->lambda + c->mu) / 2.0);
@@ -919,48 +895,60 @@ int assemble_observation(ucg_ctx *c, int okada_mode)
 
 // ---- block sources (hierarchical approximation) -----------------------------------
 
-int block_sources_build(ucg_ctx *c, int okada_mode, BlockSources *bs)
+int block_family(const ucg_ctx *c)
 {
-    if ((c->nr > 0) == (c->nt > 0) || c->nv > 0) return UCG_E_UNSUPPORTED;   // one patch family
-    UCG_CUDA(cudaSetDevice(c->device));
-    int rc = upload_receivers(c);
+    return (c->nr > 0) == (c->nt > 0) || c->nv > 0 ? UCG_E_UNSUPPORTED : UCG_OK;
+}
+
+int block_sources_build(ucg_ctx *c, int okada_mode, const std::vector<int> &perm, BlockSources *bs)
+{
+    int rc = block_family(c);
     if (rc) return rc;
-    std::vector<double> s;
+    UCG_CUDA(cudaSetDevice(c->device));
+    if ((rc = upload_receivers(c))) return rc;
     bs->family = c->nr > 0 ? 0 : 1;
     bs->okada_mode = okada_mode;
-    if (bs->family == 0) {
-        build_rect_sources(c, okada_mode, s);
-        bs->ns = c->nr;
-        const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
-        bs->med = ok_med(okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d);
-    } else {
+    if (bs->family == 1) {
         bs->ns = c->nt;
         bs->cst = NwConst{c->lambda / (c->lambda + c->mu) / 2.0, c->mu, c->lambda};
-        return tri_tables_build(c, true, &bs->tri);
+        return tri_tables_build(c, true, perm.data(), &bs->tri);
     }
+    std::vector<double> s, sp;
+    build_rect_sources(c, okada_mode, s);
+    bs->ns = c->nr;
+    sp.resize(s.size());
+    for (int f = 0; f < RS_SIZE; f++)
+        for (int j = 0; j < c->nr; j++) sp[(size_t)f * c->nr + j] = s[(size_t)f * c->nr + perm[j]];
+    const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
+    bs->med = ok_med(okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d);
     double *src;
-    if ((rc = upload(c, WS_SRC, s, &src))) return rc;
+    if ((rc = workspace_upload(c, WS_SRC, sp, &src))) return rc;
     bs->src = src;
     return UCG_OK;
 }
 
-void assemble_block(ucg_ctx *c, const BlockSources &bs, const int *ridx, int nrb, const int *sidx, int nsb,
-                    double *out)
+int assemble_blocks(ucg_ctx *c, const BlockSources &bs, const int *perm_d, const std::vector<BlockJob> &jobs)
 {
-    const int TPB = 128;
-    dim3 grid((nsb + TPB - 1) / TPB, nrb < 65535 ? nrb : 65535);
-    if (bs.family == 0) {
-        if (bs.okada_mode == UCG_OKADA_REF32IO)
-            k_block_rect<true><<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.src, bs.ns,
-                                                           bs.med, c->mu, c->lambda);
-        else
-            k_block_rect<false><<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.src, bs.ns,
-                                                            bs.med, c->mu, c->lambda);
-        c->launches.count++;
-    } else {
-        k_block_tri<<<grid, TPB, 0, c->stream>>>(out, ridx, nrb, sidx, nsb, c->rcv, bs.tri, bs.cst);
-        c->launches.count++;
+    if (jobs.empty()) return UCG_OK;
+    std::vector<int2> tiles;
+    for (size_t q = 0; q < jobs.size(); q++) {
+        const int pairs = jobs[q].nr * jobs[q].ns;
+        for (int p = 0; p < pairs; p += BLOCK_TILE) tiles.push_back(make_int2((int)q, p));
     }
+    BlockJob *jd;
+    int2 *td;
+    int rc;
+    if ((rc = workspace_upload(c, WS_JOBS, jobs, &jd)) || (rc = workspace_upload(c, WS_TILES, tiles, &td))) return rc;
+    const int grid = (int)tiles.size(), TPB = 128;
+    if (bs.family == 1)
+        k_blocks_tri<<<grid, TPB, 0, c->stream>>>(jd, td, perm_d, c->rcv, bs.tri, bs.cst);
+    else if (bs.okada_mode == UCG_OKADA_REF32IO)
+        k_blocks_rect<true><<<grid, TPB, 0, c->stream>>>(jd, td, perm_d, c->rcv, bs.src, bs.ns, bs.med, c->mu, c->lambda);
+    else
+        k_blocks_rect<false><<<grid, TPB, 0, c->stream>>>(jd, td, perm_d, c->rcv, bs.src, bs.ns, bs.med, c->mu, c->lambda);
+    c->launches.count++;
+    UCG_CUDA(cudaGetLastError());
+    return UCG_OK;
 }
 
 // element bounding boxes (lo[3], hi[3] per element, patches in K's order) and centres

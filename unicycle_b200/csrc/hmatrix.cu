@@ -16,7 +16,7 @@
 //              not admissible dense blocks, other pairs are split (the non-leaf
 //              side, or both).
 //   build      each block is assembled densely on the device into scratch by the
-//              same pair kernels as K (assemble_block), so K itself is never
+//              same pair kernels as K (assemble_blocks), so K itself is never
 //              held: N beyond what a dense K fits in HBM works.  A low-rank
 //              block is compressed by adaptive cross approximation with partial
 //              pivoting (one CTA per block) to relative accuracy eps, then
@@ -378,13 +378,48 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double 
     }
 }
 
-// row-major m x n -> column-major
-__global__ void k_to_colmajor(const double *__restrict__ a, int m, int n, double *__restrict__ b)
+// What a batch keeps, in one launch: copies of the factors and column-major
+// copies of the dense blocks.  A CTA takes KEEP_TILE values of one job.
+struct KeepJob {
+    const double *src;   // row-major m x n
+    double *dst;
+    int m, n;
+    int transpose;
+};
+
+constexpr int KEEP_TILE = 4096;
+
+__global__ void __launch_bounds__(256) k_keep(const KeepJob *__restrict__ jobs, const int2 *__restrict__ tiles)
 {
-    const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long)m * n) return;
-    const long j = t / m, i = t % m;
-    b[t] = a[i * n + j];
+    const int2 tile = tiles[blockIdx.x];
+    const KeepJob J = jobs[tile.x];
+    const long tot = (long)J.m * J.n, t0 = (long)tile.y * KEEP_TILE, t1 = min(tot, t0 + KEEP_TILE);
+    for (long t = t0 + threadIdx.x; t < t1; t += blockDim.x) {
+        if (J.transpose) {
+            const long j = t / J.m, i = t - j * J.m;
+            J.dst[t] = J.src[i * J.n + j];
+        } else {
+            J.dst[t] = J.src[t];
+        }
+    }
+}
+
+int keep_blocks(ucg_ctx *c, const std::vector<KeepJob> &jobs)
+{
+    if (jobs.empty()) return UCG_OK;
+    std::vector<int2> tiles;
+    for (size_t q = 0; q < jobs.size(); q++) {
+        const long n = ((long)jobs[q].m * jobs[q].n + KEEP_TILE - 1) / KEEP_TILE;
+        for (long t = 0; t < n; t++) tiles.push_back(make_int2((int)q, (int)t));
+    }
+    KeepJob *jd;
+    int2 *td;
+    int rc;
+    if ((rc = workspace_upload(c, WS_JOBS, jobs, &jd)) || (rc = workspace_upload(c, WS_TILES, tiles, &td))) return rc;
+    k_keep<<<(int)tiles.size(), 256, 0, c->stream>>>(jd, td);
+    c->launches.count++;
+    UCG_CUDA(cudaGetLastError());
+    return UCG_OK;
 }
 
 // ---- the product --------------------------------------------------------------------
@@ -716,7 +751,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     hmatrix_free(c);
     const int np = c->nr + c->nt;
     BlockSources bs;
-    int rc = block_sources_build(c, okada_mode, &bs);
+    int rc = block_family(c);
     if (rc) {
         c->err = "hierarchical matrix: one patch family (rectangles or triangles) and no volumes";
         return rc;
@@ -753,6 +788,8 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     for (int L = 0; L < h->n_leaves; L++) h->max_leaf = std::max(h->max_leaf, leaf_e0[L + 1] - leaf_e0[L]);
     UCG_CUDA(cudaMalloc(&h->perm_d, sizeof(int) * np));
     UCG_CUDA(cudaMemcpy(h->perm_d, h->perm.data(), sizeof(int) * np, cudaMemcpyHostToDevice));
+
+    if ((rc = block_sources_build(c, okada_mode, h->perm, &bs))) return rc;
 
     double *sc = nullptr;
     UCG_CUDA(cudaMalloc(&sc, scratch));
@@ -804,10 +841,14 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     size_t bi = 0;
     std::vector<AcaJob> jobs;
     std::vector<int> job_block;
+    std::vector<BlockJob> build;
+    std::vector<KeepJob> keep;
     while (bi < blocks.size()) {
         size_t off = 0;   // in doubles
         jobs.clear();
         job_block.clear();
+        build.clear();
+        keep.clear();
         std::vector<std::pair<int, size_t>> dense_in_batch;
         while (bi < blocks.size() && (int)jobs.size() < MAXJOBS) {
             const HBlock &B = blocks[bi];
@@ -824,7 +865,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
                 break;
             }
             double *Bd = sc + off;
-            assemble_block(c, bs, h->perm_d + B.r0, B.r1 - B.r0, h->perm_d + B.s0, B.s1 - B.s0, Bd);
+            build.push_back({Bd, B.r0, B.r1 - B.r0, B.s0, B.s1 - B.s0});
             if (B.lowrank) {
                 AcaJob J;
                 J.B = Bd;
@@ -844,9 +885,9 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
             off += need;
             bi++;
         }
-        if ((rc = (int)cudaGetLastError())) {
+        if ((rc = assemble_blocks(c, bs, h->perm_d, build))) {
             cleanup();
-            return cuda_fail(c, (cudaError_t)rc, "hierarchical matrix block assembly");
+            return rc;
         }
         std::vector<int> ranks(jobs.size());
         if (!jobs.empty()) {
@@ -867,9 +908,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
             double *d = nullptr;
             int r = store(1, sizeof(double) * (size_t)m * n, &d);
             if (r) return r;
-            const long tot = (long)m * n;
-            k_to_colmajor<<<(int)((tot + 255) / 256), 256, 0, c->stream>>>(src, m, n, d);
-            c->launches.count++;
+            keep.push_back({src, d, m, n, 1});
             h->bytes += sizeof(double) * (size_t)m * n;
             done.push_back({b, -1, d, nullptr});
             return UCG_OK;
@@ -898,13 +937,17 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
                 return rc;
             }
             if (k > 0) {
-                cudaMemcpyAsync(U, J.U, sizeof(double) * (size_t)k * J.m, cudaMemcpyDeviceToDevice, c->stream);
-                cudaMemcpyAsync(V, J.V, sizeof(double) * (size_t)k * J.n, cudaMemcpyDeviceToDevice, c->stream);
+                keep.push_back({J.U, U, k, J.m, 0});
+                keep.push_back({J.V, V, k, J.n, 0});
             }
             h->bytes += sizeof(double) * (size_t)k * (J.m + J.n);
             h->n_lowrank++;
             h->max_rank = std::max(h->max_rank, k);
             done.push_back({b, k, U, V});
+        }
+        if ((rc = keep_blocks(c, keep))) {
+            cleanup();
+            return rc;
         }
         e = cudaStreamSynchronize(c->stream);   // the scratch is reused by the next batch
         if (e != cudaSuccess) {

@@ -116,7 +116,7 @@ struct Launches {
 };
 
 // the assembly workspaces of a context
-enum { WS_SRC = 0, WS_VERT, WS_ID, WS_SIDE, WS_ENDS, WS_EDGE, WS_SCRATCH, WS_COUNT };
+enum { WS_SRC = 0, WS_VERT, WS_ID, WS_SIDE, WS_ENDS, WS_EDGE, WS_SCRATCH, WS_JOBS, WS_TILES, WS_COUNT };
 
 }  // namespace ucg
 
