@@ -107,3 +107,30 @@ def test_coupled_postseismic_relaxation_runs(ucg, small_cfg3):
     assert np.all(np.isfinite(y)) and steps > 10 and t > 0
     assert s1 < s0          # relaxation of the coseismic stress change
     sim.close()
+
+
+@pytest.mark.parametrize("nvol,npatch,q3", [(1, 0, 4.0e3), (1, 1, 0.0), (130, 3, 20.0e3), (9, 129, 15.0e3)])
+def test_volume_columns_at_tile_edges(ucg, oracle_lib, nvol, npatch, q3):
+    """The corner sums of the volume assembly with one cuboid alone (every value at
+    its own centre), a cuboid that reaches the surface, source counts that end
+    inside a CTA, rotated cuboids of unequal sides.  Tolerance: the oracle's
+    numerical derivative of the same integrals, 3e-8 as above."""
+    rng = np.random.default_rng(nvol + npatch)
+    size = rng.uniform(1.5e3, 4.0e3, (nvol, 3))
+    x = np.stack([rng.uniform(-4e4, 4e4, nvol), rng.uniform(-4e4, 4e4, nvol), q3 + rng.uniform(0, 2e4, nvol)], 1)
+    x[:, 2] = x[:, 2] if q3 else 0.0
+    vol = (x, size[:, 0], size[:, 1], size[:, 2], rng.uniform(0, 6.0, nvol))
+    sim = ucg.Simulation(3.0e4, 2.6e4, driver="viscouscycles")
+    rect = None
+    if npatch:
+        rect = (np.stack([rng.uniform(-4e4, 4e4, npatch), rng.uniform(-4e4, 4e4, npatch), rng.uniform(0, 9e3, npatch)],
+                         1), np.full(npatch, 900.0), np.full(npatch, 700.0), rng.uniform(0, 6, npatch),
+                rng.uniform(0.3, 1.5, npatch))
+        sim.set_rectangles(*rect)
+    sim.set_volumes(*vol)
+    sim.buildG()
+    K = sim.copy_G()[:, 2 * npatch:]
+    sim.close()
+    ref = oracle_lib.Mesh(3.0e4, 2.6e4, rect=rect, vol=vol).build_g()[:, 2 * npatch:]
+    assert np.all(np.isfinite(ref)) and np.all(np.isfinite(K))
+    assert _elem_err(K, ref, [3] * npatch + [6] * nvol) < 3e-8

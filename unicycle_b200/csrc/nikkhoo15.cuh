@@ -24,6 +24,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include "dual.cuh"
+#include "rows.cuh"
 
 namespace ucg {
 
@@ -468,39 +469,6 @@ __device__ inline void nw_side(const Dd X[3], const NwRec &R, int o, double nu, 
 
 // ---- stress of a pair ----------------------------------------------------------
 
-// Receiver rows.  r: the receiver's record (NED: centre, strike, dip, normal);
-// rows are the 3 tractions (ts, td, tn) of a patch or the 6 stresses (s11, s12,
-// s13, s22, s23, s33 in the element's frame) of a volume, formed from a stress
-// given in a frame where the receiver's unit vectors are vs, vd, vn.
-template <int NR>
-__device__ __forceinline__ void nw_rows(const double vs[3], const double vd[3], const double vn[3], double sxx,
-                                        double sxy, double sxz, double syy, double syz, double szz, double o[NR])
-{
-    const double t0 = sxx * vn[0] + sxy * vn[1] + sxz * vn[2];
-    const double t1 = sxy * vn[0] + syy * vn[1] + syz * vn[2];
-    const double t2 = sxz * vn[0] + syz * vn[1] + szz * vn[2];
-    if (NR == 3) {
-        // okada92.f90:390-398
-        o[0] = t0 * vs[0] + t1 * vs[1] + t2 * vs[2];
-        o[1] = t0 * vd[0] + t1 * vd[1] + t2 * vd[2];
-        o[2] = t0 * vn[0] + t1 * vn[1] + t2 * vn[2];
-    } else {
-        // okada92.f90:445-462 (the third axis is the dip vector negated)
-        const double a0 = sxx * vs[0] + sxy * vs[1] + sxz * vs[2];
-        const double a1 = sxy * vs[0] + syy * vs[1] + syz * vs[2];
-        const double a2 = sxz * vs[0] + syz * vs[1] + szz * vs[2];
-        const double b0 = sxx * vd[0] + sxy * vd[1] + sxz * vd[2];
-        const double b1 = sxy * vd[0] + syy * vd[1] + syz * vd[2];
-        const double b2 = sxz * vd[0] + syz * vd[1] + szz * vd[2];
-        o[0] = a0 * vs[0] + a1 * vs[1] + a2 * vs[2];
-        o[1] = t0 * vs[0] + t1 * vs[1] + t2 * vs[2];
-        o[2 % NR] = -(b0 * vs[0] + b1 * vs[1] + b2 * vs[2]);
-        o[3 % NR] = t0 * vn[0] + t1 * vn[1] + t2 * vn[2];
-        o[4 % NR] = -(t0 * vd[0] + t1 * vd[1] + t2 * vd[2]);
-        o[5 % NR] = b0 * vd[0] + b1 * vd[1] + b2 * vd[2];
-    }
-}
-
 // Strain of the angular dislocation of one TD corner, added to the TD-frame
 // strain (xx, 2xy, 2xz, yy, 2yz, zz) of the strike (by = 1) and dip (bz = -1)
 // modes, all over k = 1 / (8 pi (1 - nu)).  (ga, de) are the cosine and sine
@@ -622,7 +590,7 @@ __device__ __forceinline__ bool nw_td_rows(const double X[3], const double vs[3]
         double *out = t ? oD : oS;
         const double tr = la * (e[0] + e[3] + e[5]);
         double v[NR];
-        nw_rows<NR>(w[0], w[1], w[2], fl * (2.0 * mu * e[0] + tr), fl * mu * e[1], mu * e[2], 2.0 * mu * e[3] + tr,
+        receiver_rows<NR>(w[0], w[1], w[2], fl * (2.0 * mu * e[0] + tr), fl * mu * e[1], mu * e[2], 2.0 * mu * e[3] + tr,
                     mu * e[4], 2.0 * mu * e[5] + tr, v);
 #pragma unroll
         for (int q = 0; q < NR; q++) out[q] += v[q];
@@ -797,7 +765,7 @@ __device__ __forceinline__ void nw_edge_rows(const double X[3], const double vs[
 #pragma unroll
     for (int b = 0; b < 3; b++) {
         const double tr = la * (E[b][0] + E[b][3] + E[b][5]);
-        nw_rows<NR>(w0, w1, w2, 2.0 * mu * E[b][0] + tr, mu * E[b][1], mu * E[b][2], 2.0 * mu * E[b][3] + tr,
+        receiver_rows<NR>(w0, w1, w2, 2.0 * mu * E[b][0] + tr, mu * E[b][1], mu * E[b][2], 2.0 * mu * E[b][3] + tr,
                     mu * E[b][4], 2.0 * mu * E[b][5] + tr, o[b]);
     }
 #pragma unroll
