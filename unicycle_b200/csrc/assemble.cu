@@ -30,85 +30,17 @@ namespace ucg {
 // receiver record: xc[3], sv[3], dv[3], nv[3]
 enum { RC_X = 0, RC_S = 3, RC_D = 6, RC_N = 9, RC_SIZE = 12 };
 
-__device__ __forceinline__ void traction3(const double *r, const double s[6], double t[3])
+// the NR rows of a receiver record from a stress (s11, s12, s13, s22, s23, s33)
+template <int NR>
+__device__ __forceinline__ void ned_rows(const double *r, const double s[6], double o[NR])
 {
-    // okada92.f90:390-398
-    const double n0 = r[RC_N], n1 = r[RC_N + 1], n2 = r[RC_N + 2];
-    const double a = n0 * s[0] + n1 * s[1] + n2 * s[2];
-    const double b = n0 * s[1] + n1 * s[3] + n2 * s[4];
-    const double c = n0 * s[2] + n1 * s[4] + n2 * s[5];
-    t[0] = a * r[RC_S] + b * r[RC_S + 1] + c * r[RC_S + 2];
-    t[1] = a * r[RC_D] + b * r[RC_D + 1] + c * r[RC_D + 2];
-    t[2] = a * n0 + b * n1 + c * n2;
-}
-
-__device__ __forceinline__ void stress6(const double *r, const double s[6], double o[6])
-{
-    // okada92.f90:445-462
-    const double *sv = r + RC_S, *dv = r + RC_D, *nv = r + RC_N;
-    const double sa = sv[0] * s[0] + sv[1] * s[1] + sv[2] * s[2];
-    const double sb = sv[0] * s[1] + sv[1] * s[3] + sv[2] * s[4];
-    const double sc = sv[0] * s[2] + sv[1] * s[4] + sv[2] * s[5];
-    const double na = nv[0] * s[0] + nv[1] * s[1] + nv[2] * s[2];
-    const double nb = nv[0] * s[1] + nv[1] * s[3] + nv[2] * s[4];
-    const double nc = nv[0] * s[2] + nv[1] * s[4] + nv[2] * s[5];
-    const double da = -dv[0] * s[0] - dv[1] * s[1] - dv[2] * s[2];
-    const double db = -dv[0] * s[1] - dv[1] * s[3] - dv[2] * s[4];
-    const double dc = -dv[0] * s[2] - dv[1] * s[4] - dv[2] * s[5];
-    o[0] = sa * sv[0] + sb * sv[1] + sc * sv[2];
-    o[1] = sa * nv[0] + sb * nv[1] + sc * nv[2];
-    o[2] = -sa * dv[0] - sb * dv[1] - sc * dv[2];
-    o[3] = na * nv[0] + nb * nv[1] + nc * nv[2];
-    o[4] = -na * dv[0] - nb * dv[1] - nc * dv[2];
-    o[5] = -da * dv[0] - db * dv[1] - dc * dv[2];
-}
-
-struct RcvInfo {
-    long row;   // first row of K
-    int nrow;   // 3 (patch) or 6 (volume)
-};
-
-__device__ __forceinline__ RcvInfo rcv_info(int e, int np)
-{
-    RcvInfo ri;
-    if (e < np) { ri.row = 3L * e; ri.nrow = 3; }
-    else { ri.row = 3L * np + 6L * (e - np); ri.nrow = 6; }
-    return ri;
-}
-
-// write (ACC = false) or add (ACC = true) the 2 slip columns, one double2 per
-// row, of a patch source
-template <bool ACC = false>
-__device__ __forceinline__ void store_patch_source(double *K, long n, long col, const double *rc,
-                                                   const RcvInfo &ri, const double sS[6],
-                                                   const double sD[6])
-{
-    double oS[6], oD[6];
-    if (ri.nrow == 3) {
-        traction3(rc, sS, oS);
-        traction3(rc, sD, oD);
-    } else {
-        stress6(rc, sS, oS);
-        stress6(rc, sD, oD);
-    }
-#pragma unroll
-    for (int c = 0; c < 6; c++) {
-        if (c < ri.nrow) {
-            double2 *p = reinterpret_cast<double2 *>(K + (ri.row + c) * n + col);
-            if (ACC) {
-                const double2 o = *p;
-                *p = make_double2(o.x + oS[c], o.y + oD[c]);
-            } else {
-                *p = make_double2(oS[c], oD[c]);
-            }
-        }
-    }
+    receiver_rows<NR>(r + RC_S, r + RC_D, r + RC_N, s[0], s[1], s[2], s[3], s[4], s[5], o);
 }
 
 // ---- rectangles (Okada 1992) -------------------------------------------------
 
 enum { RS_Q1 = 0, RS_Q2, RS_CS, RS_SS, RS_DEPTH, RS_AL2, RS_AW1, RS_SD, RS_CD, RS_SDSD, RS_CDCD,
-       RS_SDCD, RS_SIZE };
+       RS_SDCD, RS_ICD, RS_SIZE };
 
 // Stress (s11, s12, s13, s22, s23, s33 for strike and dip slip) at receiver
 // point (x1, x2, x3) of one rectangle record sr (okada92.f90:121-205).
@@ -161,26 +93,36 @@ __device__ __forceinline__ void rect_record(const double *__restrict__ src, int 
     for (int f = 0; f < RS_SIZE; f++) sr[f] = __ldg(src + (long)f * ns + j);
     dp.sd = sr[RS_SD]; dp.cd = sr[RS_CD]; dp.sdsd = sr[RS_SDSD]; dp.cdcd = sr[RS_CDCD];
     dp.sdcd = sr[RS_SDCD];
+    dp.icd = sr[RS_ICD];
 }
 
-template <bool R32>
-__global__ void __launch_bounds__(128) k_assemble_rect(double *__restrict__ K, long n, long col0,
-        const double *__restrict__ rcv, int nrcv, int np, const double *__restrict__ src, int ns,
-        OkMed med, double mu, double lambda)
+// Bound by the FP64 pipe.  Divisions were 60 of a corner's operations and each is
+// a sequence of its own with a branch, which kept the warps waiting (28 % of the
+// pipe's cycles); four reciprocals a corner are left, parts A and B of the image
+// share their terms and the real source is rotated once, after its corner sum.
+// 2,048 rectangles on as many receivers: 3.21 -> 0.93 ms (65 % of the pipe, 240
+// registers, 8 warps an SM).
+template <bool R32, int NR>
+__global__ void __launch_bounds__(128) k_assemble_rect(double *__restrict__ K, long n, long row0,
+        const double *__restrict__ rcv, int r0, int r1, const double *__restrict__ src, int ns, OkMed med, double mu,
+        double lambda)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= ns) return;
     double sr[RS_SIZE];
     OkDip dp;
     rect_record(src, ns, j, sr, dp);
-    for (int e = blockIdx.y; e < nrcv; e += gridDim.y) {
+    for (int e = r0 + blockIdx.y; e < r1; e += gridDim.y) {
         const double *rc = rcv + (long)e * RC_SIZE;
-        double sig[2][6];
+        double sig[2][6], rloc[RC_SIZE], oS[NR], oD[NR];
         rect_pair_sig<R32>(sr, dp, __ldg(rc + 0), __ldg(rc + 1), __ldg(rc + 2), med, mu, lambda, sig);
-        double rloc[RC_SIZE];
 #pragma unroll
         for (int f = 0; f < RC_SIZE; f++) rloc[f] = __ldg(rc + f);
-        store_patch_source(K, n, col0 + 2L * j, rloc, rcv_info(e, np), sig[0], sig[1]);
+        ned_rows<NR>(rloc, sig[0], oS);
+        ned_rows<NR>(rloc, sig[1], oD);
+#pragma unroll
+        for (int c = 0; c < NR; c++)
+            *reinterpret_cast<double2 *>(K + (row0 + (long)NR * (e - r0) + c) * n + 2L * j) = make_double2(oS[c], oD[c]);
     }
 }
 
@@ -390,8 +332,8 @@ __global__ void __launch_bounds__(128) k_blocks_rect(const BlockJob *__restrict_
 #pragma unroll
         for (int f = 0; f < RC_SIZE; f++) rloc[f] = __ldg(rc + f);
         rect_pair_sig<R32>(sr, dp, rloc[0], rloc[1], rloc[2], med, mu, lambda, sig);
-        traction3(rloc, sig[0], tS);
-        traction3(rloc, sig[1], tD);
+        ned_rows<3>(rloc, sig[0], tS);
+        ned_rows<3>(rloc, sig[1], tD);
 #pragma unroll
         for (int c = 0; c < 3; c++)
             *reinterpret_cast<double2 *>(J.out + (3L * ii + c) * ld + 2L * jj) = make_double2(tS[c], tD[c]);
@@ -451,6 +393,7 @@ __global__ void __launch_bounds__(128) k_observe_rect(double *__restrict__ O, lo
     OkDip dp;
     dp.sd = sr[RS_SD]; dp.cd = sr[RS_CD]; dp.sdsd = sr[RS_SDSD]; dp.cdcd = sr[RS_CDCD];
     dp.sdcd = sr[RS_SDCD];
+    dp.icd = sr[RS_ICD];
     const double csst = sr[RS_CS], ssst = sr[RS_SS];
     for (int k = blockIdx.y; k < nobs; k += gridDim.y) {
         const double x1 = __ldg(obs + 3L * k), x2 = __ldg(obs + 3L * k + 1), x3 = __ldg(obs + 3L * k + 2);
@@ -586,6 +529,7 @@ static void build_rect_sources(ucg_ctx *c, int mode, std::vector<double> &s)
         put(RS_SDSD, j, dp.sdsd);
         put(RS_CDCD, j, dp.cdcd);
         put(RS_SDCD, j, dp.sdcd);
+        put(RS_ICD, j, dp.icd);
     }
 }
 
@@ -733,7 +677,6 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     if (rc) return rc;
 
     const int TPB = 128;
-    const int gy = ne < 65535 ? ne : 65535;
     double *dsrc = nullptr;
     // device time of each family's launches (ucg_assembly_times)
     cudaEvent_t ev[6];
@@ -742,8 +685,11 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     // load the kernels' code before the first event: under lazy module loading
     // a first launch would otherwise count the load in its family's time
     cudaFuncAttributes fa;
-    if (c->nr) UCG_CUDA(okada_mode == UCG_OKADA_REF32IO ? cudaFuncGetAttributes(&fa, k_assemble_rect<true>)
-                                                        : cudaFuncGetAttributes(&fa, k_assemble_rect<false>));
+    if (c->nr) {
+        const bool r32 = okada_mode == UCG_OKADA_REF32IO;
+        UCG_CUDA(cudaFuncGetAttributes(&fa, r32 ? k_assemble_rect<true, 3> : k_assemble_rect<false, 3>));
+        if (c->nv) UCG_CUDA(cudaFuncGetAttributes(&fa, r32 ? k_assemble_rect<true, 6> : k_assemble_rect<false, 6>));
+    }
     if (c->nt) {
         UCG_CUDA(cudaFuncGetAttributes(&fa, k_tri_edges<3>));
         UCG_CUDA(cudaFuncGetAttributes(&fa, k_assemble_tri<3>));
@@ -763,14 +709,16 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
         UCG_CUDA(cudaEventRecord(ev[0], c->stream));
         const double alpha_d = (c->lambda + c->mu) / (c->lambda + 2.0 * c->mu);
         const double alpha = okada_mode == UCG_OKADA_REF32IO ? (double)f32(alpha_d) : alpha_d;
-        dim3 grid((c->nr + TPB - 1) / TPB, gy);
-        if (okada_mode == UCG_OKADA_REF32IO)
-            k_assemble_rect<true><<<grid, TPB, 0, c->stream>>>(c->K, n, 0, c->rcv, ne, np, dsrc, c->nr,
-                                                              ok_med(alpha), c->mu, c->lambda);
-        else
-            k_assemble_rect<false><<<grid, TPB, 0, c->stream>>>(c->K, n, 0, c->rcv, ne, np, dsrc, c->nr,
-                                                               ok_med(alpha), c->mu, c->lambda);
-        c->launches.count++;
+        const int xb = (c->nr + TPB - 1) / TPB;
+        const OkMed med = ok_med(alpha);
+        auto rows = [&](auto kern, int e0, int e1, long row0) {
+            kern<<<dim3(xb, receiver_grid(c, xb, e1 - e0)), TPB, 0, c->stream>>>(c->K, n, row0, c->rcv, e0, e1, dsrc,
+                                                                                c->nr, med, c->mu, c->lambda);
+            c->launches.count++;
+        };
+        const bool r32 = okada_mode == UCG_OKADA_REF32IO;
+        rows(r32 ? k_assemble_rect<true, 3> : k_assemble_rect<false, 3>, 0, np, 0);
+        if (c->nv) rows(r32 ? k_assemble_rect<true, 6> : k_assemble_rect<false, 6>, np, ne, 3L * np);
         UCG_CUDA(cudaGetLastError());
         UCG_CUDA(cudaEventRecord(ev[1], c->stream));
     }

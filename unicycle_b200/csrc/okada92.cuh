@@ -23,6 +23,7 @@ namespace ucg {
 
 struct OkDip {           // DCCON0 (dc3d.f:509-544)
     double sd, cd, sdsd, cdcd, sdcd;
+    double icd;              // 1 / cd where cd is not 0
 };
 
 struct OkMed {           // medium constants alp1..alp5
@@ -31,7 +32,8 @@ struct OkMed {           // medium constants alp1..alp5
 
 struct OkCorner {        // DCCON2 outputs (dc3d.f:596-665)
     double xi, et, q;
-    double xi2, et2, q2, r, r2, r3, r5, y, d, x11, y11, x32, y32;
+    double xi2, et2, q2, r, r2, y, d, x11, y11, x32, y32;
+    double ir, ir2, ir3, ir5;   // reciprocal powers of r
     double ey, ez, fy, fz, gy, gz, hy, hz;
 };
 
@@ -49,6 +51,7 @@ __host__ __device__ inline OkDip ok_dip(double dip_deg)
     c.sdsd = c.sd * c.sd;
     c.cdcd = c.cd * c.cd;
     c.sdcd = c.sd * c.cd;
+    c.icd = c.cd != 0.0 ? 1.0 / c.cd : 0.0;
     return c;
 }
 
@@ -79,8 +82,10 @@ __device__ inline bool ok_corner(double &xi, double &et, double &q, const OkDip 
     c.r2 = c.xi2 + c.et2 + c.q2;
     c.r = sqrt(c.r2);
     if (c.r == 0.0) return false;
-    c.r3 = c.r * c.r2;
-    c.r5 = c.r3 * c.r2;
+    c.ir = 1.0 / c.r;
+    c.ir2 = c.ir * c.ir;
+    c.ir3 = c.ir * c.ir2;
+    c.ir5 = c.ir3 * c.ir2;
     c.y = et * dp.cd + q * dp.sd;
     c.d = et * dp.sd - q * dp.cd;
     // tt, alx and ale enter only the displacement entries of parts A/B/C, which the
@@ -91,7 +96,7 @@ __device__ inline bool ok_corner(double &xi, double &et, double &q, const OkDip 
     } else {
         double rxi = c.r + xi;
         c.x11 = 1.0 / (c.r * rxi);
-        c.x32 = (c.r + rxi) * c.x11 * c.x11 / c.r;
+        c.x32 = (c.r + rxi) * c.x11 * c.x11 * c.ir;
     }
     if (ket == 1) {
         c.y11 = 0.0;
@@ -99,12 +104,12 @@ __device__ inline bool ok_corner(double &xi, double &et, double &q, const OkDip 
     } else {
         double ret = c.r + et;
         c.y11 = 1.0 / (c.r * ret);
-        c.y32 = (c.r + ret) * c.y11 * c.y11 / c.r;
+        c.y32 = (c.r + ret) * c.y11 * c.y11 * c.ir;
     }
-    c.ey = dp.sd / c.r - c.y * q / c.r3;
-    c.ez = dp.cd / c.r + c.d * q / c.r3;
-    c.fy = c.d / c.r3 + c.xi2 * c.y32 * dp.sd;
-    c.fz = c.y / c.r3 + c.xi2 * c.y32 * dp.cd;
+    c.ey = dp.sd * c.ir - c.y * q * c.ir3;
+    c.ez = dp.cd * c.ir + c.d * q * c.ir3;
+    c.fy = c.d * c.ir3 + c.xi2 * c.y32 * dp.sd;
+    c.fz = c.y * c.ir3 + c.xi2 * c.y32 * dp.cd;
     c.gy = 2.0 * c.x11 * dp.sd - c.y * q * c.x32;
     c.gz = 2.0 * c.x11 * dp.cd + c.d * q * c.x32;
     c.hy = c.d * q * c.x32 + xi * q * c.y32 * dp.sd;
@@ -112,144 +117,148 @@ __device__ inline bool ok_corner(double &xi, double &et, double &q, const OkDip 
     return true;
 }
 
+// The parts leave out the common factor 1 / (2 pi); the sums apply it once.
 // Gradient entries g[0..8] correspond to DC3D's U(4..12):
 // uxx, uyx, uzx, uxy, uyy, uzy, uxz, uyz, uzz.
 #define OK_K (1.0 / 6.283185307179586)
 
 // Part A (dc3d.f:200-282), strike (s) and dip (d) slip, gradient entries only.
-__device__ inline void ok_part_a(const OkCorner &c, const OkDip &dp, const OkMed &m, double s[9],
+// With a2 = alp2 and h = 1/2 it is the real source's.  Part B (dc3d.f:284-400)
+// repeats its terms without the medium constants and with the halves negated, so
+// that A + B of the image source is this with a2 = alp2 - 1 and h = -1/2 plus what
+// ok_part_b adds.
+__device__ inline void ok_part_a(const OkCorner &c, const OkDip &dp, double a1, double a2, double h, double s[9],
                                  double d[9])
 {
-    const double xi = c.xi, et = c.et, q = c.q, R = c.r, R3 = c.r3;
-    const double xy = xi * c.y11, qx = q * c.x11, qy = q * c.y11;
-    (void)qx;
-    s[0] = OK_K * (-m.alp1 * qy - m.alp2 * c.xi2 * q * c.y32);
-    s[1] = OK_K * (-m.alp2 * xi * q / R3);
-    s[2] = OK_K * (m.alp1 * xy + m.alp2 * xi * c.q2 * c.y32);
-    s[3] = OK_K * (m.alp1 * xy * dp.sd + m.alp2 * xi * c.fy + c.d / 2.0 * c.x11);
-    s[4] = OK_K * (m.alp2 * c.ey);
-    s[5] = OK_K * (m.alp1 * (dp.cd / R + qy * dp.sd) - m.alp2 * q * c.fy);
-    s[6] = OK_K * (m.alp1 * xy * dp.cd + m.alp2 * xi * c.fz + c.y / 2.0 * c.x11);
-    s[7] = OK_K * (m.alp2 * c.ez);
-    s[8] = OK_K * (-m.alp1 * (dp.sd / R - qy * dp.cd) - m.alp2 * q * c.fz);
+    const double xi = c.xi, et = c.et, q = c.q;
+    const double xy = xi * c.y11, qy = q * c.y11, a1xy = a1 * xy, a1qy = a1 * qy, hxy = h * xy;
+    const double xr = a2 * xi, qr = a2 * q, er = a2 * et, qq = qr * q, q3 = qr * c.ir3;
+    const double a1r = a1 * c.ir, hx = h * c.x11, a1x = a1 * c.x11;
+    s[0] = -a1qy - qr * c.xi2 * c.y32;
+    s[1] = -xi * q3;
+    s[2] = a1xy + qq * xi * c.y32;
+    s[3] = a1xy * dp.sd + xr * c.fy + c.d * hx;
+    s[4] = a2 * c.ey;
+    s[5] = a1r * dp.cd + a1qy * dp.sd - qr * c.fy;
+    s[6] = a1xy * dp.cd + xr * c.fz + c.y * hx;
+    s[7] = a2 * c.ez;
+    s[8] = a1qy * dp.cd - a1r * dp.sd - qr * c.fz;
 
-    d[0] = OK_K * (-m.alp2 * xi * q / R3);
-    d[1] = OK_K * (-qy / 2.0 - m.alp2 * et * q / R3);
-    d[2] = OK_K * (m.alp1 / R + m.alp2 * c.q2 / R3);
-    d[3] = OK_K * (m.alp2 * c.ey);
-    d[4] = OK_K * (m.alp1 * c.d * c.x11 + xy / 2.0 * dp.sd + m.alp2 * et * c.gy);
-    d[5] = OK_K * (m.alp1 * c.y * c.x11 - m.alp2 * q * c.gy);
-    d[6] = OK_K * (m.alp2 * c.ez);
-    d[7] = OK_K * (m.alp1 * c.y * c.x11 + xy / 2.0 * dp.cd + m.alp2 * et * c.gz);
-    d[8] = OK_K * (-m.alp1 * c.d * c.x11 - m.alp2 * q * c.gz);
+    d[0] = s[1];
+    d[1] = -h * qy - et * q3;
+    d[2] = a1r + q * q3;
+    d[3] = s[4];
+    d[4] = c.d * a1x + hxy * dp.sd + er * c.gy;
+    d[5] = c.y * a1x - qr * c.gy;
+    d[6] = s[7];
+    d[7] = c.y * a1x + hxy * dp.cd + er * c.gz;
+    d[8] = -c.d * a1x - qr * c.gz;
 }
 
-// Part B (dc3d.f:284-400).
-__device__ inline void ok_part_b(const OkCorner &c, const OkDip &dp, const OkMed &m, double s[9],
-                                 double d[9])
+// Part B (dc3d.f:284-400) less what ok_part_a covers, added to s and d.
+__device__ inline void ok_part_b(const OkCorner &c, const OkDip &dp, double a3, double s[9], double d[9])
 {
-    const double xi = c.xi, et = c.et, q = c.q, R = c.r, R3 = c.r3, Y = c.y, D = c.d;
-    const double rd = R + D;
-    const double d11 = 1.0 / (R * rd);
-    const double aj2 = xi * Y / rd * d11;
-    const double aj5 = -(D + Y * Y / rd) * d11;
+    const double xi = c.xi, q = c.q, Y = c.y, D = c.d;
+    const double ird = 1.0 / (c.r + D);
+    const double d11 = c.ir * ird, yd = Y * ird;
+    const double aj2 = xi * yd * d11;
+    const double aj5 = -(D + Y * yd) * d11;
     // ai1..ai4 enter only the displacement entries and are not formed.
     double ak1, ak3, aj3, aj6;
     if (dp.cd != 0.0) {
-        ak1 = xi * (d11 - c.y11 * dp.sd) / dp.cd;
-        ak3 = (q * c.y11 - Y * d11) / dp.cd;
-        aj3 = (ak1 - aj2 * dp.sd) / dp.cd;
-        aj6 = (ak3 - aj5 * dp.sd) / dp.cd;
+        ak1 = xi * (d11 - c.y11 * dp.sd) * dp.icd;
+        ak3 = (q * c.y11 - Y * d11) * dp.icd;
+        aj3 = (ak1 - aj2 * dp.sd) * dp.icd;
+        aj6 = (ak3 - aj5 * dp.sd) * dp.icd;
     } else {
-        double rd2 = rd * rd;
-        ak1 = xi * q / rd * d11;
-        ak3 = dp.sd / rd * (c.xi2 * d11 - 1.0);
-        aj3 = -xi / rd2 * (c.q2 * d11 - 1.0 / 2.0);
-        aj6 = -Y / rd2 * (c.xi2 * d11 - 1.0 / 2.0);
+        const double ird2 = ird * ird;
+        ak1 = xi * q * ird * d11;
+        ak3 = dp.sd * ird * (c.xi2 * d11 - 1.0);
+        aj3 = -xi * ird2 * (c.q2 * d11 - 0.5);
+        aj6 = -Y * ird2 * (c.xi2 * d11 - 0.5);
     }
     const double xy = xi * c.y11;
-    const double ak2 = 1.0 / R + ak3 * dp.sd;
+    const double ak2 = c.ir + ak3 * dp.sd;
     const double ak4 = xy * dp.cd - ak1 * dp.sd;
     const double aj1 = aj5 * dp.cd - aj6 * dp.sd;
     const double aj4 = -xy - aj2 * dp.cd + aj3 * dp.sd;
-    const double qy = q * c.y11;
-    const double a3 = m.alp3;
-
-    s[0] = OK_K * (c.xi2 * q * c.y32 - a3 * aj1 * dp.sd);
-    s[1] = OK_K * (xi * q / R3 - a3 * aj2 * dp.sd);
-    s[2] = OK_K * (-xi * c.q2 * c.y32 - a3 * aj3 * dp.sd);
-    s[3] = OK_K * (-xi * c.fy - D * c.x11 + a3 * (xy + aj4) * dp.sd);
-    s[4] = OK_K * (-c.ey + a3 * (1.0 / R + aj5) * dp.sd);
-    s[5] = OK_K * (q * c.fy - a3 * (qy - aj6) * dp.sd);
-    s[6] = OK_K * (-xi * c.fz - Y * c.x11 + a3 * ak1 * dp.sd);
-    s[7] = OK_K * (-c.ez + a3 * Y * d11 * dp.sd);
-    s[8] = OK_K * (q * c.fz + a3 * ak2 * dp.sd);
-
-    d[0] = OK_K * (xi * q / R3 + a3 * aj4 * dp.sdcd);
-    d[1] = OK_K * (et * q / R3 + qy + a3 * aj5 * dp.sdcd);
-    d[2] = OK_K * (-c.q2 / R3 + a3 * aj6 * dp.sdcd);
-    d[3] = OK_K * (-c.ey + a3 * aj1 * dp.sdcd);
-    d[4] = OK_K * (-et * c.gy - xy * dp.sd + a3 * aj2 * dp.sdcd);
-    d[5] = OK_K * (q * c.gy + a3 * aj3 * dp.sdcd);
-    d[6] = OK_K * (-c.ez - a3 * ak3 * dp.sdcd);
-    d[7] = OK_K * (-et * c.gz - xy * dp.cd - a3 * xi * d11 * dp.sdcd);
-    d[8] = OK_K * (q * c.gz - a3 * ak4 * dp.sdcd);
+    const double as = a3 * dp.sd, ac = a3 * dp.sdcd;
+    s[0] -= as * aj1;
+    s[1] -= as * aj2;
+    s[2] -= as * aj3;
+    s[3] += as * (xy + aj4);
+    s[4] += as * (c.ir + aj5);
+    s[5] -= as * (q * c.y11 - aj6);
+    s[6] += as * ak1;
+    s[7] += as * (Y * d11);
+    s[8] += as * ak2;
+    d[0] += ac * aj4;
+    d[1] += ac * aj5;
+    d[2] += ac * aj6;
+    d[3] += ac * aj1;
+    d[4] += ac * aj2;
+    d[5] += ac * aj3;
+    d[6] -= ac * ak3;
+    d[7] -= ac * (xi * d11);
+    d[8] -= ac * ak4;
 }
 
 // Part C (dc3d.f:402-507).  Also returns the displacement entries 1..3 of part C
-// (c0 for strike, e0 for dip), which the image sum adds to the z-derivatives.
+// (cs for strike, cdp for dip), which the image sum adds to the z-derivatives.
 __device__ inline void ok_part_c(const OkCorner &c, const OkDip &dp, const OkMed &m, double Z,
                                  double s[9], double d[9], double cs[3], double cdp[3])
 {
-    const double xi = c.xi, et = c.et, q = c.q, R = c.r, R2 = c.r2, R3 = c.r3, R5 = c.r5;
-    const double Y = c.y, D = c.d, sd = dp.sd, cd = dp.cd;
-    const double a4 = m.alp4, a5 = m.alp5;
-    const double C = D + Z;
-    const double x53 = (8.0 * R2 + 9.0 * R * xi + 3.0 * c.xi2) * c.x11 * c.x11 * c.x11 / R2;
-    const double y53 = (8.0 * R2 + 9.0 * R * et + 3.0 * c.et2) * c.y11 * c.y11 * c.y11 / R2;
-    const double h = q * cd - Z;
-    const double z32 = sd / R3 - h * c.y32;
-    const double z53 = 3.0 * sd / R5 - h * y53;
-    const double y0 = c.y11 - c.xi2 * c.y32;
+    const double xi = c.xi, et = c.et, q = c.q, Y = c.y, D = c.d, sd = dp.sd, cd = dp.cd;
+    const double a4 = m.alp4, a5 = m.alp5, X11 = c.x11, X32 = c.x32, Y32 = c.y32;
+    const double C = D + Z, aC = a5 * C;
+    const double x53 = (8.0 * c.r2 + 9.0 * c.r * xi + 3.0 * c.xi2) * X11 * X11 * X11 * c.ir2;
+    const double y53 = (8.0 * c.r2 + 9.0 * c.r * et + 3.0 * c.et2) * c.y11 * c.y11 * c.y11 * c.ir2;
+    const double r3 = c.ir3, t5 = 3.0 * c.ir5;
+    const double qR = q * r3, yR = Y * r3, dR = D * r3, eR = et * r3, sR = sd * r3, cR = cd * r3;
+    const double h = q * cd - Z, qY = q * Y32;
+    const double z32 = sR - h * Y32;
+    const double z53 = sd * t5 - h * y53;
+    const double y0 = c.y11 - c.xi2 * Y32;
     const double z0 = z32 - c.xi2 * z53;
-    const double ppy = cd / R3 + q * c.y32 * sd;
-    const double ppz = sd / R3 - q * c.y32 * cd;
-    const double qq = Z * c.y32 + z32 + z0;
-    const double qqy = 3.0 * C * D / R5 - qq * sd;
-    const double qqz = 3.0 * C * Y / R5 - qq * cd + q * c.y32;
-    const double xy = xi * c.y11;
-    const double qy = q * c.y11;
-    const double qr = 3.0 * q / R5;
-    const double cdr = (C + D) / R3;
-    const double yy0 = Y / R3 - y0 * cd;
-    const double X11 = c.x11, X32 = c.x32, Y11 = c.y11, Y32 = c.y32, Q2 = c.q2;
+    const double ppy = cR + qY * sd;
+    const double ppz = sR - qY * cd;
+    const double qq = Z * Y32 + z32 + z0;
+    const double Ct = C * t5;
+    const double qqy = Ct * D - qq * sd;
+    const double qqz = Ct * Y - qq * cd + qY;
+    const double xy = xi * c.y11, qy = q * c.y11;
+    const double ar = a5 * Ct * q;             // a5 C qr
+    const double acdr = a5 * (C + D) * r3;     // a5 cdr
+    const double yy0 = yR - y0 * cd, qz0 = q * z0;
+    const double w1 = acdr * sd - ar * Y, w2 = acdr * cd + ar * D;
+    const double eq = et * q, aCq = aC * qR;
 
-    cs[0] = OK_K * (a4 * xy * cd - a5 * xi * q * z32);
-    cs[1] = OK_K * (a4 * (cd / R + 2.0 * qy * sd) - a5 * C * q / R3);
-    cs[2] = OK_K * (a4 * qy * cd - a5 * (C * et / R3 - Z * Y11 + c.xi2 * z32));
-    s[0] = OK_K * (a4 * y0 * cd - a5 * q * z0);
-    s[1] = OK_K * (-a4 * xi * (cd / R3 + 2.0 * q * Y32 * sd) + a5 * C * xi * qr);
-    s[2] = OK_K * (-a4 * xi * q * Y32 * cd + a5 * xi * (3.0 * C * et / R5 - qq));
-    s[3] = OK_K * (-a4 * xi * ppy * cd - a5 * xi * qqy);
-    s[4] = OK_K * (a4 * 2.0 * (D / R3 - y0 * sd) * sd - Y / R3 * cd
-                   - a5 * (cdr * sd - et / R3 - C * Y * qr));
-    s[5] = OK_K * (-a4 * q / R3 + yy0 * sd + a5 * (cdr * cd + C * D * qr - (y0 * cd + q * z0) * sd));
-    s[6] = OK_K * (a4 * xi * ppz * cd - a5 * xi * qqz);
-    s[7] = OK_K * (a4 * 2.0 * (Y / R3 - y0 * cd) * sd + D / R3 * cd - a5 * (cdr * cd + C * D * qr));
-    s[8] = OK_K * (yy0 * cd - a5 * (cdr * sd - C * Y * qr - y0 * dp.sdsd + q * z0 * cd));
+    cs[0] = xi * (a4 * c.y11 * cd - a5 * q * z32);
+    cs[1] = a4 * (cd * c.ir + 2.0 * qy * sd) - aCq;
+    cs[2] = a4 * qy * cd - aC * eR + a5 * (Z * c.y11 - c.xi2 * z32);
+    s[0] = a4 * y0 * cd - a5 * qz0;
+    s[1] = xi * (ar - a4 * (cR + 2.0 * qY * sd));
+    s[2] = xi * (a5 * (Ct * et - qq) - a4 * qY * cd);
+    s[3] = -xi * (a4 * ppy * cd + a5 * qqy);
+    s[4] = a4 * 2.0 * (dR - y0 * sd) * sd - yR * cd - w1 + a5 * eR;
+    s[5] = yy0 * sd - a4 * qR + w2 - a5 * sd * (y0 * cd + qz0);
+    s[6] = xi * (a4 * ppz * cd - a5 * qqz);
+    s[7] = a4 * 2.0 * (yR - y0 * cd) * sd + dR * cd - w2;
+    s[8] = yy0 * cd - w1 + a5 * (y0 * dp.sdsd - qz0 * cd);
 
-    cdp[0] = OK_K * (a4 * cd / R - qy * sd - a5 * C * q / R3);
-    cdp[1] = OK_K * (a4 * Y * X11 - a5 * C * et * q * X32);
-    cdp[2] = OK_K * (-D * X11 - xy * sd - a5 * C * (X11 - Q2 * X32));
-    d[0] = OK_K * (-a4 * xi / R3 * cd + a5 * C * xi * qr + xi * q * Y32 * sd);
-    d[1] = OK_K * (-a4 * Y / R3 + a5 * C * et * qr);
-    d[2] = OK_K * (D / R3 - y0 * sd + a5 * C / R3 * (1.0 - 3.0 * Q2 / R2));
-    d[3] = OK_K * (-a4 * et / R3 + y0 * dp.sdsd - a5 * (cdr * sd - C * Y * qr));
-    d[4] = OK_K * (a4 * (X11 - Y * Y * X32) - a5 * C * ((D + 2.0 * q * cd) * X32 - Y * et * q * x53));
-    d[5] = OK_K * (xi * ppy * sd + Y * D * X32 + a5 * C * ((Y + 2.0 * q * sd) * X32 - Y * Q2 * x53));
-    d[6] = OK_K * (-q / R3 + y0 * dp.sdcd - a5 * (cdr * cd + C * D * qr));
-    d[7] = OK_K * (a4 * Y * D * X32 - a5 * C * ((Y - 2.0 * q * sd) * X32 + D * et * q * x53));
-    d[8] = OK_K * (-xi * ppz * sd + X11 - D * D * X32 - a5 * C * ((D - 2.0 * q * cd) * X32 - D * Q2 * x53));
+    const double xe = eq * x53, xq = c.q2 * x53, q2c = 2.0 * q * cd, q2s = 2.0 * q * sd;
+    cdp[0] = a4 * cd * c.ir - qy * sd - aCq;
+    cdp[1] = a4 * Y * X11 - aC * eq * X32;
+    cdp[2] = -D * X11 - xy * sd - aC * (X11 - c.q2 * X32);
+    d[0] = xi * (ar - a4 * cR + qY * sd);
+    d[1] = ar * et - a4 * yR;
+    d[2] = dR - y0 * sd + aC * r3 * (1.0 - 3.0 * c.q2 * c.ir2);
+    d[3] = y0 * dp.sdsd - a4 * eR - w1;
+    d[4] = a4 * (X11 - Y * Y * X32) - aC * ((D + q2c) * X32 - Y * xe);
+    d[5] = xi * ppy * sd + Y * D * X32 + aC * ((Y + q2s) * X32 - Y * xq);
+    d[6] = y0 * dp.sdcd - qR - w2;
+    d[7] = a4 * Y * D * X32 - aC * ((Y - q2s) * X32 + D * xe);
+    d[8] = X11 - xi * ppz * sd - D * D * X32 - aC * ((D - q2c) * X32 - D * xq);
 }
 
 // Part C's displacement entries are the same statements as DU(1..3) of UC.
@@ -312,25 +321,24 @@ __device__ inline bool ok_dc3d_grad(const OkMed &m, const OkDip &dp, double x, d
         for (int kk = 0; kk < 4; kk++) {
             const int k = kk >> 1, j = kk & 1;
             ok_corner(xi[j], et[k], q, dp, kxi[k], ket[j], c);
-            ok_part_a(c, dp, m, as, ad);
+            ok_part_a(c, dp, m.alp1, m.alp2, 0.5, as, ad);
             const double sg = (j + k != 1) ? 1.0 : -1.0;
 #pragma unroll
-            for (int t = 0; t < 2; t++) {
-                const double *a = t ? ad : as;
-                double *g = t ? gd : gs;
-                double du[9];
-                // rows 1..3 of DC3D's 4x3 block rotation; the z-derivative row is negated
-                du[0] = -a[0];
-                du[1] = -a[1] * dp.cd + a[2] * dp.sd;
-                du[2] = -a[1] * dp.sd - a[2] * dp.cd;
-                du[3] = -a[3];
-                du[4] = -a[4] * dp.cd + a[5] * dp.sd;
-                du[5] = -a[4] * dp.sd - a[5] * dp.cd;
-                du[6] = -(-a[6]);
-                du[7] = -(-a[7] * dp.cd + a[8] * dp.sd);
-                du[8] = -(-a[7] * dp.sd - a[8] * dp.cd);
+            for (int i = 0; i < 9; i++) {
+                gs[i] += sg * as[i];
+                gd[i] += sg * ad[i];
+            }
+        }
+        // rows 1..3 of DC3D's 4x3 block rotation; the z-derivative row is negated
 #pragma unroll
-                for (int i = 0; i < 9; i++) g[i] = (sg > 0.0) ? g[i] + du[i] : g[i] - du[i];
+        for (int t = 0; t < 2; t++) {
+            double *g = t ? gd : gs;
+#pragma unroll
+            for (int r = 0; r < 9; r += 3) {
+                const double f = r == 6 ? 1.0 : -1.0, a1 = g[r + 1], a2 = g[r + 2];
+                g[r] = f * g[r];
+                g[r + 1] = f * (a1 * dp.cd - a2 * dp.sd);
+                g[r + 2] = f * (a1 * dp.sd + a2 * dp.cd);
             }
         }
     }
@@ -349,15 +357,14 @@ __device__ inline bool ok_dc3d_grad(const OkMed &m, const OkDip &dp, double x, d
         for (int kk = 0; kk < 4; kk++) {
             const int k = kk >> 1, j = kk & 1;
             ok_corner(xi[j], et[k], q, dp, kxi[k], ket[j], c);
-            double bs[9], bd[9], cs9[9], cd9[9], c0s[3], c0d[3];
-            ok_part_a(c, dp, m, as, ad);
-            ok_part_b(c, dp, m, bs, bd);
+            double cs9[9], cd9[9], c0s[3], c0d[3];
+            ok_part_a(c, dp, m.alp1, m.alp2 - 1.0, -0.5, as, ad);
+            ok_part_b(c, dp, m.alp3, as, ad);
             ok_part_c(c, dp, m, z, cs9, cd9, c0s, c0d);
             const double sg = (j + k != 1) ? 1.0 : -1.0;
 #pragma unroll
             for (int t = 0; t < 2; t++) {
                 const double *a = t ? ad : as;
-                const double *b = t ? bd : bs;
                 const double *cc = t ? cd9 : cs9;
                 const double *c0 = t ? c0d : c0s;
                 double *g = t ? gd : gs;
@@ -365,23 +372,23 @@ __device__ inline bool ok_dc3d_grad(const OkMed &m, const OkDip &dp, double x, d
 #pragma unroll
                 for (int r = 0; r < 3; r++) {
                     const int i = 3 * r;
-                    du[i] = a[i] + b[i] + z * cc[i];
-                    du[i + 1] = (a[i + 1] + b[i + 1] + z * cc[i + 1]) * dp.cd
-                              - (a[i + 2] + b[i + 2] + z * cc[i + 2]) * dp.sd;
-                    du[i + 2] = (a[i + 1] + b[i + 1] - z * cc[i + 1]) * dp.sd
-                              + (a[i + 2] + b[i + 2] - z * cc[i + 2]) * dp.cd;
+                    du[i] = a[i] + z * cc[i];
+                    du[i + 1] = (a[i + 1] + z * cc[i + 1]) * dp.cd - (a[i + 2] + z * cc[i + 2]) * dp.sd;
+                    du[i + 2] = (a[i + 1] - z * cc[i + 1]) * dp.sd + (a[i + 2] - z * cc[i + 2]) * dp.cd;
                 }
                 du[6] = du[6] + c0[0];
                 du[7] = du[7] + c0[1] * dp.cd - c0[2] * dp.sd;
                 du[8] = du[8] - c0[1] * dp.sd - c0[2] * dp.cd;
 #pragma unroll
-                for (int i = 0; i < 9; i++) g[i] = (sg > 0.0) ? g[i] + du[i] : g[i] - du[i];
+                for (int i = 0; i < 9; i++) g[i] += sg * du[i];
             }
         }
     }
-    if (R32) {
 #pragma unroll
-        for (int i = 0; i < 9; i++) {
+    for (int i = 0; i < 9; i++) {
+        gs[i] *= OK_K;
+        gd[i] *= OK_K;
+        if (R32) {
             gs[i] = (double)__double2float_rn(gs[i]);
             gd[i] = (double)__double2float_rn(gd[i]);
         }
@@ -521,9 +528,10 @@ __device__ inline bool ok_dc3d_disp(const OkMed &m, const OkDip &dp, double x, d
                     const double *b = t ? bd : bs;
                     const double *cc = t ? c0d : c0s;
                     double *u = t ? ud : us;
-                    const double du0 = a[0] + b[0] + z * cc[0];
-                    const double du1 = (a[1] + b[1] + z * cc[1]) * dp.cd - (a[2] + b[2] + z * cc[2]) * dp.sd;
-                    const double du2 = (a[1] + b[1] - z * cc[1]) * dp.sd + (a[2] + b[2] - z * cc[2]) * dp.cd;
+                    const double zk = z * OK_K;
+                    const double du0 = a[0] + b[0] + zk * cc[0];
+                    const double du1 = (a[1] + b[1] + zk * cc[1]) * dp.cd - (a[2] + b[2] + zk * cc[2]) * dp.sd;
+                    const double du2 = (a[1] + b[1] - zk * cc[1]) * dp.sd + (a[2] + b[2] - zk * cc[2]) * dp.cd;
                     u[0] = (sg > 0.0) ? u[0] + du0 : u[0] - du0;
                     u[1] = (sg > 0.0) ? u[1] + du1 : u[1] - du1;
                     u[2] = (sg > 0.0) ? u[2] + du2 : u[2] - du2;
