@@ -1,19 +1,26 @@
 // Right-hand side and Cash-Karp RK4(5) stepping on the device.
 //
-// One attempt of RKQSm (fortran/3d/src/ode45.f90:51-108) is a fixed sequence of
-// launches, captured once into a CUDA graph:
+// One attempt of RKQSm (fortran/3d/src/ode45.f90:51-108) is six launches, one per
+// stage, captured once into a CUDA graph.  The launch of stage s
 //
-//   stage 1   k_prologue<1>  commit an accepted candidate, v = V(cos,sin)(rake)-Vpl
-//             k_traction<1>  t = K v  fused with the rate-state / Maxwell epilogue
-//   stage s   k_prologue<s>  ytmp = y + h*sum_j b_sj k_j  (BLAS-1 order of RKCKm)
-//             k_traction<s>  k_s = f(ytmp)                              (s = 2..6)
-//   finish    k_finish       ycand, yerr, max|yerr/yscal| (ordered-bit atomicMax)
-//   control   k_control      accept/reject, step size, time, counters (1 thread)
+//   multiplies    t = K v_s (k_traction; hierarchical K: its product, then k_rhs_t)
+//   and then, element by element as the row sums arrive,
+//   evaluates     k_s = f(y_s) (rate-state / Maxwell epilogue),
+//   and forms     s < 6: y_{s+1} = y + h sum_j b_sj k_j (BLAS-1 order of RKCKm) and
+//                        the source rates v_{s+1} of the next launch;
+//                 s = 6: ycand, yerr, max|yerr/yscal| (ordered-bit atomicMax) and the
+//                        source rates of ycand.
+//
+// The last CTA of stage 6 decides: accept/reject, step size, time, counters.  All of
+// an element's stage vectors are local to it, so nothing but v crosses elements; v
+// alternates between two buffers.  Stage 1 of the next attempt commits an accepted
+// candidate into y; after a rejection it only forms y_2 again for the new h.
 //
 // Every kernel reads the control block first and returns at once when the
-// integration is inactive, or (stage 1) when the state did not change since the
-// last f(y), so the same graph serves accepted and rejected attempts and many
-// attempts can be queued without host round trips.
+// integration is inactive, so the same graph serves accepted and rejected attempts
+// and many attempts can be queued without host round trips.  Separate kernels for
+// the stage state, the error norm and the decision (14 launches an attempt) cost
+// 67 us a step at N = 512, where each launch is latency alone.
 //
 // The stage combinations, yout and yerr follow the reference's operation order
 // with explicit round-to-nearest multiplies and adds (no FMA contraction), so
@@ -57,10 +64,13 @@ __device__ __constant__ double c_B[6][5] = {
 static const double LG10 = 2.302585092994045684017991454684364208;
 
 struct StageArgs {
-    const double *y;       // state at the start of the step
-    double *ys;            // stage state written by the prologue (y itself for stage 1)
+    double *y;             // state at the start of the step
+    double *ys;            // state of the stages after the first
     double *k[6];
-    double *v;
+    double *ks;            // k of this stage
+    const double *v;       // source rates of this stage
+    double *vn;            // source rates of the next one
+    int next;              // form the next stage's state (0: only k_s)
     double *ycand, *yerr, *yscal;
     double *v1, *t1;       // stage-1 anchor (split-BF16 matrix only)
     int anchored;
@@ -79,10 +89,12 @@ __device__ __forceinline__ bool ctl_live(const Ctl *c) { return c->active && c->
 // its own successor be scheduled.  So the launch latency of every kernel of an
 // attempt overlaps the previous kernel instead of adding to it (it dominates
 // at small N).  Without a programmatic predecessor the wait returns at once.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter()
 {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    pdl_launch();
 }
 
 template <typename... KArgs, typename... Args>
@@ -108,156 +120,415 @@ __device__ __forceinline__ void atomic_max_pos(unsigned long long *p, double x)
     atomicMax(p, (unsigned long long)__double_as_longlong(x));
 }
 
-// ---- stage prologue ------------------------------------------------------------
+// ---- one element of a stage -------------------------------------------------------
+//
+// A patch takes 8 lanes of a warp, a volume 16; lane c holds component c of the
+// element's state (7 and 12), so that the stage vectors are read as short runs and
+// the combination of a component is one lane's work.  What does not depend on the
+// product (the state, the sums over the earlier stages, the friction terms of f) is
+// loaded and formed before the row sums arrive: the next launch waits for what
+// comes after them.
 
-// stage combination for one entry with the reference BLAS-1 order
-template <int S>
-__device__ __forceinline__ double stage_comb(const StageArgs &a, long i, double h)
+struct LaneState {
+    double y;             // the step's initial state
+    double r, e;          // the combination and (stage 6) the error over the stages so far
+    double cs;            // coefficient of this stage in the next one's combination
+    double yscal;         // stage 6
+    bool on;              // the lane holds a component
+};
+
+// state of stage S + 1 with the reference BLAS-1 order, ks = k_S being its last term
+__device__ __forceinline__ double stage_comb(int S, const LaneState &st, double ks, double h)
 {
-    const double y = a.y[i];
-    if (S == 1) return y;
-    if (S == 2) return __dadd_rn(y, __dmul_rn(__dmul_rn(h, c_B[1][0]), a.k[0][i]));
-    double r = __dmul_rn(c_B[S - 1][0], a.k[0][i]);
-#pragma unroll
-    for (int j = 1; j < S - 1; j++) r = __dadd_rn(r, __dmul_rn(c_B[S - 1][j], a.k[j][i]));
-    return __dadd_rn(y, __dmul_rn(h, r));
+    if (S == 1) return __dadd_rn(st.y, __dmul_rn(__dmul_rn(h, c_B[1][0]), ks));
+    return __dadd_rn(st.y, __dmul_rn(h, __dadd_rn(st.r, __dmul_rn(st.cs, ks))));
 }
 
-template <int S>
-__global__ void k_prologue(StageArgs a, Ctl *ctl)
+// x / d where rd = 1 / d is at hand before x: the quotient's residual corrects it
+// once (Markstein, IBM J. Res. Dev. 34, 1990), which rounds like the division for
+// normal quotients; three dependent operations instead of a division's sequence
+__device__ __forceinline__ double div_by(double x, double d, double rd)
+{
+    const double q = x * rd;
+    return fma(fma(-d, q, x), rd, q);
+}
+
+constexpr double INV_LG10 = 0.434294481903251827651128918916605082;   // 1 / ln 10
+
+// slip velocity and the cosine and sine of the rake atan2(td, ts)
+// (ratestate.f90:682-690); where the sum of squares is of no use the angle itself
+__device__ __forceinline__ void patch_slip(double ts, double td, double lv, double &vel, double &cr, double &sr)
+{
+    vel = exp(lv * LG10);
+    const double h2 = ts * ts + td * td;
+    if (h2 > 1.0e-280 && h2 < 1.0e280) {
+        // the square root from its reciprocal by the same correction, then the quotients
+        const double ih = rsqrt(h2), g = h2 * ih, hy = fma(fma(-g, g, h2), 0.5 * ih, g);
+        cr = div_by(ts, hy, ih);
+        sr = div_by(td, hy, ih);
+    } else {
+        const double rake = atan2(td, ts);
+        cr = cos(rake);
+        sr = sin(rake);
+    }
+}
+
+// Maxwell strain rate of component q of a volume with stresses s11 .. s33
+// (viscouscycles.f90:938-995)
+__device__ __forceinline__ double volume_rate(const Rheology &rh, int iv, int q, double s11, double s12, double s13,
+                                              double s22, double s23, double s33)
+{
+    if (!rh.nonlinear) return 0.0;
+    const double p = (s11 + s22 + s33) / 3.0;
+    s11 = s11 - p; s22 = s22 - p; s33 = s33 - p;
+    const double sII = sqrt((s11 * s11 + 2.0 * s12 * s12 + 2.0 * s13 * s13 + s22 * s22 + 2.0 * s23 * s23 + s33 * s33) /
+                            2.0);
+    const double eII = rh.gd0[iv] * pow(sII, rh.npow[iv] - 1);
+    return eII * (q == 0 ? s11 : q == 1 ? s12 : q == 2 ? s13 : q == 3 ? s22 : q == 4 ? s23 : s33);
+}
+
+// state of stage S in the lane (commits an accepted candidate at stage 1), and the
+// sums over the earlier stages
+__device__ __forceinline__ double lane_load(int S, const StageArgs &a, const Ctl *ctl, long i, bool on, LaneState &st)
+{
+    st = LaneState{0.0, 0.0, 0.0, 0.0, 1.0, on};
+    if (!on) return 0.0;
+    st.y = a.y[i];
+    if (S == 1) {
+        if (!a.next) return st.y;
+        const double yc = a.ycand[i];
+        if (ctl->pending) a.y[i] = st.y = yc;
+        return st.y;
+    }
+    const double ys = a.ys[i];
+    if (!a.next) return ys;
+    double k[5];
+#pragma unroll
+    for (int j = 0; j < 5; j++) k[j] = j < S - 1 ? a.k[j][i] : 0.0;
+    if (S < 6) {
+        double r = __dmul_rn(c_B[S][0], k[0]);
+#pragma unroll
+        for (int j = 1; j < 4; j++)
+            if (j < S - 1) r = __dadd_rn(r, __dmul_rn(c_B[S][j], k[j]));
+        st.r = r;
+        st.cs = c_B[S][S - 1];
+        return ys;
+    }
+    st.yscal = a.yscal[i];
+    // ode45.f90:184-200
+    double r = __dmul_rn(C1, k[0]);
+    r = __dadd_rn(r, __dmul_rn(C3, k[2]));
+    st.r = __dadd_rn(r, __dmul_rn(C4, k[3]));
+    double e = __dmul_rn(DC1, k[0]);
+    e = __dadd_rn(e, __dmul_rn(DC3, k[2]));
+    e = __dadd_rn(e, __dmul_rn(DC4, k[3]));
+    st.e = __dadd_rn(e, __dmul_rn(DC5, k[4]));
+    return ys;
+}
+
+// the lane's rate ks at stage S known: store it, then the next stage's component,
+// or at stage 6 the candidate and its error.  Returns the new component.
+__device__ __forceinline__ double lane_advance(int S, const StageArgs &a, long i, double h, const LaneState &st,
+                                               double ks, double &mx, bool &bad)
+{
+    if (!st.on) return 0.0;
+    a.ks[i] = ks;
+    if (!a.next) return 0.0;
+    if (S < 6) {
+        const double yn = stage_comb(S, st, ks, h);
+        a.ys[i] = yn;
+        if (S == 1) a.yscal[i] = fabs(st.y) + fabs(h * ks) + 1.0e-30;   // ratestate.f90:315; h == dt_try here
+        return yn;
+    }
+    const double yc = __dadd_rn(st.y, __dmul_rn(h, __dadd_rn(st.r, __dmul_rn(C6, ks))));
+    const double e = __dmul_rn(h, __dadd_rn(st.e, __dmul_rn(DC6, ks)));
+    a.ycand[i] = yc;
+    a.yerr[i] = e;
+    // MAXVAL semantics: a NaN ratio (0/0) does not raise the maximum; an
+    // infinite one does and drives the step to underflow as in the
+    // reference.  A non-finite candidate state is reported as such.
+    if (!isfinite(yc)) bad = true;
+    mx = fmax(mx, fabs(e / st.yscal));
+    return yc;
+}
+
+// source rate of column j of the next stage.  Anchored forms multiply increments
+// over stage 1 in the stages 2-6; vs: this stage's own rate (stage 1: the anchor)
+__device__ __forceinline__ void store_rate(int S, const StageArgs &a, long j, double vnext, double vs)
+{
+    if (a.anchored) {
+        if (S == 1) a.v1[j] = vs;
+        if (S < 6) vnext -= S == 1 ? vs : a.v1[j];
+    }
+    if (a.next) a.vn[j] = vnext;
+}
+
+// friction of a patch, and of its terms in f what the state gives
+// (ratestate.f90:731-776)
+struct PatchFriction {
+    double sig, a, b, eta, L, iL, vpl;
+};
+struct PatchTerms {
+    double vel, cr, sr, dth, q, den, rden, ev, vpl;
+};
+
+__device__ __forceinline__ PatchFriction patch_friction(const StageArgs &a, int e, int c, bool on)
+{
+    if (!on) return PatchFriction{1, 1, 0, 0, 1, 1, 0};
+    const double L = a.fr.L[e];
+    return PatchFriction{a.fr.sig[e], a.fr.a[e], a.fr.b[e], a.fr.damping[e], L, 1.0 / L,
+                         c == 0 ? a.fr.vpl_c[e] : c == 1 ? a.fr.vpl_s[e] : 0.0};
+}
+
+__device__ __forceinline__ PatchTerms patch_terms(int S, Ctl *ctl, const PatchFriction &f, int c, bool on, double ys)
+{
+    PatchTerms p;
+    const double ts = __shfl_sync(~0u, ys, 2, 8), td = __shfl_sync(~0u, ys, 3, 8);
+    const double th = __shfl_sync(~0u, ys, 5, 8), lv = __shfl_sync(~0u, ys, 6, 8);
+    patch_slip(ts, td, lv, p.vel, p.cr, p.sr);
+    p.den = f.a * f.sig + f.eta * p.vel;
+    p.rden = 1.0 / p.den;
+    p.dth = div_by(exp(-th * LG10) - div_by(p.vel, f.L, f.iL), LG10, INV_LG10);
+    p.q = f.b * f.sig * p.dth * LG10;
+    p.ev = f.eta * p.vel;
+    p.vpl = f.vpl;
+    if (S == 1 && on && c == 0) {
+        atomic_max_pos((unsigned long long *)&ctl->vmax, p.vel);
+        if (!isfinite(p.vel) || !isfinite(p.cr) || !isfinite(p.sr)) ctl->nonfinite = 1;
+    }
+    return p;
+}
+
+// patch e: rates from its tractions t, then the next stage
+__device__ __forceinline__ void patch_finish(int S, const StageArgs &a, Ctl *ctl, int e, int c, double h,
+                                             const LaneState &st, const PatchTerms &p, double t0, double t1,
+                                             double t2, double &mx, bool &bad)
+{
+    const double dv = div_by(div_by(t0 * p.cr + t1 * p.sr - p.q, p.den, p.rden), LG10, INV_LG10);
+    const double corr = p.ev * dv * LG10;
+    const double vs = p.vel * (c == 0 ? p.cr : p.sr);
+    const double ks = c < 2 ? vs : c == 2 ? t0 - corr * p.cr : c == 3 ? t1 - corr * p.sr : c == 4 ? t2
+                    : c == 5 ? p.dth : dv;
+    const double yn = lane_advance(S, a, 7L * e + c, h, st, ks, mx, bad);
+    const double ts = __shfl_sync(~0u, yn, 2, 8), td = __shfl_sync(~0u, yn, 3, 8), lv = __shfl_sync(~0u, yn, 6, 8);
+    if (!st.on || c > 1) return;
+    double vel = 0.0, cr = 1.0, sr = 0.0;
+    if (a.next) {
+        patch_slip(ts, td, lv, vel, cr, sr);
+        // (of a candidate only once it is accepted, at the next stage 1)
+        if (S < 6 && (!isfinite(vel) || !isfinite(cr) || !isfinite(sr))) ctl->nonfinite = 1;
+    }
+    store_rate(S, a, 2L * e + c, vel * (c == 0 ? cr : sr) - p.vpl, vs - p.vpl);
+}
+
+// volume iv: rates from its stress rate t (its own row for the lanes 6..11;
+// viscouscycles.f90:1072-1080), then the next stage.  ev: the lane's strain rate
+__device__ __forceinline__ void volume_finish(int S, const StageArgs &a, int iv, int c, double h, const LaneState &st,
+                                              double ev, double t, double &mx, bool &bad)
+{
+    const long o = 7L * a.np + 12L * iv;
+    const double yn = lane_advance(S, a, o + c, h, st, c < 6 ? ev : t, mx, bad);
+    double s[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) s[q] = __shfl_sync(~0u, yn, 6 + q, 16);
+    if (!st.on || c > 5) return;
+    const double ebg = a.rh.ebg[6L * iv + c];
+    const double en = a.next ? volume_rate(a.rh, iv, c, s[0], s[1], s[2], s[3], s[4], s[5]) : 0.0;
+    store_rate(S, a, 2L * a.np + 6L * iv + c, en - ebg, ev - ebg);
+}
+
+// source rates of the state y (before the first stage of a run; the attempts form
+// them as they go)
+__global__ void k_begin(StageArgs a, const Ctl *ctl, double *__restrict__ v)
 {
     pdl_enter();
-    if (!ctl_live(ctl)) return;
-    if (S == 1 && !ctl->need_stage1) return;
-    const double h = ctl->h;
+    if (!ctl_live(ctl) || !ctl->need_stage1) return;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ne = a.np + a.nvol;
-    if (e >= ne) return;
-    const bool patch = e < a.np;
-    const long o = patch ? 7L * e : 7L * a.np + 12L * (e - a.np);
-    const int w = patch ? 7 : 12;
-    double *ys = a.ys;
-    if (S == 1) {
-        if (ctl->pending) {
-            double *y = const_cast<double *>(a.y);
-            for (int q = 0; q < w; q++) y[o + q] = a.ycand[o + q];
-        }
+    if (e >= a.np + a.nvol) return;
+    if (e < a.np) {
+        const double *y = a.y + 7L * e;
+        double vel, cr, sr;
+        patch_slip(y[2], y[3], y[6], vel, cr, sr);
+        v[2L * e] = vel * cr - a.fr.vpl_c[e];
+        v[2L * e + 1] = vel * sr - a.fr.vpl_s[e];
     } else {
-        for (int q = 0; q < w; q++) ys[o + q] = stage_comb<S>(a, o + q, h);
-        if (S == 2 && ctl->need_stage1) {
-            // yscal = |y| + |dt_try*dydt| + TINY (ratestate.f90:315); h == dt_try here
-            for (int q = 0; q < w; q++)
-                a.yscal[o + q] = fabs(a.y[o + q]) + fabs(h * a.k[0][o + q]) + 1.0e-30;
-        }
-    }
-    const double *yy = (S == 1) ? a.y : ys;
-    double *ks = a.k[S - 1];
-    if (patch) {
-        // ratestate.f90:667-707
-        const double rake = atan2(yy[o + 3], yy[o + 2]);
-        const double vel = exp(yy[o + 6] * LG10);
-        const double vs = vel * cos(rake), vd = vel * sin(rake);
-        ks[o + 0] = vs;
-        ks[o + 1] = vd;
-        double v0 = vs - a.fr.vpl_c[e], v1 = vd - a.fr.vpl_s[e];
-        if (a.anchored) {
-            if (S == 1) {
-                a.v1[2L * e] = v0;
-                a.v1[2L * e + 1] = v1;
-            } else {
-                v0 -= a.v1[2L * e];
-                v1 -= a.v1[2L * e + 1];
-            }
-        }
-        a.v[2L * e + 0] = v0;
-        a.v[2L * e + 1] = v1;
-        if (S == 1) atomic_max_pos((unsigned long long *)&ctl->vmax, vel);
-        if (!isfinite(vel) || !isfinite(rake)) ctl->nonfinite = 1;
-    } else {
-        // viscouscycles.f90:938-995
         const int iv = e - a.np;
-        double s11 = yy[o + 6], s12 = yy[o + 7], s13 = yy[o + 8];
-        double s22 = yy[o + 9], s23 = yy[o + 10], s33 = yy[o + 11];
-        const double p = (s11 + s22 + s33) / 3.0;
-        s11 = s11 - p; s22 = s22 - p; s33 = s33 - p;
-        double ev[6] = {0, 0, 0, 0, 0, 0};
-        if (a.rh.nonlinear) {
-            const double sII = sqrt((s11 * s11 + 2.0 * s12 * s12 + 2.0 * s13 * s13 + s22 * s22 +
-                                     2.0 * s23 * s23 + s33 * s33) / 2.0);
-            const double eII = a.rh.gd0[iv] * pow(sII, a.rh.npow[iv] - 1);
-            ev[0] += eII * s11; ev[1] += eII * s12; ev[2] += eII * s13;
-            ev[3] += eII * s22; ev[4] += eII * s23; ev[5] += eII * s33;
+        const double *s = a.y + 7L * a.np + 12L * iv + 6;
+        for (int q = 0; q < 6; q++)
+            v[2L * a.np + 6L * iv + q] = volume_rate(a.rh, iv, q, s[0], s[1], s[2], s[3], s[4], s[5]) -
+                                         a.rh.ebg[6L * iv + q];
+    }
+}
+
+// ---- control: RKQSm decision ---------------------------------------------------
+
+// by one thread, once every element's error is in
+__device__ void decide(Ctl *ctl)
+{
+    const double SAFETY = 0.7, PGROW = -0.2, PSHRNK = -0.15, ERRCON = 1.89e-4;
+    double errmax = __longlong_as_double((long long)ctl->errbits);
+    ctl->errbits = 0ull;
+    if (ctl->status) return;
+    if (ctl->nonfinite) {
+        ctl->status = UCG_E_NONFINITE;
+        ctl->active = 0;
+        return;
+    }
+    errmax = errmax / ctl->epsilon;
+    double h = ctl->h;
+    if (errmax > 1.0) {
+        h = h * SAFETY * pow(errmax, PSHRNK);
+        if (h < 0.5 * h) h = 0.5 * h;   // never taken (ode45.f90:83)
+        ctl->h = h;
+        ctl->clamped = 0;   // a shrunk step stays short of t_stop
+        ctl->rejected += 1;
+        ctl->need_stage1 = 0;
+        ctl->pending = 0;
+        const double tnew = 0.0 + h;     // the main loop passes t0 = 0 (ratestate.f90:317)
+        if (tnew == 0.0) {
+            ctl->status = UCG_E_STEP_UNDERFLOW;
+            ctl->active = 0;
         }
-        for (int q = 0; q < 6; q++) {
-            ks[o + q] = ev[q];
-            const long j = 2L * a.np + 6L * iv + q;
-            double vq = ev[q] - a.rh.ebg[6L * iv + q];
-            if (a.anchored) {
-                if (S == 1) a.v1[j] = vq;
-                else vq -= a.v1[j];
-            }
-            a.v[j] = vq;
+    } else {
+        double hnext;
+        if (errmax > ERRCON) hnext = SAFETY * h * pow(errmax, PGROW);
+        else hnext = 10.0 * h;
+        if (hnext > ctl->hmax) hnext = ctl->hmax;
+        ctl->hdid = h;
+        ctl->time = ctl->clamped ? ctl->t_stop : ctl->time + h;
+        ctl->dt_next = hnext;
+        ctl->h = hnext;
+        ctl->clamped = 0;
+        if (ctl->stop_on && ctl->time < ctl->t_stop && ctl->time + hnext > ctl->t_stop) {
+            ctl->h = ctl->t_stop - ctl->time;
+            ctl->clamped = 1;
+        }
+        ctl->accepted += 1;
+        ctl->pending = 1;
+        ctl->vmax = 0.0;
+        ctl->need_stage1 = 1;
+        if (ctl->time >= ctl->t_end || ctl->accepted >= ctl->step_target) ctl->active = 0;
+    }
+}
+
+// End of stage 6 in one warp of every CTA that takes part: its largest error, and
+// the decision by the CTA that comes last.
+__device__ __forceinline__ void attempt_end(Ctl *ctl, double mx, bool bad)
+{
+    for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+    bad = __any_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+        if (mx > 0.0) atomic_max_pos(&ctl->errbits, mx);
+        if (bad) ctl->nonfinite = 1;
+        __threadfence();
+        if (atomicAdd(&ctl->ticket, 1) == (int)gridDim.x - 1) {
+            __threadfence();
+            ctl->ticket = 0;
+            decide(ctl);
         }
     }
+}
+
+// a rejected attempt repeats with a smaller step from the same k_1: stage 2 of a
+// patch for the new h
+__device__ __forceinline__ void retry_stage2(const StageArgs &a, Ctl *ctl, int e, int c, bool on, double h)
+{
+    const long i = 7L * e + c;
+    double yn = 0.0;
+    if (on) {
+        yn = stage_comb(1, LaneState{a.y[i], 0, 0, 0, 1, true}, a.k[0][i], h);
+        a.ys[i] = yn;
+    }
+    const double ts = __shfl_sync(~0u, yn, 2, 8), td = __shfl_sync(~0u, yn, 3, 8), lv = __shfl_sync(~0u, yn, 6, 8);
+    if (!on || c > 1) return;
+    double vel, cr, sr;
+    patch_slip(ts, td, lv, vel, cr, sr);
+    if (!isfinite(vel) || !isfinite(cr) || !isfinite(sr)) ctl->nonfinite = 1;
+    double v = vel * (c == 0 ? cr : sr) - (c == 0 ? a.fr.vpl_c[e] : a.fr.vpl_s[e]);
+    if (a.anchored) v -= a.v1[2L * e + c];
+    a.vn[2L * e + c] = v;
+}
+
+// and of a volume
+__device__ __forceinline__ void retry_stage2_volume(const StageArgs &a, int iv, int c, bool on, double h)
+{
+    const long i = 7L * a.np + 12L * iv + c;
+    double yn = 0.0;
+    if (on) {
+        yn = stage_comb(1, LaneState{a.y[i], 0, 0, 0, 1, true}, a.k[0][i], h);
+        a.ys[i] = yn;
+    }
+    double s[6];
+#pragma unroll
+    for (int q = 0; q < 6; q++) s[q] = __shfl_sync(~0u, yn, 6 + q, 16);
+    if (!on || c > 5) return;
+    const long j = 2L * a.np + 6L * iv + c;
+    double v = volume_rate(a.rh, iv, c, s[0], s[1], s[2], s[3], s[4], s[5]) - a.rh.ebg[6L * iv + c];
+    if (a.anchored) v -= a.v1[j];
+    a.vn[j] = v;
 }
 
 // ---- traction product fused with the right-hand side ----------------------------
 //
-// K (m x n, row-major) times v.  A CTA owns blocks of consecutive rows: in FP64
-// 12 rows, 4 patches (3 rows each) or 2 volumes (6 rows each); in the split
-// forms 24.  Its 8 warps sweep interleaved column slices of a block's rows, so
-// every v element loaded feeds all of them; K is streamed once.  The row
-// sums are reduced across lanes and warps, and the elementwise rate-state
-// (ratestate.f90:731-776) or Maxwell (viscouscycles.f90:1072-1080) epilogue of
-// each owned element runs on the reduced values, writing k_s directly.
+// K (m x n, row-major) times v.  A CTA owns an equal share of the patches and of
+// the volumes (to one element), taken in blocks of at most 12 rows in FP64, 4
+// patches (3 rows each) or 2 volumes (6 rows each), and 24 in the split forms.  Its
+// 8 warps sweep interleaved column slices of a block's rows, so every v element
+// loaded feeds all of them; K is streamed once.  The row sums are reduced across
+// lanes and warps, and a warp of its own runs the block's elements through the
+// stage (patch_finish, volume_finish) while the others are at the next block.
 
 constexpr int MV_WARPS = 8;
 
-__device__ __forceinline__ double2 ld_stream(const double *p)
+// Stage S of every patch from a traction vector already formed (the hierarchical
+// product): the epilogue of k_traction without the matvec, 32 patches a CTA.
+__global__ void __launch_bounds__(256) k_rhs_t(int S, StageArgs a, Ctl *ctl, const double *__restrict__ t)
 {
-    double2 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
-    return r;
-}
-
-__device__ __forceinline__ void rhs_patch(const StageArgs &a, const double *yy, double *ks, int e,
-                                          const double t[3])
-{
-    const long o = 7L * e;
-    const double rake = atan2(yy[o + 3], yy[o + 2]);
-    const double vel = exp(yy[o + 6] * LG10);
-    const double L = a.fr.L[e], bb = a.fr.b[e], sg = a.fr.sig[e], aa = a.fr.a[e], eta = a.fr.damping[e];
-    const double cr = cos(rake), sr = sin(rake);
-    const double dth = (exp(-yy[o + 5] * LG10) - vel / L) / LG10;
-    const double dtau = t[0] * cr + t[1] * sr;
-    const double dv = (dtau - bb * sg * dth * LG10) / (aa * sg + eta * vel) / LG10;
-    const double corr = eta * vel * dv * LG10;
-    ks[o + 2] = t[0] - corr * cr;
-    ks[o + 3] = t[1] - corr * sr;
-    ks[o + 4] = t[2];
-    ks[o + 5] = dth;
-    ks[o + 6] = dv;
-}
-
-// Right-hand side of every patch from a traction vector already formed (the
-// hierarchical product): the epilogue of k_traction without the matvec.
-template <int S>
-__global__ void k_rhs_t(StageArgs a, const Ctl *ctl, const double *__restrict__ t)
-{
+    pdl_enter();
     if (!ctl_live(ctl)) return;
-    if (S == 1 && !ctl->need_stage1) return;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= a.np) return;
-    const double *yy = (S == 1) ? a.y : a.ys;
-    double tr[3] = {t[3L * e], t[3L * e + 1], t[3L * e + 2]};
-    if (a.anchored) {
-        // anchored stages: stage 1 keeps t1 = K v1, the others add K (v - v1) to it
-        for (int q = 0; q < 3; q++) {
-            if (S == 1) a.t1[3L * e + q] = tr[q];
-            else tr[q] += a.t1[3L * e + q];
+    const double h = ctl->h;
+    const int c = threadIdx.x & 7, e = blockIdx.x * 32 + (threadIdx.x >> 3);
+    const bool on = e < a.np && c < 7;
+    double mx = 0.0;
+    bool bad = false;
+    if (S == 1 && !ctl->need_stage1) {
+        retry_stage2(a, ctl, e, c, on, h);
+        return;
+    }
+    LaneState st;
+    const double ys = lane_load(S, a, ctl, 7L * e + c, on, st);
+    const PatchTerms p = patch_terms(S, ctl, patch_friction(a, e, c, on), c, on, ys);
+    double tr[3] = {0.0, 0.0, 0.0};
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) tr[q] = t[3L * e + q];
+        if (a.anchored) {
+            // anchored stages: stage 1 keeps t1 = K v1, the others add K (v - v1) to it
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                if (S > 1) tr[q] += a.t1[3L * e + q];
+                else if (c == q) a.t1[3L * e + q] = tr[q];
+            }
         }
     }
-    rhs_patch(a, yy, a.k[S - 1], e, tr);
+    patch_finish(S, a, ctl, e, c, h, st, p, tr[0], tr[1], tr[2], mx, bad);
+    if (S == 6) {
+        __shared__ double smx[8];
+        __shared__ int sbad[8];
+        for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        bad = __any_sync(0xffffffffu, bad);
+        if ((threadIdx.x & 31) == 0) {
+            smx[threadIdx.x >> 5] = mx;
+            sbad[threadIdx.x >> 5] = bad;
+        }
+        // every thread's candidate and rates are out before the CTA counts itself in
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            const int w = threadIdx.x & 7;
+            attempt_end(ctl, smx[w], sbad[w] != 0);
+        }
+    }
 }
 
 // ---- TMA bulk-copy pipeline ------------------------------------------------------
@@ -328,7 +599,6 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 // element traits: FP64 K (2 columns per thread) or split-BF16 pairs (4 per thread)
 template <class KT> struct TmTraits;
@@ -353,7 +623,6 @@ constexpr size_t tm_smem_bytes()
 {
     return (size_t)TmTraits<KT>::STAGES * TmTraits<KT>::ROWS * TmTraits<KT>::CH * sizeof(KT);
 }
-
 // the thread's PER values of v for one chunk, loaded once and used for all the
 // rows of the stage; then one row's contribution
 template <class KT> struct TmV;
@@ -456,31 +725,128 @@ __device__ __forceinline__ void tm_accumulate<__half>(const __half *srow, int cl
     acc += (double)p;
 }
 
-template <int S, class KT>
-__global__ void __launch_bounds__((MV_WARPS + 1) * 32, 1) k_traction(const KT *__restrict__ K, long n, long ldk,
-        const float *__restrict__ scale, StageArgs a, Ctl *ctl, int pblocks, int vblocks)
+// Sums of ROWS values over the lanes of a warp, row by row, each the xor butterfly
+// with offsets 16, 8, 4, 2, 1.  Instead of 5 exchanges a row, each step sends half
+// of the rows a lane still holds to its partner and keeps the other half (13
+// exchanges and adds for 12 rows instead of 60: 1.38 -> 0.3 us of a launch at N = 512).  Lane
+// l ends up with the sum of row warp_row(l).
+template <int ROWS>
+struct RowHalves {
+    static constexpr int n1 = ROWS / 2, n2 = (n1 + 1) / 2, n3 = (n2 + 1) / 2, n4 = (n3 + 1) / 2,
+                         n5 = (n4 + 1) / 2;
+};
+template <int N, int H>
+__device__ __forceinline__ void fold_rows(double *x, int lane, int off)
+{
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < H; i++) {
+        const double hi = H + i < N ? x[H + i] : 0.0;
+        const double keep = up ? hi : x[i], give = up ? x[i] : hi;
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, give, off);
+    }
+}
+template <int ROWS>
+__device__ __forceinline__ double warp_row_sums(double *x, int lane)
+{
+    using R = RowHalves<ROWS>;
+    fold_rows<ROWS, R::n1>(x, lane, 16);
+    fold_rows<R::n1, R::n2>(x, lane, 8);
+    fold_rows<R::n2, R::n3>(x, lane, 4);
+    fold_rows<R::n3, R::n4>(x, lane, 2);
+    fold_rows<R::n4, R::n5>(x, lane, 1);
+    static_assert(R::n5 == 1, "at most 32 rows");
+    return x[0];
+}
+// the row of a lane's sum, ROWS where it has none
+template <int ROWS>
+__device__ __forceinline__ int warp_row(int lane)
+{
+    using R = RowHalves<ROWS>;
+    int n = ROWS, row = 0;
+    const int h[5] = {R::n1, R::n2, R::n3, R::n4, R::n5};
+#pragma unroll
+    for (int s = 0; s < 5; s++) {
+        const bool up = lane & (16 >> s);
+        row += up ? h[s] : 0;
+        n = up ? n - h[s] : n < h[s] ? n : h[s];
+    }
+    return n > 0 ? row : ROWS;
+}
+
+// the blocks of a CTA: its patches, then its volumes, each share in blocks of
+// nearly equal size
+template <class KT>
+struct Share {
+    static constexpr int PB = TmTraits<KT>::ROWS / 3, VB = TmTraits<KT>::ROWS / 6;   // patches, volumes per block
+    int p0, np, v0, nv;     // this CTA's patches and volumes
+    int bp, bv;             // their blocks
+    long prows;             // rows of all patches
+
+    __device__ __forceinline__ Share(int npatch, int nvol, int cta, int ctas)
+    {
+        // the first `more` CTAs take one element above the quotient
+        const int qp = npatch / ctas, mp = npatch - qp * ctas, qv = nvol / ctas, mv = nvol - qv * ctas;
+        p0 = qp * cta + min(cta, mp);
+        np = qp + (cta < mp);
+        v0 = qv * cta + min(cta, mv);
+        nv = qv + (cta < mv);
+        bp = (np + PB - 1) / PB;
+        bv = (nv + VB - 1) / VB;
+        prows = 3L * npatch;
+    }
+    __device__ __forceinline__ int blocks() const { return bp + bv; }
+    // first row and rows of block b, its first element and their number
+    __device__ __forceinline__ bool block(int b, long &row0, int &nrows, int &e0, int &nel) const
+    {
+        const bool patch = b < bp;
+        if (patch) {
+            const int lo = np * b / bp;
+            nel = np * (b + 1) / bp - lo;
+            e0 = p0 + lo;
+            row0 = 3L * e0;
+            nrows = 3 * nel;
+        } else {
+            const int q = b - bp, lo = nv * q / bv;
+            nel = nv * (q + 1) / bv - lo;
+            e0 = v0 + lo;
+            row0 = prows + 6L * e0;
+            nrows = 6 * nel;
+        }
+        return patch;
+    }
+};
+
+constexpr int TM_THREADS = (MV_WARPS + 2) * 32;   // consumers, producer, epilogue
+
+// named barriers between the consumers and the epilogue warp: buffer b of the row
+// sums is full (1 + b), or read and free again (3 + b)
+__device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(MV_WARPS * 32 + 32) : "memory"); }
+__device__ __forceinline__ void bar_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(MV_WARPS * 32 + 32) : "memory"); }
+
+// The stage number is an argument: the six launches of an attempt run the same
+// code, which then stays in the instruction caches.
+template <class KT>
+__global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__restrict__ K, long n,
+        long ldk, const float *__restrict__ scale, StageArgs a, Ctl *ctl)
 {
     using Tr = TmTraits<KT>;
     using Acc = typename Tr::Acc;
-    constexpr int CH = Tr::CH, PER = Tr::PER, ROWS = Tr::ROWS, STAGES = Tr::STAGES;
-    constexpr int PB = ROWS / 3, VB = ROWS / 6;   // patches, volumes per block
-    pdl_enter();
-    if (!ctl_live(ctl)) return;
-    if (S == 1 && !ctl->need_stage1) return;
+    constexpr int CH = Tr::CH, PER = Tr::PER, ROWS = Tr::ROWS, stages = Tr::STAGES;
     extern __shared__ __align__(128) unsigned char tm_smem[];
     KT *stage = reinterpret_cast<KT *>(tm_smem);
-    __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES];
-    // row sums of a block, double-buffered: the few threads that run a
-    // block's epilogue read one buffer while the other warps already
-    // accumulate the next block into the other; the next block's barrier
-    // orders the epilogue before its buffer comes round again
+    __shared__ __align__(8) uint64_t full[Tr::STAGES], empty[Tr::STAGES];
     __shared__ double red[2][MV_WARPS][ROWS];
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nblk = pblocks + vblocks;
-    const long nch = (n + CH - 1) / CH;
+    // the next launch may come as soon as there is room: before its own wait it only
+    // reads K and the friction, which no launch changes
+    pdl_launch();
+    const Share<KT> share(a.np, a.nvol, blockIdx.x, gridDim.x);
+    const int nblk = share.blocks();
+    const int nch = (int)((n + CH - 1) / CH);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; s++) {
+        for (int s = 0; s < stages; s++) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], MV_WARPS);
         }
@@ -489,78 +855,158 @@ __global__ void __launch_bounds__((MV_WARPS + 1) * 32, 1) k_traction(const KT *_
     }
     __syncthreads();
 
-    auto block_rows = [&](int blk, long &row0, int &nrows, int &e0, int &nel, bool &patch) {
-        patch = blk < pblocks;
-        if (patch) {
-            e0 = blk * PB; nel = min(PB, a.np - e0); row0 = 3L * e0; nrows = 3 * nel;
-        } else {
-            e0 = (blk - pblocks) * VB; nel = min(VB, a.nvol - e0); row0 = 3L * a.np + 6L * e0; nrows = 6 * nel;
-        }
-    };
-
-    const unsigned long long wait_lim = ctl->wait_ns ? ctl->wait_ns : TM_TIMEOUT_NS;
     if (warp == MV_WARPS) {
-        // producer: one lane issues the row copies of each (block, chunk) item
-        if (lane == 0) {
-            long item = 0;
-            // (test_hold: the first CTA issues nothing, its consumers' waits run out)
-            const bool hold = ctl->test_hold && blockIdx.x == 0;
-            for (int blk = blockIdx.x; blk < nblk && !abort_flag && !hold; blk += gridDim.x) {
-                long row0; int nrows, e0, nel; bool patch;
-                block_rows(blk, row0, nrows, e0, nel, patch);
-                for (long ch = 0; ch < nch; ch++, item++) {
-                    const int s = (int)(item % STAGES);
-                    const uint32_t ph = (uint32_t)((item / STAGES) & 1);
-                    if (!mbar_wait(&empty[s], ph ^ 1u, &abort_flag)) {
-                        abort_flag = 1;
-                        ctl->status = UCG_E_TIMEOUT;
-                        break;
-                    }
-                    const long c0 = ch * CH;
-                    const long w = min((long)CH, ldk - c0);
-                    const uint32_t rowbytes = (uint32_t)(w * sizeof(KT));
-                    mbar_expect_tx(&full[s], rowbytes * nrows);
-                    KT *dst = stage + (size_t)s * ROWS * CH;
-                    for (int r = 0; r < nrows; r++)
-                        bulk_g2s(dst + (size_t)r * CH, K + (row0 + r) * ldk + c0, rowbytes, &full[s]);
+        // producer: one lane issues the row copies of each (block, chunk) item.  K does
+        // not depend on the launches before, so the first stages are filled before
+        // the wait for them.
+        if (lane != 0) return;
+        int item = 0, s = 0, ph = 0, b = 0, ch = 0, nrows = 0, e0, nel;
+        long row0 = 0;
+        const int total = nblk * nch;
+        auto issue = [&]() {
+            if (ch == 0) share.block(b, row0, nrows, e0, nel);
+            const long c0 = (long)ch * CH;
+            const long w = min((long)CH, ldk - c0);
+            const uint32_t rowbytes = (uint32_t)(w * sizeof(KT));
+            mbar_expect_tx(&full[s], rowbytes * nrows);
+            KT *dst = stage + (size_t)s * ROWS * CH;
+            for (int r = 0; r < nrows; r++)
+                bulk_g2s(dst + (size_t)r * CH, K + (row0 + r) * ldk + c0, rowbytes, &full[s]);
+            item++;
+            if (++ch == nch) { ch = 0; b++; }
+            if (++s == stages) { s = 0; ph ^= 1; }
+        };
+        // (test_hold: the first CTA issues nothing, its consumers' waits run out)
+        const bool hold = blockIdx.x == 0 && *(volatile int *)&ctl->test_hold;
+        if (!hold)
+            while (item < total && item < stages) issue();
+        pdl_wait();
+        if (!hold && ctl_live(ctl) && !(S == 1 && !ctl->need_stage1)) {
+            while (item < total && !*(volatile int *)&abort_flag) {
+                if (!mbar_wait(&empty[s], ph ^ 1, &abort_flag)) {
+                    abort_flag = 1;
+                    ctl->status = UCG_E_TIMEOUT;
+                    break;
                 }
+                issue();
             }
-            // items are issued in order, so the last copies into each stage are
-            // those of the last STAGES items: they land before the CTA may exit,
-            // also when the consumers gave up on them (bounded at the normal limit)
-            for (long i = item > STAGES ? item - STAGES : 0; i < item; i++)
-                mbar_wait(&full[i % STAGES], (uint32_t)((i / STAGES) & 1), nullptr);
         }
+        // items are issued in order, so the last copies into each stage are those
+        // of the last items: they land before the CTA may exit, also when the
+        // consumers gave up on them or never started (bounded at the normal limit)
+        for (int i = item > stages ? item - stages : 0; i < item; i++)
+            mbar_wait(&full[i % stages], (uint32_t)((i / stages) & 1), nullptr);
         return;
     }
 
-    // consumers
-    const double *yy = (S == 1) ? a.y : a.ys;
-    double *ks = a.k[S - 1];
-    long item = 0;
-    const int t = threadIdx.x;
-    int rb = 0;
-    for (int blk = blockIdx.x; blk < nblk; blk += gridDim.x, rb ^= 1) {
-        long row0; int nrows, e0, nel; bool patch;
-        block_rows(blk, row0, nrows, e0, nel, patch);
+    if (warp == MV_WARPS + 1) {
+        // epilogue: the elements of one block after the other.  The first patches'
+        // friction is asked for before the wait for the launches before.
+        PatchFriction fr{1, 1, 0, 0, 1, 1, 0};
+        {
+            long row0;
+            int nrows, e0, nel;
+            if (nblk > 0 && share.block(0, row0, nrows, e0, nel))
+                fr = patch_friction(a, e0 + (lane >> 3), lane & 7, (lane >> 3) < nel && (lane & 7) < 7);
+        }
+        pdl_wait();
+        if (!ctl_live(ctl)) return;
+        const double h = ctl->h;
+        const bool first = S > 1 || ctl->need_stage1;
+        double mx = 0.0;
+        bool bad = false;
+        for (int b = 0; b < nblk; b++) {
+            long row0;
+            int nrows, e0, nel;
+            const bool patch = share.block(b, row0, nrows, e0, nel);
+            const int per = patch ? 4 : 2, c = patch ? lane & 7 : lane & 15, nc = patch ? 7 : 12;
+            const int sub = patch ? lane >> 3 : lane >> 4;
+            for (int q0 = 0; q0 < nel; q0 += per) {
+                const int q = q0 + sub, e = e0 + q;
+                const bool on = q < nel && c < nc;
+                if (!first) {
+                    if (patch) retry_stage2(a, ctl, e, c, on, h);
+                    else retry_stage2_volume(a, e, c, on, h);
+                    continue;
+                }
+                // rows of the element that this lane adds up over the warps: a patch's
+                // three in its lanes 0..2, a volume's six in 6..11
+                const int r = patch ? 3 * q + c : 6 * q + c - 6;
+                const bool sum = on && (patch ? c < 3 : c > 5);
+                if (patch) {
+                    LaneState st;
+                    const double ys = lane_load(S, a, ctl, 7L * e + c, on, st);
+                    if (b + q0 > 0) fr = patch_friction(a, e, c, on);
+                    const PatchTerms p = patch_terms(S, ctl, fr, c, on, ys);
+                    if (q0 == 0) bar_wait(1 + (b & 1));
+                    double t = 0.0;
+                    if (sum) {
+                        for (int w = 0; w < MV_WARPS; w++) t += red[b & 1][w][r];
+                        if (scale) t = t * (double)scale[row0 + r];
+                        if (a.anchored) {
+                            if (S == 1) a.t1[row0 + r] = t;
+                            else t += a.t1[row0 + r];
+                        }
+                    }
+                    const double t0 = __shfl_sync(~0u, t, 0, 8), t1 = __shfl_sync(~0u, t, 1, 8),
+                                 t2 = __shfl_sync(~0u, t, 2, 8);
+                    if (!abort_flag) patch_finish(S, a, ctl, e, c, h, st, p, t0, t1, t2, mx, bad);
+                } else {
+                    LaneState st;
+                    const double ys = lane_load(S, a, ctl, 7L * a.np + 12L * e + c, on, st);
+                    double sv[6];
+#pragma unroll
+                    for (int k = 0; k < 6; k++) sv[k] = __shfl_sync(~0u, ys, 6 + k, 16);
+                    const double ev = on && c < 6 ? volume_rate(a.rh, e, c, sv[0], sv[1], sv[2], sv[3], sv[4], sv[5])
+                                                  : 0.0;
+                    if (q0 == 0) bar_wait(1 + (b & 1));
+                    double t = 0.0;
+                    if (sum) {
+                        for (int w = 0; w < MV_WARPS; w++) t += red[b & 1][w][r];
+                        if (scale) t = t * (double)scale[row0 + r];
+                        if (a.anchored) {
+                            if (S == 1) a.t1[row0 + r] = t;
+                            else t += a.t1[row0 + r];
+                        }
+                    }
+                    if (!abort_flag) volume_finish(S, a, e, c, h, st, ev, t, mx, bad);
+                }
+            }
+            // the buffer comes round again two blocks later
+            if (first && b + 2 < nblk) bar_arrive(3 + (b & 1));
+        }
+        if (S == 6 && a.next) attempt_end(ctl, mx, bad);
+        return;
+    }
+
+    // consumers.  The first v values are asked for together with the control block.
+    const int t = threadIdx.x, cl = PER * t;
+    pdl_wait();
+    TmVRaw<KT> vn;
+    if (cl < n) tm_load_raw<KT>(a.v, cl, n, vn);
+    const unsigned long long wait_ns = ctl->wait_ns;   // (looked at only where a wait has to be timed)
+    if (!ctl_live(ctl)) return;
+    if (S == 1 && !ctl->need_stage1) return;
+    int s = 0, ph = 0;
+    for (int b = 0; b < nblk; b++) {
+        long row0;
+        int nrows, e0, nel;
+        share.block(b, row0, nrows, e0, nel);
         Acc acc[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; r++) acc[r] = Acc(0);
         // v does not depend on the stage: each chunk's values are loaded one
         // chunk ahead, so their latency overlaps the previous chunk's products
-        const int cl = PER * t;
-        TmVRaw<KT> vn;
-        if (cl < n) tm_load_raw<KT>(a.v, cl, n, vn);
-        for (long ch = 0; ch < nch; ch++, item++) {
-            const int s = (int)(item % STAGES);
-            const uint32_t ph = (uint32_t)((item / STAGES) & 1);
+        for (int ch = 0; ch < nch; ch++) {
             // on a timed-out wait every consumer keeps walking the same item
             // sequence without computing, so all of them reach each named barrier
-            const long c = ch * CH + cl;
+            const long c = (long)ch * CH + cl;
             TmV<KT> vr;
             if (c < n) tm_cook<KT>(vn, vr);
-            if (c + CH < n) tm_load_raw<KT>(a.v, c + CH, n, vn);
-            const bool ready = !abort_flag && mbar_wait(&full[s], ph, &abort_flag, wait_lim);
+            const long cn = ch + 1 < nch ? c + CH : cl;   // the next block starts at its first chunk
+            if (cn < n) tm_load_raw<KT>(a.v, cn, n, vn);
+            const bool ready = !abort_flag && (mbar_try(&full[s], ph) ||
+                                               mbar_wait(&full[s], ph, &abort_flag, wait_ns ? wait_ns : TM_TIMEOUT_NS));
             if (!ready && !abort_flag) {
                 abort_flag = 1;
                 ctl->status = UCG_E_TIMEOUT;
@@ -573,141 +1019,14 @@ __global__ void __launch_bounds__((MV_WARPS + 1) * 32, 1) k_traction(const KT *_
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
+            if (++s == stages) { s = 0; ph ^= 1; }
         }
-        double rs[ROWS];
-#pragma unroll
-        for (int r = 0; r < ROWS; r++) {
-            Acc x = acc[r];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-            rs[r] = (double)x;
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < ROWS; r++) red[rb][warp][r] = rs[r];
-        }
-        consumer_sync();
-        if (t < nel && !abort_flag) {
-            const int q = t;
-            if (patch) {
-                double tr[3];
-                for (int c3 = 0; c3 < 3; c3++) {
-                    double sum = 0.0;
-                    for (int w = 0; w < MV_WARPS; w++) sum += red[rb][w][3 * q + c3];
-                    tr[c3] = scale ? sum * (double)scale[row0 + 3 * q + c3] : sum;
-                    if (a.anchored) {
-                        const long row = row0 + 3 * q + c3;
-                        if (S == 1) a.t1[row] = tr[c3];
-                        else tr[c3] += a.t1[row];
-                    }
-                }
-                rhs_patch(a, yy, ks, e0 + q, tr);
-            } else {
-                const long o = 7L * a.np + 12L * (e0 + q);
-                for (int c6 = 0; c6 < 6; c6++) {
-                    double sum = 0.0;
-                    for (int w = 0; w < MV_WARPS; w++) sum += red[rb][w][6 * q + c6];
-                    double sv = scale ? sum * (double)scale[row0 + 6 * q + c6] : sum;
-                    if (a.anchored) {
-                        const long row = row0 + 6 * q + c6;
-                        if (S == 1) a.t1[row] = sv;
-                        else sv += a.t1[row];
-                    }
-                    ks[o + 6 + c6] = sv;
-                }
-            }
-        }
-    }
-}
-
-// ---- finish: candidate, error estimate, error norm ------------------------------
-
-__global__ void k_finish(StageArgs a, Ctl *ctl)
-{
-    pdl_enter();
-    if (!ctl_live(ctl)) return;
-    const double h = ctl->h;
-    double mx = 0.0;
-    bool bad = false;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.len; i += (long)gridDim.x * blockDim.x) {
-        const double k1 = a.k[0][i], k3 = a.k[2][i], k4 = a.k[3][i], k5 = a.k[4][i], k6 = a.k[5][i];
-        // ode45.f90:184-200
-        double r = __dmul_rn(C1, k1);
-        r = __dadd_rn(r, __dmul_rn(C3, k3));
-        r = __dadd_rn(r, __dmul_rn(C4, k4));
-        r = __dadd_rn(r, __dmul_rn(C6, k6));
-        const double yc = __dadd_rn(a.y[i], __dmul_rn(h, r));
-        double e = __dmul_rn(DC1, k1);
-        e = __dadd_rn(e, __dmul_rn(DC3, k3));
-        e = __dadd_rn(e, __dmul_rn(DC4, k4));
-        e = __dadd_rn(e, __dmul_rn(DC5, k5));
-        e = __dadd_rn(e, __dmul_rn(DC6, k6));
-        e = __dmul_rn(h, e);
-        a.ycand[i] = yc;
-        a.yerr[i] = e;
-        // MAXVAL semantics: a NaN ratio (0/0) does not raise the maximum; an
-        // infinite one does and drives the step to underflow as in the
-        // reference.  A non-finite candidate state is reported as such.
-        const double q = fabs(e / a.yscal[i]);
-        if (!isfinite(yc)) bad = true;
-        mx = fmax(mx, q);
-    }
-    for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (mx > 0.0) atomic_max_pos(&ctl->errbits, mx);
-        if (bad) ctl->nonfinite = 1;
-    }
-}
-
-// ---- control: RKQSm decision ---------------------------------------------------
-
-__global__ void k_control(Ctl *ctl)
-{
-    pdl_enter();
-    if (!ctl_live(ctl)) return;
-    const double SAFETY = 0.7, PGROW = -0.2, PSHRNK = -0.15, ERRCON = 1.89e-4;
-    double errmax = __longlong_as_double((long long)ctl->errbits);
-    ctl->errbits = 0ull;
-    if (ctl->nonfinite) {
-        ctl->status = UCG_E_NONFINITE;
-        ctl->active = 0;
-        return;
-    }
-    errmax = errmax / ctl->epsilon;
-    double h = ctl->h;
-    if (errmax > 1.0) {
-        h = h * SAFETY * pow(errmax, PSHRNK);
-        if (h < 0.5 * h) h = 0.5 * h;   // never taken (ode45.f90:83)
-        ctl->h = h;
-        ctl->clamped = 0;   // a shrunk step stays short of t_stop
-        ctl->rejected += 1;
-        ctl->need_stage1 = 0;
-        ctl->pending = 0;
-        const double tnew = 0.0 + h;     // the main loop passes t0 = 0 (ratestate.f90:317)
-        if (tnew == 0.0) {
-            ctl->status = UCG_E_STEP_UNDERFLOW;
-            ctl->active = 0;
-        }
-    } else {
-        double hnext;
-        if (errmax > ERRCON) hnext = SAFETY * h * pow(errmax, PGROW);
-        else hnext = 10.0 * h;
-        if (hnext > ctl->hmax) hnext = ctl->hmax;
-        ctl->hdid = h;
-        ctl->time = ctl->clamped ? ctl->t_stop : ctl->time + h;
-        ctl->dt_next = hnext;
-        ctl->h = hnext;
-        ctl->clamped = 0;
-        if (ctl->stop_on && ctl->time < ctl->t_stop && ctl->time + hnext > ctl->t_stop) {
-            ctl->h = ctl->t_stop - ctl->time;
-            ctl->clamped = 1;
-        }
-        ctl->accepted += 1;
-        ctl->pending = 1;
-        ctl->vmax = 0.0;
-        ctl->need_stage1 = 1;
-        if (ctl->time >= ctl->t_end || ctl->accepted >= ctl->step_target) ctl->active = 0;
+        const double x = warp_row_sums<ROWS>(acc, lane);
+        if (b > 1) bar_wait(3 + (b & 1));
+        const int row = warp_row<ROWS>(lane);
+        if (row < ROWS) red[b & 1][warp][row] = x;
+        __syncwarp();
+        bar_arrive(1 + (b & 1));
     }
 }
 
@@ -765,9 +1084,8 @@ __global__ void k_commit(StageArgs a, const Ctl *ctl)
 {
     pdl_enter();
     if (!ctl->pending) return;
-    double *y = const_cast<double *>(a.y);
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.len; i += (long)gridDim.x * blockDim.x)
-        y[i] = a.ycand[i];
+        a.y[i] = a.ycand[i];
 }
 
 __global__ void k_clear_pending(Ctl *ctl)
@@ -794,13 +1112,18 @@ void rk_drop_graph(ucg_ctx *c)
     c->attempt_graph = nullptr;
 }
 
-static StageArgs stage_args(ucg_ctx *c, int s)
+// stage s reads its source rates from buffer s & 1 and writes the next stage's
+// into the other
+static StageArgs stage_args(ucg_ctx *c, int s, int next)
 {
     StageArgs a;
     a.y = c->st.y;
-    a.ys = (s == 1) ? c->st.y : c->st.ytmp;
+    a.ys = c->st.ytmp;
     for (int j = 0; j < 6; j++) a.k[j] = c->st.k[j];
-    a.v = c->st.v;
+    a.ks = c->st.k[s - 1];
+    a.v = c->st.v[s & 1];
+    a.vn = c->st.v[(s + 1) & 1];
+    a.next = next;
     a.ycand = c->st.ycand;
     a.yerr = c->st.yerr;
     a.yscal = c->st.yscal;
@@ -825,7 +1148,8 @@ int rk_alloc(ucg_ctx *c)
         if (cudaMalloc(b, sizeof(double) * (len + 2)) != cudaSuccess) return UCG_E_OOM;
         cudaMemsetAsync(*b, 0, sizeof(double) * (len + 2), c->stream);
     }
-    if (cudaMalloc(&c->st.v, sizeof(double) * (c->n + 2)) != cudaSuccess) return UCG_E_OOM;
+    for (double *&v : c->st.v)
+        if (cudaMalloc(&v, sizeof(double) * (c->n + 2)) != cudaSuccess) return UCG_E_OOM;
     if (cudaMalloc(&c->st.v1, sizeof(double) * (c->n + 2)) != cudaSuccess) return UCG_E_OOM;
     if (cudaMalloc(&c->st.t1, sizeof(double) * (c->m + 2)) != cudaSuccess) return UCG_E_OOM;
     if (cudaMalloc(&c->ctl, sizeof(Ctl)) != cudaSuccess) return UCG_E_OOM;
@@ -848,7 +1172,7 @@ void rk_free(ucg_ctx *c)
 {
     double **bufs[] = {&c->st.y, &c->st.ycand, &c->st.ytmp, &c->st.yerr, &c->st.yscal,
                        &c->st.k[0], &c->st.k[1], &c->st.k[2], &c->st.k[3], &c->st.k[4], &c->st.k[5],
-                       &c->st.v, &c->st.v1, &c->st.t1};
+                       &c->st.v[0], &c->st.v[1], &c->st.v1, &c->st.t1};
     for (double **b : bufs) {
         if (*b) cudaFree(*b);
         *b = nullptr;
@@ -873,81 +1197,67 @@ void rk_free(ucg_ctx *c)
     c->attempt_graph = nullptr;
 }
 
-// the blocks of ROWS rows (patches first, then volumes) and the grid
 template <class KT>
-static int traction_grid(ucg_ctx *c, int *pb, int *vb)
+static void launch_traction_t(ucg_ctx *c, int S, const StageArgs &a, const KT *K, long ldk, const float *scale)
 {
-    constexpr int PB = TmTraits<KT>::ROWS / 3, VB = TmTraits<KT>::ROWS / 6;
-    const int np = c->nr + c->nt;
-    *pb = (np + PB - 1) / PB;
-    *vb = (c->nv + VB - 1) / VB;
-    const int blocks = *pb + *vb;
-    const int cap = c->sms;
-    return blocks < cap ? blocks : cap;
-}
-
-template <int S, class KT>
-static void launch_traction_t(ucg_ctx *c, const StageArgs &a, const KT *K, long ldk, const float *scale)
-{
-    int pb, vb;
-    const int grid = traction_grid<KT>(c, &pb, &vb);
+    const int ne = a.np + a.nvol, grid = ne < c->sms ? ne : c->sms;
     const size_t smem = tm_smem_bytes<KT>();
-    auto kfn = k_traction<S, KT>;
+    auto kfn = k_traction<KT>;
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kfn, dim3(grid), dim3((MV_WARPS + 1) * 32), smem, c->stream, K, c->n, ldk, scale, a, c->ctl, pb, vb);
+    launch_pdl(kfn, dim3(grid), dim3(TM_THREADS), smem, c->stream, S, K, c->n, ldk, scale, a, c->ctl);
 }
 
-template <int S>
-static void launch_traction(ucg_ctx *c, const StageArgs &a)
+static void launch_traction(ucg_ctx *c, int S, const StageArgs &a)
 {
     if (S > 1 && c->precision == UCG_PREC_SPLIT_BF16 && rk_anchored(c) && c->Khi_plane) {
         // anchored stages multiply the increments by the fp16 plane
-        launch_traction_t<S, __half>(c, a, c->Khi_plane, c->ldk_split, c->Kscale);
+        launch_traction_t<__half>(c, S, a, c->Khi_plane, c->ldk_split, c->Kscale);
     } else if ((c->precision == UCG_PREC_SPLIT_BF16 || c->precision == UCG_PREC_SPLIT_PAIR) && c->Ksp) {
-        launch_traction_t<S, float>(c, a, c->Ksp, c->ldk_split, c->Kscale);
+        launch_traction_t<float>(c, S, a, c->Ksp, c->ldk_split, c->Kscale);
     } else {
-        launch_traction_t<S, double>(c, a, c->K, c->n, nullptr);
+        launch_traction_t<double>(c, S, a, c->K, c->n, nullptr);
     }
 }
 
-template <int S>
-static void enqueue_stage(ucg_ctx *c)
+static void enqueue_stage(ucg_ctx *c, int S, int next)
 {
-    const int ne = c->nr + c->nt + c->nv;
-    StageArgs a = stage_args(c, S);
-    launch_pdl(k_prologue<S>, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl);
-    c->launches.count += 1;
+    const StageArgs a = stage_args(c, S, next);
     if (c->precision == UCG_PREC_HMATRIX || c->precision == UCG_PREC_HMATRIX_SPLIT) {
         double *t = hmatrix_t(c);
-        if (c->precision == UCG_PREC_HMATRIX) hmatrix_apply(c, c->st.v, t);
-        else hmatrix_apply_split(c, c->st.v, t, true);     // every stage on the FP32 planes (hi + lo)
-        k_rhs_t<S><<<(c->nr + c->nt + 127) / 128, 128, 0, c->stream>>>(a, c->ctl, t);
-        c->launches.count += 1;
-        return;
+        if (c->precision == UCG_PREC_HMATRIX) hmatrix_apply(c, a.v, t);
+        else hmatrix_apply_split(c, a.v, t, true);     // every stage on the FP32 planes (hi + lo)
+        k_rhs_t<<<(a.np + 31) / 32, 256, 0, c->stream>>>(S, a, c->ctl, t);
+    } else {
+        launch_traction(c, S, a);
     }
-    launch_traction<S>(c, a);
+    c->launches.count += 1;
+}
+
+// source rates of the state y, before a run's first attempt
+static void enqueue_begin(ucg_ctx *c)
+{
+    const StageArgs a = stage_args(c, 1, 0);
+    const int ne = a.np + a.nvol;
+    launch_pdl(k_begin, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl, c->st.v[1]);
     c->launches.count += 1;
 }
 
 static void enqueue_attempt_raw(ucg_ctx *c)
 {
-    enqueue_stage<1>(c);
+    enqueue_stage(c, 1, 1);
     // the recorder joins the attempt (and its graph) only while recording is on
     if (c->rec_host.enabled) {
-        launch_pdl(k_record, dim3(c->sms), dim3(256), 0, c->stream, stage_args(c, 1), c->ctl, c->rec);
+        launch_pdl(k_record, dim3(c->sms), dim3(256), 0, c->stream, stage_args(c, 1, 0), c->ctl, c->rec);
         c->launches.count += 1;
     }
-    enqueue_stage<2>(c);
-    enqueue_stage<3>(c);
-    enqueue_stage<4>(c);
-    enqueue_stage<5>(c);
-    enqueue_stage<6>(c);
-    StageArgs a = stage_args(c, 6);
-    const int fin_grid = (int)((c->state_len + 255) / 256 < (long)c->sms * 4 ? (c->state_len + 255) / 256 : c->sms * 4);
-    launch_pdl(k_finish, dim3(fin_grid > 0 ? fin_grid : 1), dim3(256), 0, c->stream, a, c->ctl);
-    launch_pdl(k_control, dim3(1), dim3(1), 0, c->stream, c->ctl);
-    c->launches.count += 2;
+    enqueue_stage(c, 2, 1);
+    enqueue_stage(c, 3, 1);
+    enqueue_stage(c, 4, 1);
+    enqueue_stage(c, 5, 1);
+    enqueue_stage(c, 6, 1);
 }
+
+void rk_enqueue_begin(ucg_ctx *c) { enqueue_begin(c); }
 
 void rk_enqueue_attempt(ucg_ctx *c)
 {
@@ -978,7 +1288,7 @@ void rk_enqueue_attempt(ucg_ctx *c)
 
 void rk_enqueue_commit(ucg_ctx *c)
 {
-    StageArgs a = stage_args(c, 1);
+    StageArgs a = stage_args(c, 1, 0);
     launch_pdl(k_commit, dim3((unsigned)((c->state_len + 255) / 256)), dim3(256), 0, c->stream, a, c->ctl);
     launch_pdl(k_clear_pending, dim3(1), dim3(1), 0, c->stream, c->ctl);
     c->launches.count += 2;
@@ -996,13 +1306,13 @@ int rk_profile_traction(ucg_ctx *c, int reps, double *ms)
     h->active = 1;
     h->status = 0;
     UCG_CUDA(cudaMemcpyAsync(c->ctl, h, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
-    StageArgs a = stage_args(c, 2);
+    StageArgs a = stage_args(c, 2, 0);
     cudaEvent_t e0, e1;
     UCG_CUDA(cudaEventCreate(&e0));
     UCG_CUDA(cudaEventCreate(&e1));
     UCG_CUDA(cudaEventRecord(e0, c->stream));
     for (int r = 0; r < reps; r++) {
-        launch_traction<2>(c, a);
+        launch_traction(c, 2, a);
     }
     c->launches.count += reps;
     UCG_CUDA(cudaEventRecord(e1, c->stream));
@@ -1083,8 +1393,10 @@ int rk_odefun(ucg_ctx *c)
     h->pending = 0;
     h->vmax = 0.0;
     h->nonfinite = 0;
+    h->ticket = 0;
     UCG_CUDA(cudaMemcpyAsync(c->ctl, h, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
-    enqueue_stage<1>(c);
+    enqueue_begin(c);
+    enqueue_stage(c, 1, 0);
     UCG_CUDA(cudaGetLastError());
     UCG_CUDA(cudaMemcpyAsync(h, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
     UCG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1179,9 +1491,9 @@ extern "C" int ucg_odefun_noalloc(const double *K, long n, long m, int np, const
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
     StageArgs sa{};
-    sa.y = y;
-    sa.ys = const_cast<double *>(y);   // stage 1 reads y and writes nothing into it
-    for (int j = 0; j < 6; j++) sa.k[j] = dydt;
+    sa.y = const_cast<double *>(y);   // stage 1 without a pending candidate reads y only
+    sa.ys = sa.y;
+    sa.ks = dydt;
     sa.v = v;
     sa.fr.vpl_c = const_cast<double *>(Vpl_cos_rake);
     sa.fr.vpl_s = const_cast<double *>(Vpl_sin_rake);
@@ -1197,15 +1509,14 @@ extern "C" int ucg_odefun_noalloc(const double *K, long n, long m, int np, const
     int dcount = 0;
     if (cudaDeviceGetAttribute(&dcount, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || dcount <= 0)
         return UCG_E_CUDA;
+    const int grid = np < dcount ? np : dcount;
     const size_t smem = tm_smem_bytes<double>();
-    auto kfn = k_traction<1, double>;
+    auto kfn = k_traction<double>;
     if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return UCG_E_CUDA;
     k_noalloc_ctl_reset<<<1, 1, 0, st>>>(ctl);
-    k_prologue<1><<<(np + 127) / 128, 128, 0, st>>>(sa, ctl);
-    const int pb = (np + 3) / 4;
-    const int grid = pb < dcount ? pb : dcount;
-    kfn<<<grid, (MV_WARPS + 1) * 32, smem, st>>>(K, n, n, nullptr, sa, ctl, pb, 0);
+    k_begin<<<(np + 127) / 128, 128, 0, st>>>(sa, ctl, v);
+    kfn<<<grid, TM_THREADS, smem, st>>>(1, K, n, n, nullptr, sa, ctl);
     if (status) k_noalloc_status<<<1, 1, 0, st>>>(ctl, status);
     return cudaGetLastError() == cudaSuccess ? UCG_OK : UCG_E_CUDA;
 }

@@ -741,6 +741,7 @@ int ucg_set_tolerance(ucg_ctx *c, double epsilon, double max_step)
 // control block every `batch` attempts
 static int drive(ucg_ctx *c, int batch)
 {
+    rk_enqueue_begin(c);
     for (;;) {
         for (int i = 0; i < batch; i++) rk_enqueue_attempt(c);
         int rc = pull_ctl(c);
@@ -775,6 +776,7 @@ int ucg_rkqs(ucg_ctx *c, double *t, double *y, const double *dydt, const double 
     h->pending = 0;
     h->status = 0;
     h->active = 1;
+    h->ticket = 0;
     h->nonfinite = 0;
     h->errbits = 0;
     h->epsilon = c->epsilon;
@@ -812,6 +814,7 @@ int ucg_step(ucg_ctx *c, double *time, double *y, double *dydt, double *dt_next,
     h->pending = 0;
     h->status = 0;
     h->active = 1;
+    h->ticket = 0;
     h->nonfinite = 0;
     h->errbits = 0;
     h->vmax = 0.0;
@@ -928,6 +931,8 @@ int ucg_run(ucg_ctx *c, double t_end, long max_steps, long *steps)
         h->step_target = acc0 + max_steps;
         h->status = 0;
         h->active = 1;
+        h->ticket = 0;
+        h->errbits = 0;
         h->nonfinite = 0;
         h->epsilon = c->epsilon;
         h->hmax = c->hmax;

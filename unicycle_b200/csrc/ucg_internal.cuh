@@ -37,7 +37,8 @@ struct Ctl {
     // test_hold makes the product's first CTA issue no copies, so that its
     // consumers wait on data that never comes and give up
     unsigned long long wait_ns;
-    int test_hold, pad_;
+    int test_hold;
+    int ticket;        // CTAs of stage 6 that are done (the last one decides the attempt)
 };
 
 // Device-side output recorder (the reference's export/exportPoints,
@@ -106,7 +107,7 @@ struct Rheology {
 struct Stages {
     double *y, *ycand, *ytmp, *yerr, *yscal;
     double *k[6];            // k[0] = dydt (stage 1), k[1..5] = AK2..AK6
-    double *v;               // source-DOF velocity / strain-rate vector (n)
+    double *v[2];            // source-DOF velocity / strain-rate vector (n), alternating by stage
     double *t;               // receiver traction / stress (m) for odefun reads
     double *v1, *t1;         // stage-1 anchor of the split-BF16 product (n, m)
 };
@@ -219,6 +220,7 @@ void rk_free(ucg_ctx *c);
 int rk_odefun(ucg_ctx *c);                  // k[0] = f(y) on device, sets vmax
 int rk_test_wait_timeout(ucg_ctx *c, unsigned long long wait_ns, int hold);
 int rk_profile_traction(ucg_ctx *c, int reps, double *ms);
+void rk_enqueue_begin(ucg_ctx *c);          // source rates of the state, before a run's first attempt
 void rk_enqueue_attempt(ucg_ctx *c);        // one Cash-Karp attempt + control
 void rk_enqueue_commit(ucg_ctx *c);         // copy a pending candidate into y
 bool rk_anchored(const ucg_ctx *c);         // stages contract increments over the stage-1 anchor
