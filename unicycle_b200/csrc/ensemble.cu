@@ -3091,7 +3091,7 @@ int ucg_ens_create(ucg_ensemble **out, int device)
     E->h_glob->hmax = E->hmax;
     E->h_glob->ev_on = 1.0e-3;
     E->h_glob->ev_off = 1.0e-4;
-    cudaMemcpy(E->d_glob, E->h_glob, sizeof(EnsGlobal), cudaMemcpyHostToDevice);
+    ucg::copy_in(E->d_glob, E->h_glob, sizeof(EnsGlobal));
     *out = E;
     return UCG_OK;
 }
@@ -3177,7 +3177,7 @@ int ucg_ens_add_geometry(ucg_ensemble *E, ucg_ctx *c, int n_instances, int *geom
             x.need_stage1 = 1;
             x.status = UCG_E_STATE;    // no state yet: inactive until ucg_ens_set_state
         }
-        e = cudaMemcpy(g.ctl, ctl.data(), sizeof(InstCtl) * g.ninst, cudaMemcpyHostToDevice);
+        e = ucg::copy_in(g.ctl, ctl.data(), sizeof(InstCtl) * g.ninst);
     }
     if (e == cudaSuccess && !hier) {
         // K = diag(row scale) (block scale) (hi + 2^-11 lo): the contraction's
@@ -3249,7 +3249,7 @@ int ucg_ens_set_state(ucg_ensemble *E, int gi, int inst, double time, const doub
     const long len = 7L * g.np;
     ECUDA(cudaSetDevice(E->device));
     ECUDA(cudaStreamSynchronize(E->stream));
-    ECUDA(cudaMemcpy(g.state + (long)inst * len, y, sizeof(double) * len, cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(g.state + (long)inst * len, y, sizeof(double) * len));
     InstCtl x;
     memset(&x, 0, sizeof x);
     x.h = dt_next;
@@ -3258,7 +3258,7 @@ int ucg_ens_set_state(ucg_ensemble *E, int gi, int inst, double time, const doub
     x.need_stage1 = 1;
     x.status = UCG_OK;
     x.thmin_key = ~0ull;
-    ECUDA(cudaMemcpy(g.ctl + inst, &x, sizeof x, cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(g.ctl + inst, &x, sizeof x));
     return UCG_OK;
 }
 
@@ -3323,7 +3323,7 @@ int ucg_ens_set_increment_terms(ucg_ensemble *E, int terms)
     ECUDA(cudaStreamSynchronize(E->stream));
     E->inc_full = terms == 3;
     E->h_glob->inc_full = E->inc_full ? 1 : 0;
-    ECUDA(cudaMemcpy(&E->d_glob->inc_full, &E->h_glob->inc_full, sizeof(int), cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(&E->d_glob->inc_full, &E->h_glob->inc_full, sizeof(int)));
     if (E->graph) cudaGraphExecDestroy(E->graph);   // the launches differ: capture again
     E->graph = nullptr;
     return UCG_OK;
@@ -3337,9 +3337,9 @@ int ucg_ens_test_wait_timeout(ucg_ensemble *E, long wait_ns, int hold)
     E->h_glob->wait_ns = (unsigned long long)wait_ns;
     E->h_glob->test_hold = hold != 0;
     E->h_glob->err = 0;
-    ECUDA(cudaMemcpy(&E->d_glob->wait_ns, &E->h_glob->wait_ns, sizeof(unsigned long long), cudaMemcpyHostToDevice));
-    ECUDA(cudaMemcpy(&E->d_glob->test_hold, &E->h_glob->test_hold, sizeof(int), cudaMemcpyHostToDevice));
-    ECUDA(cudaMemcpy(&E->d_glob->err, &E->h_glob->err, sizeof(int), cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(&E->d_glob->wait_ns, &E->h_glob->wait_ns, sizeof(unsigned long long)));
+    ECUDA(ucg::copy_in(&E->d_glob->test_hold, &E->h_glob->test_hold, sizeof(int)));
+    ECUDA(ucg::copy_in(&E->d_glob->err, &E->h_glob->err, sizeof(int)));
     return UCG_OK;
 }
 
@@ -3587,7 +3587,7 @@ int ucg_ens_set_step_model(ucg_ensemble *E, const ucg_mlp *model)
     ECUDA(cudaSetDevice(E->device));
     ECUDA(cudaStreamSynchronize(E->stream));
     mlp_device_params(model, &E->h_glob->mlp_P, &E->h_glob->mlp_N);
-    ECUDA(cudaMemcpy(&E->d_glob->mlp_P, &E->h_glob->mlp_P, sizeof(void *) * 2, cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(&E->d_glob->mlp_P, &E->h_glob->mlp_P, sizeof(void *) * 2));
     return UCG_OK;
 }
 
@@ -3634,7 +3634,7 @@ int ucg_ens_set_event_threshold(ucg_ensemble *E, double vmax_on, double vmax_off
     ECUDA(cudaStreamSynchronize(E->stream));
     E->h_glob->ev_on = vmax_on;
     E->h_glob->ev_off = vmax_off;
-    ECUDA(cudaMemcpy(&E->d_glob->ev_on, &E->h_glob->ev_on, 2 * sizeof(double), cudaMemcpyHostToDevice));
+    ECUDA(ucg::copy_in(&E->d_glob->ev_on, &E->h_glob->ev_on, 2 * sizeof(double)));
     return UCG_OK;
 }
 

@@ -40,6 +40,7 @@
 #include <cuda_bf16.h>
 #include <cstring>
 #include <numeric>
+#include <utility>
 #include <vector>
 #include "ucg_internal.cuh"
 #include "blocks.cuh"
@@ -68,8 +69,10 @@ struct HLeafTerm {           // the rows of one row leaf in one block (or a rang
 };
 
 struct HChunk {              // consecutive terms [q0, q1) of one row leaf, packed contiguously
-    int leaf, q0, q1;
+    int rows, cols;          // rows of the leaf; columns over the terms
+    int q0, q1;
     int bytes;               // of its panel (a multiple of 16)
+    int id;                  // its place in the leaf's order: slot of its partial sums
     long off;                // panel offset (doubles)
 };
 
@@ -86,14 +89,15 @@ struct HMat {
     double build_ms = 0;
     // product
     HLowRank *lr_d = nullptr;            // low-rank descriptors
-    int2 *items_d = nullptr;             // (block, rank index) work items of the first kernel
+    int2 *items_d = nullptr;             // (block, first rank index) work items of the first kernel
     long n_items = 0;
     HLeafTerm *terms_d = nullptr;        // per row leaf, its terms (consecutive)
     HChunk *chunks_d = nullptr;          // work of the row kernel
     int *leaf_chunk_d = nullptr;         // per row leaf, its chunks (CSR)
-    int n_chunks = 0;
+    int n_chunks = 0, n_dense_chunks = 0;
     int *leaf_e0_d = nullptr;            // row leaves: element ranges (permuted)
     int n_leaves = 0, max_leaf = 0;
+    int max_cols = 0;                    // columns of the widest chunk
     double *z_d = nullptr;               // low-rank workspace
     long nz = 0;
     double *part_d = nullptr;            // partial row sums (chunk, row)
@@ -423,6 +427,29 @@ int keep_blocks(ucg_ctx *c, const std::vector<KeepJob> &jobs)
 }
 
 // ---- the product --------------------------------------------------------------------
+//
+// The kernels are launched with programmatic dependent launch: each lets the next
+// be scheduled and waits for the ones before it itself, the row kernel only after
+// it has asked for its panel, which does not depend on them.
+
+__device__ __forceinline__ void hm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void hm_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static cudaError_t hm_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
 
 // v in the permuted element order (so that every block's columns are a
 // contiguous range of xp)
@@ -434,36 +461,29 @@ __global__ void k_hm_gather(const int *__restrict__ perm, int np, const double *
     reinterpret_cast<double2 *>(xp)[i] = reinterpret_cast<const double2 *>(v)[perm[i]];
 }
 
-// z_b[l] = V_b[l, :] . xp(sigma_b): one warp per (block, rank index)
-__global__ void k_hm_z(const HLowRank *__restrict__ lr, const int2 *__restrict__ items, long n_items,
-                       const double *__restrict__ xp, double *__restrict__ z)
-{
-    const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= n_items) return;
-    const int2 it = items[w];
-    const HLowRank b = lr[it.x];
-    const double2 *Vl = reinterpret_cast<const double2 *>(b.V + (long)it.y * b.n);
-    const double2 *x = reinterpret_cast<const double2 *>(xp + 2L * b.s0);
-    double s0 = 0.0, s1 = 0.0;
-    for (int j = lane; j < (b.n >> 1); j += 32) {
-        const double2 a = Vl[j], xx = x[j];
-        s0 = fma(a.x, xx.x, s0);
-        s1 = fma(a.y, xx.y, s1);
-    }
-    double s = s0 + s1;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) z[b.zoff + it.y] = s;
-}
-
+// Two kernels form the partial sums, bound by HBM.  The first works on z and, in
+// every other CTA, on the chunks of dense blocks, which do not need it; the second
+// on the chunks of low-rank factors, which do.  (z by itself took 29 us of a product
+// at N = 7,200 for 17 us worth of its 110 MB, the few longest blocks being the tail.)
+//
+// z_b[l] = V_b[l, :] . xp(sigma_b): one warp per (block, HM_ZR rank indices), which
+// share the loads of xp, with HM_ZU loads of each in flight, the longest blocks
+// first.  Stage of an attempt at N = 7,200, FP64 / split / N = 1,800: HM_ZR, HM_ZU =
+// 2, 2 135 / 92 / 26.5 us; 1, 4 148 / 91 / 27; 2, 4 139 / 91 / 27; 4, 2 132 / 97 / 30.
+//
 // Partial row sums over one chunk of a row leaf's terms: the chunk's panel
 // (at most HM_CHUNK_BYTES, contiguous) arrives in shared memory by one bulk
-// copy; then one thread per row multiplies its rows of the pieces by their
-// slices of xp (dense) or z (low-rank).  k_hm_reduce adds a leaf's chunks in
-// order.  Many small CTAs per SM keep many copies in flight.  The wait for the
-// copy is bounded (about 4 s); when it runs out the chunk writes NaN, which the
-// integrator reports as a non-finite rate, and the kernel flags status.
-constexpr long HM_CHUNK_BYTES = 16 * 1024;
+// copy, asked for first of all; meanwhile the entries of xp (dense) or z
+// (low-rank) that multiply its columns are gathered beside it; then one thread per
+// row multiplies.  k_hm_reduce (in an attempt k_hm_stage, rk.cu) adds a leaf's
+// chunks in order.  Many small CTAs per SM keep many copies in flight.  The wait
+// for the copy is bounded (about 4 s); when it runs out the chunk writes NaN, which
+// the integrator reports as a non-finite rate, and the kernel flags status.  24 KB
+// chunks: 16 KB 4 % slower for the split form, whose chunks are half as large, 32 KB
+// 5 % for FP64 (fewer CTAs an SM).  Before these kernels a stage took 150 / 120 / 46.
+constexpr long HM_CHUNK_BYTES = 24 * 1024;
+constexpr int HM_THREADS = 128;   // at most; the launch takes a leaf's rows rounded up to warps
+constexpr int HM_ZR = 2, HM_ZU = 2;
 constexpr unsigned long long HM_TIMEOUT_NS = 4000000000ull;
 
 __device__ __forceinline__ uint32_t hm_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -489,58 +509,6 @@ __device__ __forceinline__ bool hm_wait(uint64_t *bar)
             if (t - t0 > HM_TIMEOUT_NS) return false;
         }
     }
-}
-
-__global__ void __launch_bounds__(128) k_hm_rows(const HLeafTerm *__restrict__ terms,
-        const HChunk *__restrict__ chunks, const int *__restrict__ leaf_e0, const double *__restrict__ panel,
-        const double *__restrict__ xp, const double *__restrict__ z, double *__restrict__ part, int rows_max,
-        int *status)
-{
-    extern __shared__ __align__(128) double sm[];
-    __shared__ __align__(8) uint64_t bar;
-    const HChunk ch = chunks[blockIdx.x];
-    const int rows = 3 * (leaf_e0[ch.leaf + 1] - leaf_e0[ch.leaf]);
-    const int i = threadIdx.x;
-    if (ch.bytes == 0) {
-        if (i < rows) part[(long)blockIdx.x * rows_max + i] = 0.0;
-        return;
-    }
-    if (i == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(hm_smem(&bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (i == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(hm_smem(&bar)), "r"(ch.bytes)
-                     : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(hm_smem(sm)), "l"(panel + ch.off), "r"(ch.bytes), "r"(hm_smem(&bar)) : "memory");
-    }
-    const bool ok = hm_wait(&bar);
-    if (!ok) {
-        if (i == 0) atomicExch(status, 1);
-        if (i < rows) part[(long)blockIdx.x * rows_max + i] = nan("");
-        hm_wait(&bar);   // the copy may still land in this CTA's shared memory: wait once more (bounded)
-        return;
-    }
-    if (i >= rows) return;
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    long off = 0;
-    for (int q = ch.q0; q < ch.q1; q++) {
-        const HLeafTerm T = terms[q];
-        const double *x = (T.xsel ? z : xp) + T.xoff;
-        const double *col = sm + off + i;
-        int j = 0;
-        for (; j + 3 < T.cols; j += 4) {
-            a0 = fma(col[j * rows], x[j], a0);
-            a1 = fma(col[(j + 1) * rows], x[j + 1], a1);
-            a2 = fma(col[(j + 2) * rows], x[j + 2], a2);
-            a3 = fma(col[(j + 3) * rows], x[j + 3], a3);
-        }
-        for (; j < T.cols; j++) a0 = fma(col[j * rows], x[j], a0);
-        off += ((long)rows * T.cols + 7) & ~7L;
-    }
-    part[(long)blockIdx.x * rows_max + i] = (a0 + a1) + (a2 + a3);
 }
 
 // ---- split (hi + lo) form ---------------------------------------------------------------
@@ -582,102 +550,182 @@ __global__ void k_split_jobs(const SplitJob *__restrict__ jobs, __nv_bfloat16 *_
     for (long t = threadIdx.x; t < J.n; t += blockDim.x) split32(J.src[t], hi[J.dst + t], lo[J.dst + t]);
 }
 
-template <bool LO>
-__global__ void k_hm_z_split(const HLowRank *__restrict__ lr, const int2 *__restrict__ items, long n_items,
-                             const double *__restrict__ xp, const __nv_bfloat16 *__restrict__ vh,
-                             const __nv_bfloat16 *__restrict__ vl, double *__restrict__ z)
-{
-    const long w = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= n_items) return;
-    const int2 it = items[w];
-    const HLowRank b = lr[it.x];
-    const long o = b.vsoff + (long)it.y * b.n;
-    const __nv_bfloat162 *h2 = reinterpret_cast<const __nv_bfloat162 *>(vh + o);
-    const __nv_bfloat162 *l2 = reinterpret_cast<const __nv_bfloat162 *>(vl + o);
-    const double2 *x = reinterpret_cast<const double2 *>(xp + 2L * b.s0);
-    double s0 = 0.0, s1 = 0.0;
-    for (int j = lane; j < (b.n >> 1); j += 32) {
-        const double2 xx = x[j];
-        double a0, a1;
-        if (LO) {
-            a0 = join32(h2[j].x, l2[j].x);
-            a1 = join32(h2[j].y, l2[j].y);
-        } else {
-            const float2 a = __bfloat1622float2(h2[j]);
-            a0 = a.x;
-            a1 = a.y;
-        }
-        s0 = fma(a0, xx.x, s0);
-        s1 = fma(a1, xx.y, s1);
+// ---- product kernels ----------------------------------------------------------------
+
+struct HmProduct {
+    const HLowRank *lr;
+    const int2 *items;        // (block, first rank index) of the z warps
+    long n_items;
+    const HLeafTerm *terms;
+    const HChunk *chunks;     // of dense blocks, then of low-rank factors
+    int n_dense;
+    const double *panel;                      // FP64 form
+    const __nv_bfloat16 *ph, *pl, *vh, *vl;   // split form
+    const double *xp;
+    double *z, *part;
+    int rows_max;
+    int *status;
+};
+
+// two columns of V of one rank index, FP64 or split
+template <bool SPLIT> struct ZPair;
+template <> struct ZPair<false> {
+    const double2 *v;
+    double2 x;
+    __device__ __forceinline__ void at(const HmProduct &P, const HLowRank &b, int l)
+    {
+        (void)P;
+        v = reinterpret_cast<const double2 *>(b.V + (long)l * b.n);
     }
-    double s = s0 + s1;
-    for (int o2 = 16; o2 > 0; o2 >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o2);
-    if (lane == 0) z[b.zoff + it.y] = s;
+    __device__ __forceinline__ void load(int j) { x = v[j]; }
+    __device__ __forceinline__ double2 get() const { return x; }
+};
+template <> struct ZPair<true> {
+    const __nv_bfloat162 *h, *l;
+    __nv_bfloat162 xh, xl;
+    __device__ __forceinline__ void at(const HmProduct &P, const HLowRank &b, int r)
+    {
+        const long o = b.vsoff + (long)r * b.n;
+        h = reinterpret_cast<const __nv_bfloat162 *>(P.vh + o);
+        l = reinterpret_cast<const __nv_bfloat162 *>(P.vl + o);
+    }
+    __device__ __forceinline__ void load(int j) { xh = h[j]; xl = l[j]; }
+    __device__ __forceinline__ double2 get() const
+    {
+        return make_double2((double)join32(xh.x, xl.x), (double)join32(xh.y, xl.y));
+    }
+};
+
+template <bool SPLIT>
+__device__ __forceinline__ void hm_z(const HmProduct &P, long w)
+{
+    if (w >= P.n_items) return;
+    const int lane = threadIdx.x & 31;
+    const int2 it = P.items[w];
+    const HLowRank b = P.lr[it.x];
+    const int n2 = b.n >> 1;
+    const double2 *x = reinterpret_cast<const double2 *>(P.xp + 2L * b.s0);
+    ZPair<SPLIT> v[HM_ZR][HM_ZU];
+#pragma unroll
+    for (int r = 0; r < HM_ZR; r++)
+#pragma unroll
+        for (int u = 0; u < HM_ZU; u++)   // past the last rank: the last one again, not stored
+            v[r][u].at(P, b, min(it.y + r, b.k - 1));
+    double s[HM_ZR][2] = {};
+    auto add = [&](int r, double2 a, double2 xx) {
+        s[r][0] = fma(a.x, xx.x, s[r][0]);
+        s[r][1] = fma(a.y, xx.y, s[r][1]);
+    };
+    int j = lane;
+    for (; j + 32 * (HM_ZU - 1) < n2; j += 32 * HM_ZU) {
+        double2 xx[HM_ZU];
+#pragma unroll
+        for (int u = 0; u < HM_ZU; u++) {
+            xx[u] = x[j + 32 * u];
+#pragma unroll
+            for (int r = 0; r < HM_ZR; r++) v[r][u].load(j + 32 * u);
+        }
+#pragma unroll
+        for (int u = 0; u < HM_ZU; u++)
+#pragma unroll
+            for (int r = 0; r < HM_ZR; r++) add(r, v[r][u].get(), xx[u]);
+    }
+    for (; j < n2; j += 32) {
+        const double2 xx = x[j];
+#pragma unroll
+        for (int r = 0; r < HM_ZR; r++) {
+            v[r][0].load(j);
+            add(r, v[r][0].get(), xx);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < HM_ZR; r++) {
+        double t = s[r][0] + s[r][1];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0 && it.y + r < b.k) P.z[b.zoff + it.y + r] = t;
+    }
 }
 
-// k_hm_rows on the split panels: the chunk's hi (and lo) bf16 values arrive by
-// bulk copy (a chunk of e values is 2 e bytes per half)
-template <bool LO>
-__global__ void __launch_bounds__(128) k_hm_rows_split(const HLeafTerm *__restrict__ terms,
-        const HChunk *__restrict__ chunks, const int *__restrict__ leaf_e0, const __nv_bfloat16 *__restrict__ ph,
-        const __nv_bfloat16 *__restrict__ pl, const double *__restrict__ xp, const double *__restrict__ z,
-        double *__restrict__ part, int rows_max, int *status)
+// FIRST: z and the chunks of dense blocks; otherwise the chunks of low-rank factors
+template <bool SPLIT, bool FIRST>
+__global__ void __launch_bounds__(HM_THREADS) k_hm_rows(HmProduct P, int zblocks)
 {
-    extern __shared__ __align__(128) __nv_bfloat16 sb[];
+    extern __shared__ __align__(128) double sm[];
     __shared__ __align__(8) uint64_t bar;
-    const HChunk ch = chunks[blockIdx.x];
-    const int rows = 3 * (leaf_e0[ch.leaf + 1] - leaf_e0[ch.leaf]);
-    const int i = threadIdx.x;
-    const long nel = ch.bytes / 8;            // values in the chunk
-    const uint32_t half = (uint32_t)(2 * nel);
-    if (nel == 0) {
-        if (i < rows) part[(long)blockIdx.x * rows_max + i] = 0.0;
-        return;
+    int slot = blockIdx.x;
+    if (FIRST) {
+        // z and dense CTAs in turn until one kind runs out: z alone keeps too little in flight
+        const int both = 2 * min(zblocks, P.n_dense);
+        const bool z = slot < both ? !(slot & 1) : zblocks > P.n_dense;
+        slot = slot < both ? slot >> 1 : slot - (both >> 1);
+        if (z) {
+            hm_pdl_wait();
+            hm_pdl_launch();
+            hm_z<SPLIT>(P, ((long)slot * blockDim.x + threadIdx.x) >> 5);
+            return;
+        }
     }
-    if (i == 0) {
+    const HChunk ch = P.chunks[FIRST ? slot : P.n_dense + slot];
+    const int i = threadIdx.x, rows = ch.rows;
+    const long nel = ch.bytes / 8;                      // values in the chunk
+    const __nv_bfloat16 *sb = reinterpret_cast<const __nv_bfloat16 *>(sm);   // split: hi, then lo
+    double *xs = sm + (SPLIT ? HM_CHUNK_BYTES / 16 : HM_CHUNK_BYTES / 8);
+    if (i == 0 && nel) {
+        const uint32_t bytes = SPLIT ? ch.bytes / 2 : ch.bytes, half = ch.bytes / 4;
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(hm_smem(&bar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(hm_smem(&bar)), "r"(bytes)
+                     : "memory");
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(hm_smem(sm)), "l"(SPLIT ? (const void *)(P.ph + ch.off) : (const void *)(P.panel + ch.off)),
+                     "r"(SPLIT ? half : bytes), "r"(hm_smem(&bar)) : "memory");
+        if (SPLIT)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                         ::"r"(hm_smem(sb + nel)), "l"(P.pl + ch.off), "r"(half), "r"(hm_smem(&bar)) : "memory");
+    }
+    hm_pdl_wait();
+    hm_pdl_launch();
+    double *part = P.part + (long)ch.id * P.rows_max + i;
+    if (nel == 0) {
+        if (i < rows) *part = 0.0;
+        return;
+    }
+    // the entries of xp or z, column after column of the chunk's terms
+    for (int q = ch.q0, base = 0; q < ch.q1; q++) {
+        const HLeafTerm T = P.terms[q];
+        const double *x = (FIRST ? P.xp : P.z) + T.xoff;
+        for (int j = i; j < T.cols; j += blockDim.x) xs[base + j] = x[j];
+        base += T.cols;
     }
     __syncthreads();
-    if (i == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(hm_smem(&bar)),
-                     "r"(LO ? 2 * half : half) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                     ::"r"(hm_smem(sb)), "l"(ph + ch.off), "r"(half), "r"(hm_smem(&bar)) : "memory");
-        if (LO)
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                         ::"r"(hm_smem(sb + nel)), "l"(pl + ch.off), "r"(half), "r"(hm_smem(&bar)) : "memory");
-    }
-    const bool ok = hm_wait(&bar);
-    if (!__syncthreads_and(ok ? 1 : 0)) {
-        if (i == 0) atomicExch(status, 1);
-        if (i < rows) part[(long)blockIdx.x * rows_max + i] = nan("");
-        hm_wait(&bar);
+    if (!hm_wait(&bar)) {
+        if (i == 0) atomicExch(P.status, 1);
+        if (i < rows) *part = nan("");
+        hm_wait(&bar);   // the copy may still land in this CTA's shared memory: wait once more (bounded)
         return;
     }
     if (i >= rows) return;
     double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
     long off = 0;
+    const double *x = xs;
     for (int q = ch.q0; q < ch.q1; q++) {
-        const HLeafTerm T = terms[q];
-        const double *x = (T.xsel ? z : xp) + T.xoff;
-        const __nv_bfloat16 *col = sb + off + i;
+        const int cols = P.terms[q].cols;
         auto val = [&](int j) -> double {
-            if (LO) return (double)join32(col[(long)j * rows], col[nel + (long)j * rows]);
-            return (double)__bfloat162float(col[(long)j * rows]);
+            const long o = off + i + (long)j * rows;
+            return SPLIT ? (double)join32(sb[o], sb[nel + o]) : sm[o];
         };
         int j = 0;
-        for (; j + 3 < T.cols; j += 4) {
+        for (; j + 3 < cols; j += 4) {
             a0 = fma(val(j), x[j], a0);
             a1 = fma(val(j + 1), x[j + 1], a1);
             a2 = fma(val(j + 2), x[j + 2], a2);
             a3 = fma(val(j + 3), x[j + 3], a3);
         }
-        for (; j < T.cols; j++) a0 = fma(val(j), x[j], a0);
-        off += ((long)rows * T.cols + 7) & ~7L;
+        for (; j < cols; j++) a0 = fma(val(j), x[j], a0);
+        off += ((long)rows * cols + 7) & ~7L;
+        x += cols;
     }
-    part[(long)blockIdx.x * rows_max + i] = (a0 + a1) + (a2 + a3);
+    *part = (a0 + a1) + (a2 + a3);
 }
 
 struct PackJob {
@@ -787,7 +835,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     leaf_e0.push_back(np);
     for (int L = 0; L < h->n_leaves; L++) h->max_leaf = std::max(h->max_leaf, leaf_e0[L + 1] - leaf_e0[L]);
     UCG_CUDA(cudaMalloc(&h->perm_d, sizeof(int) * np));
-    UCG_CUDA(cudaMemcpy(h->perm_d, h->perm.data(), sizeof(int) * np, cudaMemcpyHostToDevice));
+    UCG_CUDA(cudaMemcpyAsync(h->perm_d, h->perm.data(), sizeof(int) * np, cudaMemcpyHostToDevice, c->stream));
 
     if ((rc = block_sources_build(c, okada_mode, h->perm, &bs))) return rc;
 
@@ -975,7 +1023,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         } else if (d.rank > 0) {
             const int id = (int)lr.size();
             lr.push_back({d.A, d.V, d.rank, m, n, B.s0, B.r0, (int)zoff});
-            for (int l = 0; l < d.rank; l++) items.push_back(make_int2(id, l));
+            for (int l = 0; l < d.rank; l += HM_ZR) items.push_back(make_int2(id, l));
             for (int L = leaf_of(B.r0); L < h->n_leaves && leaf_e0[L] < B.r1; L++)
                 per_leaf[L].push_back({d.A + 3L * (leaf_e0[L] - B.r0), m, d.rank, 1, zoff});
             zoff += d.rank;
@@ -987,31 +1035,41 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     std::vector<HLeafTerm> terms;
     std::vector<HChunk> chunks;
     std::vector<int> leaf_chunk(1, 0);
+    std::vector<HChunk> by_kind[2];   // chunks of dense and of low-rank pieces
     std::vector<PackJob> pk;
     long poff = 0;
     for (int L = 0; L < h->n_leaves; L++) {
         const int rows = 3 * (leaf_e0[L + 1] - leaf_e0[L]);
         const int maxc = (int)std::max<long>(1, HM_CHUNK_BYTES / (8L * rows + 16));
-        HChunk ch{L, (int)terms.size(), (int)terms.size(), 0, poff};
-        for (const HLeafTerm &T : per_leaf[L]) {
-            for (int c0 = 0; c0 < T.cols; c0 += maxc) {
-                const int nc = std::min(maxc, T.cols - c0);
-                const long sz = ((long)rows * nc + 7) & ~7L;   // padded to 8 elements (64 / 16 bytes)
-                if (ch.bytes + 8L * sz > HM_CHUNK_BYTES) {
-                    chunks.push_back(ch);
-                    ch = HChunk{L, (int)terms.size(), (int)terms.size(), 0, poff};
+        // dense pieces first: a chunk is of one kind
+        for (int kind = 0; kind < 2; kind++) {
+            HChunk ch{rows, 0, (int)terms.size(), (int)terms.size(), 0, 0, poff};
+            auto close = [&]() {
+                ch.id = (int)chunks.size();
+                chunks.push_back(ch);
+                by_kind[kind].push_back(ch);
+                ch = HChunk{rows, 0, (int)terms.size(), (int)terms.size(), 0, 0, poff};
+            };
+            for (const HLeafTerm &T : per_leaf[L]) {
+                if (T.xsel != kind) continue;
+                for (int c0 = 0; c0 < T.cols; c0 += maxc) {
+                    const int nc = std::min(maxc, T.cols - c0);
+                    const long sz = ((long)rows * nc + 7) & ~7L;   // padded to 8 elements (64 / 16 bytes)
+                    if (ch.bytes + 8L * sz > HM_CHUNK_BYTES) close();
+                    HLeafTerm P = T;
+                    P.cols = nc;
+                    P.xoff = T.xoff + c0;
+                    pk.push_back({T.A + (long)c0 * T.lda, T.lda, rows, nc, poff});
+                    terms.push_back(P);
+                    poff += sz;
+                    ch.q1 = (int)terms.size();
+                    ch.bytes += (int)(8L * sz);
+                    ch.cols += nc;
+                    h->max_cols = std::max(h->max_cols, ch.cols);
                 }
-                HLeafTerm P = T;
-                P.cols = nc;
-                P.xoff = T.xoff + c0;
-                pk.push_back({T.A + (long)c0 * T.lda, T.lda, rows, nc, poff});
-                terms.push_back(P);
-                poff += sz;
-                ch.q1 = (int)terms.size();
-                ch.bytes += (int)(8L * sz);
             }
+            if (ch.bytes || kind == 0) close();   // possibly empty: the leaf's dense rows are then zero
         }
-        chunks.push_back(ch);   // possibly empty: the leaf's rows are then zero
         leaf_chunk.push_back((int)chunks.size());
     }
     h->n_chunks = (int)chunks.size();
@@ -1029,7 +1087,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         if (!pk.empty()) {
             PackJob *pk_d = nullptr;
             UCG_CUDA(cudaMalloc(&pk_d, sizeof(PackJob) * pk.size()));
-            UCG_CUDA(cudaMemcpy(pk_d, pk.data(), sizeof(PackJob) * pk.size(), cudaMemcpyHostToDevice));
+            UCG_CUDA(cudaMemcpyAsync(pk_d, pk.data(), sizeof(PackJob) * pk.size(), cudaMemcpyHostToDevice, c->stream));
             k_pack<<<(int)pk.size(), 256, 0, c->stream>>>(pk_d, panel);
             c->launches.count++;
             UCG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1040,7 +1098,10 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         for (HLeafTerm &T : terms) T.A = nullptr;
         h->terms_h = terms;
     }
+    // the longest blocks' warps first
+    std::stable_sort(items.begin(), items.end(), [&](const int2 &x, const int2 &y) { return lr[x.x].n > lr[y.x].n; });
     h->n_items = (long)items.size();
+    h->n_dense_chunks = (int)by_kind[0].size();
     h->nz = std::max<long>(zoff, 1);
     UCG_CUDA(cudaMalloc(&h->lr_d, sizeof(HLowRank) * std::max<size_t>(lr.size(), 1)));
     UCG_CUDA(cudaMalloc(&h->items_d, sizeof(int2) * std::max<size_t>(items.size(), 1)));
@@ -1051,7 +1112,6 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     UCG_CUDA(cudaMalloc(&h->z_d, sizeof(double) * h->nz));
     UCG_CUDA(cudaMalloc(&h->t_d, sizeof(double) * (3L * np + 2)));
     UCG_CUDA(cudaMalloc(&h->xp_d, sizeof(double) * (2L * np + 2)));
-    UCG_CUDA(cudaFuncSetAttribute(k_hm_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HM_CHUNK_BYTES));
     UCG_CUDA(cudaMalloc(&h->status_d, sizeof(int)));
     UCG_CUDA(cudaMemset(h->status_d, 0, sizeof(int)));
     UCG_CUDA(cudaMalloc(&h->part_d, sizeof(double) * (size_t)h->n_chunks * 3 * h->max_leaf));
@@ -1063,14 +1123,16 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         }
     }
     h->lr_h = lr;
-    if (!lr.empty()) UCG_CUDA(cudaMemcpy(h->lr_d, lr.data(), sizeof(HLowRank) * lr.size(), cudaMemcpyHostToDevice));
+    if (!lr.empty()) UCG_CUDA(cudaMemcpyAsync(h->lr_d, lr.data(), sizeof(HLowRank) * lr.size(), cudaMemcpyHostToDevice, c->stream));
     if (!items.empty())
-        UCG_CUDA(cudaMemcpy(h->items_d, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice));
+        UCG_CUDA(cudaMemcpyAsync(h->items_d, items.data(), sizeof(int2) * items.size(), cudaMemcpyHostToDevice, c->stream));
     if (!terms.empty())
-        UCG_CUDA(cudaMemcpy(h->terms_d, terms.data(), sizeof(HLeafTerm) * terms.size(), cudaMemcpyHostToDevice));
-    UCG_CUDA(cudaMemcpy(h->chunks_d, chunks.data(), sizeof(HChunk) * chunks.size(), cudaMemcpyHostToDevice));
-    UCG_CUDA(cudaMemcpy(h->leaf_chunk_d, leaf_chunk.data(), sizeof(int) * leaf_chunk.size(), cudaMemcpyHostToDevice));
-    UCG_CUDA(cudaMemcpy(h->leaf_e0_d, leaf_e0.data(), sizeof(int) * leaf_e0.size(), cudaMemcpyHostToDevice));
+        UCG_CUDA(cudaMemcpyAsync(h->terms_d, terms.data(), sizeof(HLeafTerm) * terms.size(), cudaMemcpyHostToDevice, c->stream));
+    // on the device the dense chunks come first: the two product kernels take one kind each
+    by_kind[0].insert(by_kind[0].end(), by_kind[1].begin(), by_kind[1].end());
+    UCG_CUDA(cudaMemcpyAsync(h->chunks_d, by_kind[0].data(), sizeof(HChunk) * chunks.size(), cudaMemcpyHostToDevice, c->stream));
+    UCG_CUDA(cudaMemcpyAsync(h->leaf_chunk_d, leaf_chunk.data(), sizeof(int) * leaf_chunk.size(), cudaMemcpyHostToDevice, c->stream));
+    UCG_CUDA(cudaMemcpyAsync(h->leaf_e0_d, leaf_e0.data(), sizeof(int) * leaf_e0.size(), cudaMemcpyHostToDevice, c->stream));
     UCG_CUDA(cudaEventRecord(ev1, c->stream));
     UCG_CUDA(cudaEventSynchronize(ev1));
     float ms = 0.0f;
@@ -1081,24 +1143,47 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     return UCG_OK;
 }
 
+// the chunks' partial row sums of H xp (split: of its FP32 planes), enqueued on
+// the context stream
+template <bool SPLIT>
+static void launch_products(ucg_ctx *c)
+{
+    HMat *h = c->hm;
+    const HmProduct P{h->lr_d, h->items_d, h->n_items, h->terms_d, h->chunks_d, h->n_dense_chunks, h->panel,
+                      h->ph, h->pl, h->vh, h->vl, h->xp_d, h->z_d, h->part_d, 3 * h->max_leaf, h->status_d};
+    const size_t smem = (SPLIT ? HM_CHUNK_BYTES / 2 : HM_CHUNK_BYTES) + sizeof(double) * h->max_cols;
+    const int thr = (3 * h->max_leaf + 31) & ~31;
+    const int zb = (int)((h->n_items * 32 + thr - 1) / thr), lowrank = h->n_chunks - h->n_dense_chunks;
+    hm_launch(k_hm_rows<SPLIT, true>, dim3(zb + h->n_dense_chunks), dim3(thr), smem, c->stream, P, zb);
+    c->launches.count++;
+    if (lowrank > 0) {
+        hm_launch(k_hm_rows<SPLIT, false>, dim3(lowrank), dim3(thr), smem, c->stream, P, 0);
+        c->launches.count++;
+    }
+}
+
+void hmatrix_products(ucg_ctx *c, bool split)
+{
+    if (split) launch_products<true>(c);
+    else launch_products<false>(c);
+}
+
+HmParts hmatrix_parts(const ucg_ctx *c)
+{
+    const HMat *h = c->hm;
+    return HmParts{h->leaf_e0_d, h->leaf_chunk_d, h->perm_d, h->part_d, h->xp_d, 3 * h->max_leaf, h->n_leaves};
+}
+
 // t = H v (K's row order), enqueued on the context stream
 void hmatrix_apply(ucg_ctx *c, const double *v, double *t)
 {
     HMat *h = c->hm;
     k_hm_gather<<<(h->np + 255) / 256, 256, 0, c->stream>>>(h->perm_d, h->np, v, h->xp_d);
-    if (h->n_items > 0) {
-        const long threads = h->n_items * 32;
-        k_hm_z<<<(int)((threads + 255) / 256), 256, 0, c->stream>>>(h->lr_d, h->items_d, h->n_items, h->xp_d,
-                                                                    h->z_d);
-        c->launches.count++;
-    }
-    const int rows = 3 * h->max_leaf;
-    k_hm_rows<<<h->n_chunks, ((rows + 31) / 32) * 32, HM_CHUNK_BYTES, c->stream>>>(
-        h->terms_d, h->chunks_d, h->leaf_e0_d, h->panel, h->xp_d, h->z_d, h->part_d, rows, h->status_d);
-    const int gs = ((rows + 31) / 32) * 32, nthr = std::max(gs, (1024 / gs) * gs);
+    hmatrix_products(c, false);
+    const int rows = 3 * h->max_leaf, gs = ((rows + 31) / 32) * 32, nthr = std::max(gs, (1024 / gs) * gs);
     k_hm_reduce<<<h->n_leaves, nthr, sizeof(double) * nthr, c->stream>>>(h->leaf_e0_d, h->leaf_chunk_d, h->perm_d,
                                                                          h->part_d, rows, t, gs);
-    c->launches.count += 3;
+    c->launches.count += 2;
 }
 
 // hi / lo planes of the FP32 copies of the panels and of V (once; kept with the matrix)
@@ -1124,7 +1209,7 @@ int hmatrix_split_build(ucg_ctx *c)
     if (!jobs.empty()) {
         SplitJob *jd = nullptr;
         UCG_CUDA(cudaMalloc(&jd, sizeof(SplitJob) * jobs.size()));
-        UCG_CUDA(cudaMemcpy(jd, jobs.data(), sizeof(SplitJob) * jobs.size(), cudaMemcpyHostToDevice));
+        UCG_CUDA(cudaMemcpyAsync(jd, jobs.data(), sizeof(SplitJob) * jobs.size(), cudaMemcpyHostToDevice, c->stream));
         k_split_jobs<<<(int)jobs.size(), 256, 0, c->stream>>>(jd, h->vh, h->vl);
         c->launches.count++;
         UCG_CUDA(cudaStreamSynchronize(c->stream));
@@ -1132,38 +1217,6 @@ int hmatrix_split_build(ucg_ctx *c)
     }
     UCG_CUDA(cudaStreamSynchronize(c->stream));
     return UCG_OK;
-}
-
-// t = H v on the split copies: hi + lo (lo = true) or hi alone
-void hmatrix_apply_split(ucg_ctx *c, const double *v, double *t, bool lo)
-{
-    HMat *h = c->hm;
-    k_hm_gather<<<(h->np + 255) / 256, 256, 0, c->stream>>>(h->perm_d, h->np, v, h->xp_d);
-    if (h->n_items > 0) {
-        const long threads = h->n_items * 32;
-        if (lo)
-            k_hm_z_split<true><<<(int)((threads + 255) / 256), 256, 0, c->stream>>>(h->lr_d, h->items_d, h->n_items,
-                                                                                 h->xp_d, h->vh, h->vl, h->z_d);
-        else
-            k_hm_z_split<false><<<(int)((threads + 255) / 256), 256, 0, c->stream>>>(h->lr_d, h->items_d, h->n_items,
-                                                                                  h->xp_d, h->vh, h->vl, h->z_d);
-        c->launches.count++;
-    }
-    const int rows = 3 * h->max_leaf;
-    const int thr = ((rows + 31) / 32) * 32;
-    const size_t smem = (size_t)(lo ? 2 : 1) * 2 * (HM_CHUNK_BYTES / 8);
-    if (lo)
-        k_hm_rows_split<true><<<h->n_chunks, thr, smem, c->stream>>>(h->terms_d, h->chunks_d, h->leaf_e0_d, h->ph,
-                                                                     h->pl, h->xp_d, h->z_d, h->part_d, rows,
-                                                                     h->status_d);
-    else
-        k_hm_rows_split<false><<<h->n_chunks, thr, smem, c->stream>>>(h->terms_d, h->chunks_d, h->leaf_e0_d, h->ph,
-                                                                      h->pl, h->xp_d, h->z_d, h->part_d, rows,
-                                                                      h->status_d);
-    const int gs = thr, nthr = std::max(gs, (1024 / gs) * gs);
-    k_hm_reduce<<<h->n_leaves, nthr, sizeof(double) * nthr, c->stream>>>(h->leaf_e0_d, h->leaf_chunk_d, h->perm_d,
-                                                                         h->part_d, rows, t, gs);
-    c->launches.count += 3;
 }
 
 double *hmatrix_t(ucg_ctx *c) { return c->hm ? c->hm->t_d : nullptr; }

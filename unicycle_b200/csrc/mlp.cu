@@ -275,11 +275,11 @@ int ucg_mlp_create(ucg_mlp **out, int device, unsigned long long seed)
     }
     m->hnorm.ym = 0.0f;
     m->hnorm.ys = 1.0f;
-    cudaMemcpy(m->W, w.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice);
+    ucg::copy_in(m->W, w.data(), sizeof(float) * NPARAM);
     cudaMemset(m->M, 0, sizeof(float) * NPARAM);
     cudaMemset(m->V, 0, sizeof(float) * NPARAM);
     cudaMemset(m->G, 0, sizeof(float) * NPARAM);
-    cudaMemcpy(m->norm, &m->hnorm, sizeof(Norm), cudaMemcpyHostToDevice);
+    ucg::copy_in(m->norm, &m->hnorm, sizeof(Norm));
     k_mlp_to_half<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->W, m->P);
     k_mlp_inference_copy<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->P, m->T);
     cudaStreamSynchronize(m->stream);
@@ -307,7 +307,7 @@ int ucg_mlp_set_params(ucg_mlp *m, const float *params, const float *norm)
     MCUDA(cudaSetDevice(m->device));
     MCUDA(cudaStreamSynchronize(m->stream));
     if (params) {
-        MCUDA(cudaMemcpy(m->W, params, sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
+        MCUDA(ucg::copy_in(m->W, params, sizeof(float) * NPARAM));
         k_mlp_to_half<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->W, m->P);
         k_mlp_inference_copy<<<(NPARAM + 255) / 256, 256, 0, m->stream>>>(m->P, m->T);
         MCUDA(cudaGetLastError());
@@ -330,7 +330,7 @@ int ucg_mlp_set_params(ucg_mlp *m, const float *params, const float *norm)
         memcpy(m->hnorm.xs, norm + NIN, sizeof(float) * NIN);
         m->hnorm.ym = norm[2 * NIN];
         m->hnorm.ys = norm[2 * NIN + 1];
-        MCUDA(cudaMemcpy(m->norm, &m->hnorm, sizeof(Norm), cudaMemcpyHostToDevice));
+        MCUDA(ucg::copy_in(m->norm, &m->hnorm, sizeof(Norm)));
     }
     MCUDA(cudaStreamSynchronize(m->stream));
     return UCG_OK;
@@ -365,8 +365,8 @@ int ucg_mlp_set_data(ucg_mlp *m, const float *x, const float *y, long n, int sta
     MCUDA(cudaMalloc(&m->X, sizeof(float) * NIN * n));
     MCUDA(cudaMalloc(&m->Y, sizeof(float) * n));
     MCUDA(cudaMalloc(&m->idx, sizeof(int) * n));
-    MCUDA(cudaMemcpy(m->X, x, sizeof(float) * NIN * n, cudaMemcpyHostToDevice));
-    MCUDA(cudaMemcpy(m->Y, y, sizeof(float) * n, cudaMemcpyHostToDevice));
+    MCUDA(ucg::copy_in(m->X, x, sizeof(float) * NIN * n));
+    MCUDA(ucg::copy_in(m->Y, y, sizeof(float) * n));
     m->n = n;
     if (standardise) {
         // means and deviations of the training set (FP64 sums)
@@ -387,7 +387,7 @@ int ucg_mlp_set_data(ucg_mlp *m, const float *x, const float *y, long n, int sta
                 m->hnorm.ys = sd;
             }
         }
-        MCUDA(cudaMemcpy(m->norm, &m->hnorm, sizeof(Norm), cudaMemcpyHostToDevice));
+        MCUDA(ucg::copy_in(m->norm, &m->hnorm, sizeof(Norm)));
     }
     return UCG_OK;
 }

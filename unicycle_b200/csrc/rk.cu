@@ -70,6 +70,7 @@ struct StageArgs {
     double *ks;            // k of this stage
     const double *v;       // source rates of this stage
     double *vn;            // source rates of the next one
+    const int *perm;       // hierarchical K: vn is in the order perm (position -> element)
     int next;              // form the next stage's state (0: only k_s)
     double *ycand, *yerr, *yscal;
     double *v1, *t1;       // stage-1 anchor (split-BF16 matrix only)
@@ -252,15 +253,15 @@ __device__ __forceinline__ double lane_advance(int S, const StageArgs &a, long i
     return yc;
 }
 
-// source rate of column j of the next stage.  Anchored forms multiply increments
+// source rate of column j (at jn of the buffer) of the next stage.  Anchored forms multiply increments
 // over stage 1 in the stages 2-6; vs: this stage's own rate (stage 1: the anchor)
-__device__ __forceinline__ void store_rate(int S, const StageArgs &a, long j, double vnext, double vs)
+__device__ __forceinline__ void store_rate(int S, const StageArgs &a, long j, long jn, double vnext, double vs)
 {
     if (a.anchored) {
         if (S == 1) a.v1[j] = vs;
         if (S < 6) vnext -= S == 1 ? vs : a.v1[j];
     }
-    if (a.next) a.vn[j] = vnext;
+    if (a.next) a.vn[jn] = vnext;
 }
 
 // friction of a patch, and of its terms in f what the state gives
@@ -300,7 +301,7 @@ __device__ __forceinline__ PatchTerms patch_terms(int S, Ctl *ctl, const PatchFr
 }
 
 // patch e: rates from its tractions t, then the next stage
-__device__ __forceinline__ void patch_finish(int S, const StageArgs &a, Ctl *ctl, int e, int c, double h,
+__device__ __forceinline__ void patch_finish(int S, const StageArgs &a, Ctl *ctl, int e, int pos, int c, double h,
                                              const LaneState &st, const PatchTerms &p, double t0, double t1,
                                              double t2, double &mx, bool &bad)
 {
@@ -318,7 +319,7 @@ __device__ __forceinline__ void patch_finish(int S, const StageArgs &a, Ctl *ctl
         // (of a candidate only once it is accepted, at the next stage 1)
         if (S < 6 && (!isfinite(vel) || !isfinite(cr) || !isfinite(sr))) ctl->nonfinite = 1;
     }
-    store_rate(S, a, 2L * e + c, vel * (c == 0 ? cr : sr) - p.vpl, vs - p.vpl);
+    store_rate(S, a, 2L * e + c, 2L * pos + c, vel * (c == 0 ? cr : sr) - p.vpl, vs - p.vpl);
 }
 
 // volume iv: rates from its stress rate t (its own row for the lanes 6..11;
@@ -334,7 +335,8 @@ __device__ __forceinline__ void volume_finish(int S, const StageArgs &a, int iv,
     if (!st.on || c > 5) return;
     const double ebg = a.rh.ebg[6L * iv + c];
     const double en = a.next ? volume_rate(a.rh, iv, c, s[0], s[1], s[2], s[3], s[4], s[5]) : 0.0;
-    store_rate(S, a, 2L * a.np + 6L * iv + c, en - ebg, ev - ebg);
+    const long j = 2L * a.np + 6L * iv + c;
+    store_rate(S, a, j, j, en - ebg, ev - ebg);
 }
 
 // source rates of the state y (before the first stage of a run; the attempts form
@@ -343,16 +345,17 @@ __global__ void k_begin(StageArgs a, const Ctl *ctl, double *__restrict__ v)
 {
     pdl_enter();
     if (!ctl_live(ctl) || !ctl->need_stage1) return;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= a.np + a.nvol) return;
-    if (e < a.np) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.np + a.nvol) return;
+    if (p < a.np) {
+        const int e = a.perm ? a.perm[p] : p;
         const double *y = a.y + 7L * e;
         double vel, cr, sr;
         patch_slip(y[2], y[3], y[6], vel, cr, sr);
-        v[2L * e] = vel * cr - a.fr.vpl_c[e];
-        v[2L * e + 1] = vel * sr - a.fr.vpl_s[e];
+        v[2L * p] = vel * cr - a.fr.vpl_c[e];
+        v[2L * p + 1] = vel * sr - a.fr.vpl_s[e];
     } else {
-        const int iv = e - a.np;
+        const int iv = p - a.np;
         const double *s = a.y + 7L * a.np + 12L * iv + 6;
         for (int q = 0; q < 6; q++)
             v[2L * a.np + 6L * iv + q] = volume_rate(a.rh, iv, q, s[0], s[1], s[2], s[3], s[4], s[5]) -
@@ -421,7 +424,7 @@ __device__ __forceinline__ void attempt_end(Ctl *ctl, double mx, bool bad)
         if (mx > 0.0) atomic_max_pos(&ctl->errbits, mx);
         if (bad) ctl->nonfinite = 1;
         __threadfence();
-        if (atomicAdd(&ctl->ticket, 1) == (int)gridDim.x - 1) {
+        if (atomicAdd(&ctl->ticket, 1) == (int)(gridDim.x * gridDim.y) - 1) {
             __threadfence();
             ctl->ticket = 0;
             decide(ctl);
@@ -431,7 +434,7 @@ __device__ __forceinline__ void attempt_end(Ctl *ctl, double mx, bool bad)
 
 // a rejected attempt repeats with a smaller step from the same k_1: stage 2 of a
 // patch for the new h
-__device__ __forceinline__ void retry_stage2(const StageArgs &a, Ctl *ctl, int e, int c, bool on, double h)
+__device__ __forceinline__ void retry_stage2(const StageArgs &a, Ctl *ctl, int e, int pos, int c, bool on, double h)
 {
     const long i = 7L * e + c;
     double yn = 0.0;
@@ -446,7 +449,7 @@ __device__ __forceinline__ void retry_stage2(const StageArgs &a, Ctl *ctl, int e
     if (!isfinite(vel) || !isfinite(cr) || !isfinite(sr)) ctl->nonfinite = 1;
     double v = vel * (c == 0 ? cr : sr) - (c == 0 ? a.fr.vpl_c[e] : a.fr.vpl_s[e]);
     if (a.anchored) v -= a.v1[2L * e + c];
-    a.vn[2L * e + c] = v;
+    a.vn[2L * pos + c] = v;
 }
 
 // and of a volume
@@ -480,54 +483,87 @@ __device__ __forceinline__ void retry_stage2_volume(const StageArgs &a, int iv, 
 
 constexpr int MV_WARPS = 8;
 
-// Stage S of every patch from a traction vector already formed (the hierarchical
-// product): the epilogue of k_traction without the matvec, 32 patches a CTA.
-__global__ void __launch_bounds__(256) k_rhs_t(int S, StageArgs a, Ctl *ctl, const double *__restrict__ t)
+// Stage S on the hierarchical K: a CTA takes HS_P patches of a row leaf, adds up
+// their rows over the leaf's chunks (HS_G groups of threads each every HS_G-th
+// chunk, then the groups in order) and runs them through the stage, their source
+// rates straight into the product's permuted input.  As separate kernels (gather,
+// reduction, right-hand side, stage state) these took 24 more launches an attempt.
+// One CTA for a whole leaf (225 of 1,024 threads at N = 7,200) left two uneven
+// waves: 32 us against 16 with eight patches a CTA (both cold).
+constexpr int HS_P = 8, HS_ROWS = 3 * HS_P, HS_G = 8, HS_EL = 8 * HS_P, HS_THREADS = HS_EL + HS_ROWS * HS_G;
+
+__global__ void __launch_bounds__(HS_THREADS, 4) k_hm_stage(int S, StageArgs a, Ctl *ctl, HmParts hp)
 {
+    __shared__ double sh[HS_G][HS_ROWS];
+    __shared__ double tt[HS_ROWS];
     pdl_enter();
     if (!ctl_live(ctl)) return;
     const double h = ctl->h;
-    const int c = threadIdx.x & 7, e = blockIdx.x * 32 + (threadIdx.x >> 3);
-    const bool on = e < a.np && c < 7;
+    const int L = blockIdx.x, p0 = blockIdx.y * HS_P, e0 = hp.leaf_e0[L] + p0;
+    const int nel = min(HS_P, hp.leaf_e0[L + 1] - e0), rows = 3 * nel;   // nel <= 0: a short leaf
+    // the first two warps take the patches, the others the sums
+    const int c = threadIdx.x & 7, q = threadIdx.x >> 3, pos = e0 + q;
+    const bool elem = threadIdx.x < HS_EL, on = elem && q < nel && c < 7;
+    const int e = on ? hp.perm[pos] : 0;
     double mx = 0.0;
     bool bad = false;
     if (S == 1 && !ctl->need_stage1) {
-        retry_stage2(a, ctl, e, c, on, h);
+        if (elem) retry_stage2(a, ctl, e, pos, c, on, h);
         return;
     }
     LaneState st;
-    const double ys = lane_load(S, a, ctl, 7L * e + c, on, st);
-    const PatchTerms p = patch_terms(S, ctl, patch_friction(a, e, c, on), c, on, ys);
-    double tr[3] = {0.0, 0.0, 0.0};
-    if (on) {
-#pragma unroll
-        for (int q = 0; q < 3; q++) tr[q] = t[3L * e + q];
-        if (a.anchored) {
-            // anchored stages: stage 1 keeps t1 = K v1, the others add K (v - v1) to it
-#pragma unroll
-            for (int q = 0; q < 3; q++) {
-                if (S > 1) tr[q] += a.t1[3L * e + q];
-                else if (c == q) a.t1[3L * e + q] = tr[q];
-            }
-        }
+    PatchTerms p;
+    if (elem) {
+        const double ys = lane_load(S, a, ctl, 7L * e + c, on, st);
+        p = patch_terms(S, ctl, patch_friction(a, e, c, on), c, on, ys);
     }
-    patch_finish(S, a, ctl, e, c, h, st, p, tr[0], tr[1], tr[2], mx, bad);
-    if (S == 6) {
-        __shared__ double smx[8];
-        __shared__ int sbad[8];
+    const int c0 = hp.leaf_chunk[L], c1 = hp.leaf_chunk[L + 1];
+    if (!elem) {
+        const int g = (threadIdx.x - HS_EL) / HS_ROWS, i = (threadIdx.x - HS_EL) % HS_ROWS;
+        double s[8] = {};
+        if (i < rows) {
+            const double *part = hp.part + 3 * p0 + i;
+            int k = c0 + g;
+            for (; k + 7 * HS_G < c1; k += 8 * HS_G) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = part[(long)(k + u * HS_G) * hp.rows_max];
+#pragma unroll
+                for (int u = 0; u < 8; u++) s[u] += v[u];
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (k + u * HS_G < c1) s[u] += part[(long)(k + u * HS_G) * hp.rows_max];
+        }
+        sh[g][i] = ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7]));
+    }
+    __syncthreads();
+    if (threadIdx.x < HS_ROWS) {
+        const int i = threadIdx.x;
+        double t = 0.0;
+        for (int k = 0; k < HS_G; k++) t += sh[k][i];
+        if (a.anchored && i < rows) {
+            // anchored stages: stage 1 keeps t1 = K v1, the others add K (v - v1) to it
+            double *t1 = a.t1 + 3L * hp.perm[e0 + i / 3] + i % 3;
+            if (S == 1) *t1 = t;
+            else t += *t1;
+        }
+        tt[i] = t;
+    }
+    __syncthreads();
+    if (!elem) return;
+    patch_finish(S, a, ctl, e, pos, c, h, st, p, tt[3 * q], tt[3 * q + 1], tt[3 * q + 2], mx, bad);
+    if (S == 6 && a.next) {
+        __shared__ double smx;
+        __shared__ int sbad;
         for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
         bad = __any_sync(0xffffffffu, bad);
-        if ((threadIdx.x & 31) == 0) {
-            smx[threadIdx.x >> 5] = mx;
-            sbad[threadIdx.x >> 5] = bad;
+        if (threadIdx.x == 32) {
+            smx = mx;
+            sbad = bad;
         }
-        // every thread's candidate and rates are out before the CTA counts itself in
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x < 32) {
-            const int w = threadIdx.x & 7;
-            attempt_end(ctl, smx[w], sbad[w] != 0);
-        }
+        asm volatile("bar.sync 1, 64;" ::: "memory");   // the two warps of the patches
+        if (threadIdx.x < 32) attempt_end(ctl, fmax(mx, smx), bad || sbad);
     }
 }
 
@@ -925,7 +961,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
                 const int q = q0 + sub, e = e0 + q;
                 const bool on = q < nel && c < nc;
                 if (!first) {
-                    if (patch) retry_stage2(a, ctl, e, c, on, h);
+                    if (patch) retry_stage2(a, ctl, e, e, c, on, h);
                     else retry_stage2_volume(a, e, c, on, h);
                     continue;
                 }
@@ -950,7 +986,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
                     }
                     const double t0 = __shfl_sync(~0u, t, 0, 8), t1 = __shfl_sync(~0u, t, 1, 8),
                                  t2 = __shfl_sync(~0u, t, 2, 8);
-                    if (!abort_flag) patch_finish(S, a, ctl, e, c, h, st, p, t0, t1, t2, mx, bad);
+                    if (!abort_flag) patch_finish(S, a, ctl, e, e, c, h, st, p, t0, t1, t2, mx, bad);
                 } else {
                     LaneState st;
                     const double ys = lane_load(S, a, ctl, 7L * a.np + 12L * e + c, on, st);
@@ -1112,8 +1148,13 @@ void rk_drop_graph(ucg_ctx *c)
     c->attempt_graph = nullptr;
 }
 
+static bool rk_hierarchical(const ucg_ctx *c)
+{
+    return c->precision == UCG_PREC_HMATRIX || c->precision == UCG_PREC_HMATRIX_SPLIT;
+}
+
 // stage s reads its source rates from buffer s & 1 and writes the next stage's
-// into the other
+// into the other (hierarchical K: one buffer, the product's permuted input)
 static StageArgs stage_args(ucg_ctx *c, int s, int next)
 {
     StageArgs a;
@@ -1123,6 +1164,12 @@ static StageArgs stage_args(ucg_ctx *c, int s, int next)
     a.ks = c->st.k[s - 1];
     a.v = c->st.v[s & 1];
     a.vn = c->st.v[(s + 1) & 1];
+    a.perm = nullptr;
+    if (rk_hierarchical(c)) {
+        const HmParts hp = hmatrix_parts(c);
+        a.vn = hp.xp;
+        a.perm = hp.perm;
+    }
     a.next = next;
     a.ycand = c->st.ycand;
     a.yerr = c->st.yerr;
@@ -1222,11 +1269,11 @@ static void launch_traction(ucg_ctx *c, int S, const StageArgs &a)
 static void enqueue_stage(ucg_ctx *c, int S, int next)
 {
     const StageArgs a = stage_args(c, S, next);
-    if (c->precision == UCG_PREC_HMATRIX || c->precision == UCG_PREC_HMATRIX_SPLIT) {
-        double *t = hmatrix_t(c);
-        if (c->precision == UCG_PREC_HMATRIX) hmatrix_apply(c, a.v, t);
-        else hmatrix_apply_split(c, a.v, t, true);     // every stage on the FP32 planes (hi + lo)
-        k_rhs_t<<<(a.np + 31) / 32, 256, 0, c->stream>>>(S, a, c->ctl, t);
+    if (rk_hierarchical(c)) {
+        hmatrix_products(c, c->precision == UCG_PREC_HMATRIX_SPLIT);
+        const HmParts hp = hmatrix_parts(c);
+        launch_pdl(k_hm_stage, dim3(hp.n_leaves, (hp.rows_max + HS_ROWS - 1) / HS_ROWS), dim3(HS_THREADS), 0, c->stream,
+                   S, a, c->ctl, hp);
     } else {
         launch_traction(c, S, a);
     }
@@ -1238,7 +1285,8 @@ static void enqueue_begin(ucg_ctx *c)
 {
     const StageArgs a = stage_args(c, 1, 0);
     const int ne = a.np + a.nvol;
-    launch_pdl(k_begin, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl, c->st.v[1]);
+    launch_pdl(k_begin, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl,
+               a.perm ? a.vn : c->st.v[1]);
     c->launches.count += 1;
 }
 

@@ -479,7 +479,7 @@ int ucg_record(ucg_ctx *c, int every, const int *elements, int nelem, long capac
         UCG_CUDA(cudaMalloc(&c->rec_buf, sizeof(double) * (size_t)r.len * (size_t)capacity));
         if (nelem > 0) {
             UCG_CUDA(cudaMalloc(&c->rec_elem, sizeof(int) * nelem));
-            UCG_CUDA(cudaMemcpy(c->rec_elem, elements, sizeof(int) * nelem, cudaMemcpyHostToDevice));
+            UCG_CUDA(ucg::copy_in(c->rec_elem, elements, sizeof(int) * nelem));
         }
         r.buf = c->rec_buf;
         r.cap = capacity;
@@ -534,7 +534,7 @@ static int stop_recording(ucg_ctx *c)
     UCG_CUDA(cudaStreamSynchronize(c->stream));
     rk_drop_graph(c);
     c->rec_host = Rec{};
-    UCG_CUDA(cudaMemcpy(c->rec, &c->rec_host, sizeof(Rec), cudaMemcpyHostToDevice));
+    UCG_CUDA(ucg::copy_in(c->rec, &c->rec_host, sizeof(Rec)));
     if (c->rec_buf) cudaFree(c->rec_buf);
     if (c->rec_elem) cudaFree(c->rec_elem);
     c->rec_buf = nullptr;

@@ -11,6 +11,15 @@
 namespace ucg {
 struct HMat;
 
+// Host memory to the device, complete on return.  cudaMemcpy alone may return while
+// the last staged piece of a pageable source is on its way, and the library's
+// (non-blocking) streams do not wait for the legacy stream that carries it.
+inline cudaError_t copy_in(void *dst, const void *src, size_t bytes)
+{
+    const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(cudaStreamLegacy);
+}
+
 // Device-resident integrator control block (one per context).
 struct Ctl {
     double h;          // step size of the current attempt
@@ -233,7 +242,19 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf);
 void hmatrix_free(ucg_ctx *c);
 void hmatrix_apply(ucg_ctx *c, const double *v, double *t);   // t = H v, K's row order
 int hmatrix_split_build(ucg_ctx *c);                          // bf16 hi / lo copies (UCG_PREC_HMATRIX_SPLIT)
-void hmatrix_apply_split(ucg_ctx *c, const double *v, double *t, bool lo);
+// The product inside an attempt: partial row sums of H xp per chunk of a row leaf
+// (split: on the FP32 planes), added up by the stage kernel (rk.cu), which also
+// writes xp, the source rates in the permuted order.
+struct HmParts {
+    const int *leaf_e0;      // element ranges of the row leaves (permuted)
+    const int *leaf_chunk;   // chunk ranges of the row leaves
+    const int *perm;         // permuted position -> element
+    const double *part;      // rows_max values per chunk
+    double *xp;
+    int rows_max, n_leaves;
+};
+void hmatrix_products(ucg_ctx *c, bool split);
+HmParts hmatrix_parts(const ucg_ctx *c);
 double *hmatrix_t(ucg_ctx *c);                                 // the product's output buffer
 void hmatrix_info(const ucg_ctx *c, long *n_dense, long *n_lowrank, long *n_fallback, size_t *bytes,
                   int *max_rank, double *build_ms);
