@@ -216,11 +216,9 @@ struct AcaJob {
     int m, n, kmax;
     double *U, *V;           // kmax x m, kmax x n
     unsigned char *used;     // m row flags
-    int *rank;               // out: rank, or -1 when the block stays dense
-    double *err;             // out: relative probe error
 };
 
-constexpr int ACA_THREADS = 256;
+constexpr int ACA_THREADS = 512;
 constexpr int ACA_KMAX = 256;
 
 __device__ double aca_probe(long j)
@@ -273,13 +271,53 @@ __device__ void block_argmax(double v, int idx, double *shv, int *shi, double &b
         }
 }
 
-__global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double eps, double check)
+// b[j] - sum_l cs[l] F[l, j] for j < len, handed to put(j, r): a row (or column) of
+// a block less the crosses so far.  Four entries a thread at a time, eight crosses
+// deep: the loads, not the arithmetic, take the time.
+template <class Put>
+__device__ __forceinline__ void aca_residual(const double *b, long stride, const double *F, int len, int k,
+                                             const double *cs, int tid, Put put)
+{
+    for (int j0 = tid; j0 < len; j0 += 4 * ACA_THREADS) {
+        int j[4];
+        double r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            j[q] = min(j0 + q * ACA_THREADS, len - 1);
+            r[q] = b[j[q] * stride];
+        }
+#pragma unroll 8
+        for (int l = 0; l < k; l++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) r[q] -= cs[l] * F[(long)l * len + j[q]];
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            if (j0 + q * ACA_THREADS < len) put(j[q], r[q]);
+    }
+}
+
+// the probe vector, shared by all blocks
+__global__ void k_probe(double *__restrict__ w, int n)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) w[j] = aca_probe(j);
+}
+
+// Adaptive cross approximation with partial pivoting, one CTA per block.  rank and
+// z (ACA_KMAX a block) receive the number of crosses and V^T w.  The largest blocks
+// come first and set the kernel's time, a rank at a time: the products of a new
+// cross with the earlier ones (for the norm) go one warp each, not one after the
+// other through the whole CTA with eight barriers each, and the check against the
+// dense block is a kernel of its own over all SMs (N = 7,200: 25 -> 7.9 ms).
+__global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *__restrict__ jobs, double eps,
+                                                     const double *__restrict__ probe, int *__restrict__ rank,
+                                                     double *__restrict__ z)
 {
     const AcaJob J = jobs[blockIdx.x];
     __shared__ double shv[ACA_THREADS / 32];
     __shared__ int shi[ACA_THREADS / 32];
-    __shared__ double zs[ACA_KMAX];
-    const int m = J.m, n = J.n, tid = threadIdx.x;
+    __shared__ double cs[ACA_KMAX];
+    const int m = J.m, n = J.n, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
     const double *B = J.B;
     for (int i = tid; i < m; i += ACA_THREADS) J.used[i] = 0;
     __syncthreads();
@@ -291,12 +329,12 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double 
         // residual of the row; its largest entry picks the pivot column
         double best = -1.0;
         int bj = -1;
-        for (int j = tid; j < n; j += ACA_THREADS) {
-            double r = B[(long)row * n + j];
-            for (int l = 0; l < k; l++) r -= J.U[(long)l * m + row] * J.V[(long)l * n + j];
+        for (int l = tid; l < k; l += ACA_THREADS) cs[l] = J.U[(long)l * m + row];
+        __syncthreads();
+        aca_residual(B + (long)row * n, 1, J.V, n, k, cs, tid, [&](int j, double r) {
             v[j] = r;
             if (fabs(r) > best) { best = fabs(r); bj = j; }
-        }
+        });
         if (tid == 0) J.used[row] = 1;
         double pv;
         int pj;
@@ -318,11 +356,9 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double 
         __syncthreads();
         for (int j = tid; j < n; j += ACA_THREADS) v[j] = v[j] / p;
         // residual of the pivot column
-        for (int i = tid; i < m; i += ACA_THREADS) {
-            double r = B[(long)i * n + pj];
-            for (int l = 0; l < k; l++) r -= J.V[(long)l * n + pj] * J.U[(long)l * m + i];
-            u[i] = r;
-        }
+        for (int l = tid; l < k; l += ACA_THREADS) cs[l] = J.V[(long)l * n + pj];
+        __syncthreads();
+        aca_residual(B + pj, n, J.U, m, k, cs, tid, [&](int i, double r) { u[i] = r; });
         __syncthreads();
         // ||S_k||_F^2 update: |u|^2 |v|^2 + 2 sum_l (u_l . u)(v_l . v)
         double a = 0.0, b = 0.0;
@@ -330,13 +366,19 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double 
         for (int j = tid; j < n; j += ACA_THREADS) b += v[j] * v[j];
         const double nu2 = block_sum(a, shv), nv2 = block_sum(b, shv);
         double cross = 0.0;
-        for (int l = 0; l < k; l++) {
+        for (int l = w; l < k; l += ACA_THREADS / 32) {
             double cu = 0.0, cv = 0.0;
-            for (int i = tid; i < m; i += ACA_THREADS) cu += J.U[(long)l * m + i] * u[i];
-            for (int j = tid; j < n; j += ACA_THREADS) cv += J.V[(long)l * n + j] * v[j];
-            const double su = block_sum(cu, shv);
-            cross += su * block_sum(cv, shv);
+#pragma unroll 8
+            for (int i = lane; i < m; i += 32) cu += J.U[(long)l * m + i] * u[i];
+#pragma unroll 8
+            for (int j = lane; j < n; j += 32) cv += J.V[(long)l * n + j] * v[j];
+            for (int o = 16; o > 0; o >>= 1) {
+                cu += __shfl_xor_sync(0xffffffffu, cu, o);
+                cv += __shfl_xor_sync(0xffffffffu, cv, o);
+            }
+            if (lane == 0) cross += cu * cv;
         }
+        cross = block_sum(cross, shv);
         frob2 += nu2 * nv2 + 2.0 * cross;
         k++;
         if (sqrt(nu2 * nv2) <= eps * sqrt(fabs(frob2))) break;
@@ -350,36 +392,71 @@ __global__ void __launch_bounds__(ACA_THREADS) k_aca(const AcaJob *jobs, double 
         if (ni < 0) break;
         row = ni;
     }
-    // probe: || B w - U (V^T w) || / || B w || for a pseudo-random w
-    const int kk = k;
-    for (int l = 0; l < kk; l++) {
-        double s = 0.0;
-        for (int j = tid; j < n; j += ACA_THREADS) s += J.V[(long)l * n + j] * aca_probe(j);
-        s = block_sum(s, shv);
-        if (tid == 0) zs[l] = s;
-    }
+    if (tid == 0) rank[blockIdx.x] = k;
     __syncthreads();
-    const int w = tid >> 5, lane = tid & 31;
-    double e2 = 0.0, y2 = 0.0;
-    for (int i = w; i < m; i += ACA_THREADS / 32) {
+    for (int l = w; l < k; l += ACA_THREADS / 32) {
         double s = 0.0;
-        for (int j = lane; j < n; j += 32) s += B[(long)i * n + j] * aca_probe(j);
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) s += J.V[(long)l * n + j] * probe[j];
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        double a = 0.0;
-        for (int l = lane; l < kk; l += 32) a += J.U[(long)l * m + i] * zs[l];
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) z[(long)blockIdx.x * ACA_KMAX + l] = s;
+    }
+}
+
+// The check of every block against its dense form for the probe vector w: sums of
+// |B w - U z|^2 and |B w|^2 over one tile of rows
+constexpr int CHECK_ROWS = 32;
+
+__global__ void __launch_bounds__(256) k_aca_check(const AcaJob *__restrict__ jobs, const int2 *__restrict__ tiles,
+                                                   const double *__restrict__ probe, const int *__restrict__ rank,
+                                                   const double *__restrict__ z, double2 *__restrict__ sums)
+{
+    __shared__ double2 sh[8];
+    const int2 tile = tiles[blockIdx.x];
+    const AcaJob J = jobs[tile.x];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, k = rank[tile.x];
+    const double *zj = z + (long)tile.x * ACA_KMAX;
+    double e2 = 0.0, y2 = 0.0;
+    for (int i = tile.y + w; i < min(J.m, tile.y + CHECK_ROWS); i += 8) {
+        double s = 0.0, a = 0.0;
+#pragma unroll 4
+        for (int j = lane; j < J.n; j += 32) s += J.B[(long)i * J.n + j] * probe[j];
+        for (int l = lane; l < k; l += 32) a += J.U[(long)l * J.m + i] * zj[l];
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+        }
         e2 += (s - a) * (s - a);
         y2 += s * s;
     }
-    // every lane of a warp holds the same sums; count lane 0's
-    const double te = block_sum(lane == 0 ? e2 : 0.0, shv);
-    const double ty = block_sum(lane == 0 ? y2 : 0.0, shv);
-    if (tid == 0) {
-        const double err = ty > 0.0 ? sqrt(te / ty) : (te > 0.0 ? INFINITY : 0.0);
-        *J.err = err;
-        const bool smaller = (double)kk * (m + n) < 0.5 * (double)m * n;
-        *J.rank = (err <= check && smaller) ? kk : -1;
+    if (lane == 0) sh[w] = make_double2(e2, y2);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double2 t = sh[0];
+        for (int i = 1; i < 8; i++) {
+            t.x += sh[i].x;
+            t.y += sh[i].y;
+        }
+        sums[blockIdx.x] = t;
     }
+}
+
+// rank of every block, or -1 where it stays dense: the probe error above `check`,
+// or factors of more than half its size.  first: first tile of every block.
+__global__ void k_aca_accept(const AcaJob *__restrict__ jobs, int n_jobs, const int *__restrict__ first,
+                             const double2 *__restrict__ sums, double check, int *__restrict__ rank)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= n_jobs) return;
+    double e2 = 0.0, y2 = 0.0;
+    for (int t = first[q]; t < first[q + 1]; t++) {
+        e2 += sums[t].x;
+        y2 += sums[t].y;
+    }
+    const double err = y2 > 0.0 ? sqrt(e2 / y2) : (e2 > 0.0 ? INFINITY : 0.0);
+    const int k = rank[q], m = jobs[q].m, n = jobs[q].n;
+    const bool smaller = (double)k * (m + n) < 0.5 * (double)m * n;
+    if (!(err <= check && smaller)) rank[q] = -1;
 }
 
 // What a batch keeps, in one launch: copies of the factors and column-major
@@ -824,9 +901,9 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     tb.build(0, np);
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    const size_t scratch = std::min<size_t>((size_t)8 << 30, free_b / 4);
+    const size_t bound = std::min<size_t>((size_t)8 << 30, free_b / 4);   // of the build scratch
     std::vector<HBlock> blocks;
-    block_tree(tb.nodes, 0, 0, eta, 0.4 * (double)scratch / sizeof(double), blocks);
+    block_tree(tb.nodes, 0, 0, eta, 0.4 * (double)bound / sizeof(double), blocks);
     std::vector<int> leaf_e0;
     for (const Node &nd : tb.nodes)
         if (nd.c[0] < 0) leaf_e0.push_back(nd.e0);
@@ -839,6 +916,21 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
 
     if ((rc = block_sources_build(c, okada_mode, h->perm, &bs))) return rc;
 
+    // scratch of a batch: what all blocks need, within the bound (few large batches:
+    // each waits for its largest block)
+    auto block_need = [&](const HBlock &B) -> size_t {   // doubles
+        const long m = 3L * (B.r1 - B.r0), n = 2L * (B.s1 - B.s0);
+        const long kmax = std::min<long>(ACA_KMAX, std::min(m, n));
+        const size_t need = (size_t)m * n + (B.lowrank ? (size_t)kmax * (m + n) + (m + 7) / 8 + 2 : 0);
+        return (need + 31) & ~(size_t)31;
+    };
+    size_t total_need = 0, largest = 0;
+    for (const HBlock &B : blocks) {
+        total_need += block_need(B);
+        largest = std::max(largest, block_need(B));
+    }
+    const size_t scratch =
+        std::min(bound, std::max(sizeof(double) * largest, sizeof(double) * total_need));
     double *sc = nullptr;
     UCG_CUDA(cudaMalloc(&sc, scratch));
     struct Done {
@@ -873,16 +965,20 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     const int MAXJOBS = 4096;
     AcaJob *jobs_d = nullptr;
     int *ranks_d = nullptr;
-    double *errs_d = nullptr;
+    double *aca_z = nullptr, *probe_d = nullptr;
     UCG_CUDA(cudaMalloc(&jobs_d, sizeof(AcaJob) * MAXJOBS));
     UCG_CUDA(cudaMalloc(&ranks_d, sizeof(int) * MAXJOBS));
-    UCG_CUDA(cudaMalloc(&errs_d, sizeof(double) * MAXJOBS));
+    UCG_CUDA(cudaMalloc(&aca_z, sizeof(double) * (size_t)MAXJOBS * ACA_KMAX));
+    UCG_CUDA(cudaMalloc(&probe_d, sizeof(double) * 2 * np));
+    k_probe<<<(2 * np + 255) / 256, 256, 0, c->stream>>>(probe_d, 2 * np);
+    c->launches.count++;
     auto cleanup = [&]() {
         cudaStreamSynchronize(c->stream);
         cudaFree(sc);
         cudaFree(jobs_d);
         cudaFree(ranks_d);
-        cudaFree(errs_d);
+        cudaFree(aca_z);
+        cudaFree(probe_d);
     };
 
     // the blocks in batches that fit the scratch
@@ -902,8 +998,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
             const HBlock &B = blocks[bi];
             const long m = 3L * (B.r1 - B.r0), n = 2L * (B.s1 - B.s0);
             const int kmax = (int)std::min<long>(ACA_KMAX, std::min(m, n));
-            size_t need = (size_t)m * n + (B.lowrank ? (size_t)kmax * (m + n) + (m + 7) / 8 + 2 : 0);
-            need = (need + 31) & ~(size_t)31;
+            const size_t need = block_need(B);
             if ((off + need) * sizeof(double) > scratch) {
                 if (off == 0) {
                     cleanup();
@@ -923,8 +1018,6 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
                 J.U = Bd + (size_t)m * n;
                 J.V = J.U + (size_t)kmax * m;
                 J.used = (unsigned char *)(J.V + (size_t)kmax * n);
-                J.rank = ranks_d + jobs.size();
-                J.err = errs_d + jobs.size();
                 jobs.push_back(J);
                 job_block.push_back((int)bi);
             } else {
@@ -939,9 +1032,37 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
         }
         std::vector<int> ranks(jobs.size());
         if (!jobs.empty()) {
+            // the largest first
+            std::vector<int> order(jobs.size());
+            std::iota(order.begin(), order.end(), 0);
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
+                return (long)jobs[x].m + jobs[x].n > (long)jobs[y].m + jobs[y].n;
+            });
+            std::vector<AcaJob> sorted;
+            std::vector<int> sorted_block, first(1, 0);
+            std::vector<int2> tiles;
+            for (int q : order) {
+                for (int i = 0; i < jobs[q].m; i += CHECK_ROWS) tiles.push_back(make_int2((int)sorted.size(), i));
+                first.push_back((int)tiles.size());
+                sorted.push_back(jobs[q]);
+                sorted_block.push_back(job_block[q]);
+            }
+            jobs.swap(sorted);
+            job_block.swap(sorted_block);
+            int2 *td;
+            int *fd;
+            double2 *sums;
+            if ((rc = workspace_upload(c, WS_TILES, tiles, &td)) || (rc = workspace_upload(c, WS_JOBS, first, &fd)) ||
+                (rc = workspace(c, WS_SCRATCH, sizeof(double2) * tiles.size(), &sums))) {
+                cleanup();
+                return rc;
+            }
+            const int nj = (int)jobs.size();
             cudaMemcpyAsync(jobs_d, jobs.data(), sizeof(AcaJob) * jobs.size(), cudaMemcpyHostToDevice, c->stream);
-            k_aca<<<(int)jobs.size(), ACA_THREADS, 0, c->stream>>>(jobs_d, eps, 10.0 * eps);
-            c->launches.count++;
+            k_aca<<<nj, ACA_THREADS, 0, c->stream>>>(jobs_d, eps, probe_d, ranks_d, aca_z);
+            k_aca_check<<<(int)tiles.size(), 256, 0, c->stream>>>(jobs_d, td, probe_d, ranks_d, aca_z, sums);
+            k_aca_accept<<<(nj + 127) / 128, 128, 0, c->stream>>>(jobs_d, nj, fd, sums, 10.0 * eps, ranks_d);
+            c->launches.count += 3;
             cudaMemcpyAsync(ranks.data(), ranks_d, sizeof(int) * jobs.size(), cudaMemcpyDeviceToHost, c->stream);
         }
         cudaError_t e = cudaStreamSynchronize(c->stream);
