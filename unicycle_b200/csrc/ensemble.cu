@@ -92,9 +92,13 @@ constexpr int A_IMG = 2 * A_HALF;       // hi + lo
 constexpr float LO_SCALE = 2048.0f, LO_UNSCALE = 1.0f / 2048.0f;   // dense images: lo = 2^11 residual
 constexpr int MAX_GEOM = 16;
 constexpr int EW_THREADS = 128;         // element-wise kernels: elements per block
-constexpr int ST_THREADS = 256;         // finish / commit kernels: threads per block
+constexpr int EW_BLOCKS = 8;            // and resident blocks per SM
+constexpr int ST_THREADS = 256;         // commit kernel: threads per block
 constexpr int ST_PER = 4;               // state entries per thread (independent loads in flight)
 constexpr int ST_SPAN = ST_THREADS * ST_PER;
+// an instance's state vectors: y, k1..k5, the candidate, yscal, and the four
+// entries an element that a stage's rate reads of its state
+constexpr int STATE_CAND = 6, STATE_VECS = 9;
 constexpr unsigned long long TIMEOUT_NS = 4000000000ull;
 
 // KLO: the stage also reads the K lo image (three MMAs per k-step); without it
@@ -202,7 +206,8 @@ struct GeomDev {
     uint8_t *B;                 // V images [ntile][kblock][hi | lo]
     float *vscale;              // dense: V image scale per [ntile][kblock][instance of the tile]
     const float *rscale;        // per K row (mtiles * 128)
-    double *y, *ys, *k[6], *ycand, *yerr, *yscal;           // [ninst][7 np]
+    double *y, *k[5], *ycand, *yscal;                       // [ninst][7 np]
+    double *vel, *cr, *sr, *eth;                            // [ninst][np]: of the stage state, for its rate
     double *v1, *t1;            // stage-1 anchor: [ninst][2 np] velocities, [ninst][3 np] tractions
     const double *vpl_c, *vpl_s, *a, *b, *sig, *L, *damping; // [ninst][np]
     InstCtl *ctl;               // [ninst]
@@ -1526,59 +1531,46 @@ __device__ __forceinline__ int geom_of(const EnsArgs *A, int blk, bool state_gri
     return gi;
 }
 
-template <int S>
-__device__ __forceinline__ double ens_comb(const GeomDev &G, long i, double h)
+#define E_C1 (37.0 / 378.0)
+#define E_C3 (250.0 / 621.0)
+#define E_C4 (125.0 / 594.0)
+#define E_C6 (512.0 / 1771.0)
+#define E_DC1 (E_C1 - 2825.0 / 27648.0)
+#define E_DC3 (E_C3 - 18575.0 / 48384.0)
+#define E_DC4 (E_C4 - 13525.0 / 55296.0)
+#define E_DC5 (-277.0 / 14336.0)
+#define E_DC6 (E_C6 - 0.25)
+
+// The element-wise kernels: a block holds EW_THREADS consecutive elements of
+// one instance, whose 7-double state tuples are one contiguous range.  Sums over
+// stages run over that range flat (coalesced), per-element work reads and
+// writes the element's tuple in shared memory.
+struct EwBlock {
+    int i, e0, ne;      // instance, first element, elements
+    long base;          // first state entry
+};
+
+__device__ __forceinline__ bool ew_block(const GeomDev &G, EwBlock &b)
 {
-    const double y = G.y[i];
-    if (S == 1) return y;
-    if (S == 2) return __dadd_rn(y, __dmul_rn(__dmul_rn(h, e_B[1][0]), G.k[0][i]));
-    double r = __dmul_rn(e_B[S - 1][0], G.k[0][i]);
-#pragma unroll
-    for (int j = 1; j < S - 1; j++) r = __dadd_rn(r, __dmul_rn(e_B[S - 1][j], G.k[j][i]));
-    return __dadd_rn(y, __dmul_rn(h, r));
+    const int local = blockIdx.x - G.blk_e0;
+    b.i = local / G.epb_e;
+    b.e0 = (local % G.epb_e) * EW_THREADS;
+    b.ne = min(EW_THREADS, G.np - b.e0);
+    b.base = (long)b.i * 7 * G.np + 7L * b.e0;
+    return b.i < G.ninst;
 }
 
-// stage state, velocities and the V images (ratestate.f90:667-707 per instance).
-// A block holds EW_THREADS consecutive elements of one instance, whose 7-double
-// state tuples are one contiguous range: the stage state is formed over that
-// range flat (coalesced), kept in shared memory, and each thread then takes its
-// element's velocity from there.  The velocity components of the stage rate
-// are written by k_ens_rhs with the rest of the tuple.
+// source velocities of stage S (ratestate.f90:667-707) from the stage state sh
+// (7 doubles an element) into the V images, and what the stage's right-hand side
+// needs of the state (the speed, the slip direction, exp(-psi ln 10)): four
+// doubles an element for the state's seven, and the transcendentals once.
+// Stage 1 also keeps the anchor velocities and reduces max V and min log10 theta
 template <int S>
-__global__ void __launch_bounds__(EW_THREADS) k_ens_prologue(const EnsArgs *__restrict__ A)
+__device__ __forceinline__ void ens_sources(const EnsArgs *__restrict__ A, const GeomDev &G, InstCtl *c,
+                                            const EwBlock &b, bool work, const double *sh)
 {
-    __shared__ double sh[7 * EW_THREADS];
-    const int gi = geom_of(A, blockIdx.x, false);
-    const GeomDev &G = A->g[gi];
-    const int local = blockIdx.x - G.blk_e0;
-    const int i = local / G.epb_e;
-    const int e0 = (local % G.epb_e) * EW_THREADS;
-    if (i >= G.ninst) return;                        // uniform over the block
-    const int ne = min(EW_THREADS, G.np - e0);
-    const int e = e0 + threadIdx.x;
-    const bool valid = threadIdx.x < ne;
-    InstCtl *c = G.ctl + i;
-    const bool pend = S == 1 && c->pending;
-    const bool work = inst_live(c, A->glob) && !(S == 1 && !c->need_stage1);
-    const double h = c->h;
-    const long base = (long)i * 7 * G.np + 7L * e0;
-#pragma unroll
-    for (int u = 0; u < 7; u++) {
-        const int f = threadIdx.x + u * EW_THREADS;
-        if (f >= 7 * ne) break;
-        const long x = base + f;
-        double v = 0.0;
-        if (S == 1) {
-            v = pend ? G.ycand[x] : G.y[x];
-            if (pend) G.y[x] = v;
-        } else if (work) {
-            v = ens_comb<S>(G, x, h);
-            G.ys[x] = v;
-            if (S == 2 && c->need_stage1) G.yscal[x] = fabs(G.y[x]) + fabs(h * G.k[0][x]) + 1.0e-30;
-        }
-        sh[f] = v;
-    }
-    __syncthreads();
+    const int i = b.i, e = b.e0 + threadIdx.x;
+    const bool valid = threadIdx.x < b.ne;
     unsigned long long vkey = 0ull, tkey = ~0ull;   // max V and min log10 theta of this element (stage 1)
     double v0 = 0.0, v1 = 0.0;
     if (valid) {
@@ -1586,10 +1578,14 @@ __global__ void __launch_bounds__(EW_THREADS) k_ens_prologue(const EnsArgs *__re
         if (work) {
             const double rake = atan2(yy[3], yy[2]);
             const double vel = exp(yy[6] * E_LG10);
-            const double vs = vel * cos(rake), vd = vel * sin(rake);
+            const double cr = cos(rake), sr = sin(rake);
             const long pe = (long)i * G.np + e;
-            v0 = vs - G.vpl_c[pe];
-            v1 = vd - G.vpl_s[pe];
+            G.vel[pe] = vel;
+            G.cr[pe] = cr;
+            G.sr[pe] = sr;
+            G.eth[pe] = exp(-yy[5] * E_LG10);
+            v0 = vel * cr - G.vpl_c[pe];
+            v1 = vel * sr - G.vpl_s[pe];
             if (!isfinite(vel) || !isfinite(rake)) {
                 c->nonfinite = 1;
                 v0 = v1 = 0.0;
@@ -1611,7 +1607,7 @@ __global__ void __launch_bounds__(EW_THREADS) k_ens_prologue(const EnsArgs *__re
         // a warp holds the 32 elements (64 sources) of one k-block: its scale,
         // then every element's pair of sources
         const float sv = warp_block_scale(v0, v1);
-        const int ew = e0 + (threadIdx.x & ~31);          // the warp's first element
+        const int ew = b.e0 + (threadIdx.x & ~31);        // the warp's first element
         if ((threadIdx.x & 31) == 0 && ew < G.np)
             G.vscale[((size_t)(i / A->ni) * G.kblocks + ew / 32) * A->ni + i % A->ni] = sv;
         if (valid) put_v(G.B, A->ni, G.kblocks, i, 2L * e, v0, v1, sv);
@@ -1630,15 +1626,40 @@ __global__ void __launch_bounds__(EW_THREADS) k_ens_prologue(const EnsArgs *__re
     }
 }
 
-// the stage rate of one element (ratestate.f90:731-776) from its stage state
-// yy (7 doubles) and traction t: all 7 components into k
-__device__ __forceinline__ void ens_rate(const double *yy, const double t[3], double L, double bb, double sg,
-                                         double aa, double eta, double *k)
+// the start of an attempt: the accepted candidate becomes the state, and stage
+// 1's sources.  An instance that does no stage 1 (rejected, or done) gets zero
+// images; a done one keeps them through the attempt
+__global__ void __launch_bounds__(EW_THREADS) k_ens_start(const EnsArgs *__restrict__ A)
 {
-    const double rake = atan2(yy[3], yy[2]);
-    const double vel = exp(yy[6] * E_LG10);
-    const double cr = cos(rake), sr = sin(rake);
-    const double dth = (exp(-yy[5] * E_LG10) - vel / L) / E_LG10;
+    __shared__ double sh[7 * EW_THREADS];
+    const int gi = geom_of(A, blockIdx.x, false);
+    const GeomDev &G = A->g[gi];
+    EwBlock b;
+    if (!ew_block(G, b)) return;                     // uniform over the block
+    InstCtl *c = G.ctl + b.i;
+    const bool pend = c->pending;
+    const bool work = inst_live(c, A->glob) && c->need_stage1;
+    if (pend || work) {
+#pragma unroll
+        for (int u = 0; u < 7; u++) {
+            const int f = threadIdx.x + u * EW_THREADS;
+            if (f >= 7 * b.ne) break;
+            const long x = b.base + f;
+            const double v = pend ? G.ycand[x] : G.y[x];
+            if (pend) G.y[x] = v;
+            sh[f] = v;
+        }
+    }
+    __syncthreads();
+    ens_sources<1>(A, G, c, b, work, sh);
+}
+
+// the stage rate of one element (ratestate.f90:731-776) from the speed and slip
+// direction of its stage state, exp(-psi ln 10) and its traction rate t
+__device__ __forceinline__ void ens_rate(double vel, double cr, double sr, double eth, const double t[3], double L,
+                                         double bb, double sg, double aa, double eta, double *k)
+{
+    const double dth = (eth - vel / L) / E_LG10;
     const double dtau = t[0] * cr + t[1] * sr;
     const double dv = (dtau - bb * sg * dth * E_LG10) / (aa * sg + eta * vel) / E_LG10;
     const double corr = eta * vel * dv * E_LG10;
@@ -1651,50 +1672,68 @@ __device__ __forceinline__ void ens_rate(const double *yy, const double t[3], do
     k[6] = dv;
 }
 
-// traction rates from the contraction and the rate-state right-hand side
-// (ratestate.f90:731-776 per instance).  The block's contiguous state range and
-// rate range go through shared memory (coalesced); a hierarchical geometry
-// gathers each element's partial sums from the cluster order.
-// 12 blocks per SM (40 registers, a few spilled): the kernel waits on memory,
-// and more resident warps hide it better than fewer that spill nothing
-// (measured at N = 20k x 64: 5.96 ms per attempt against 6.08 at 80 registers)
+// Stage S behind its contraction: traction rates from the partial sums, the
+// rate-state right-hand side (ratestate.f90:731-776), and, of the same block of
+// elements, the next stage's state and sources; after stage 6 the candidate, the
+// error estimate and max |yerr / yscal| (ode45.f90:184-200, 68-76).
+// Memory and latency bound.  One kernel where the right-hand side, the next
+// stage's state and the error norm were three: a stage's rate, its state and the
+// error vector are not read back (31 state arrays an attempt instead of 49), the
+// transcendentals run once, and an attempt of a dense geometry is 14 launches
+// instead of 20.  The sums over the earlier stages are formed before the partial
+// sums are read, so that the two chains of loads overlap; 8 blocks of 64
+// registers an SM (a few spilled).  An attempt, contractions included: 2,048
+// rectangles x 64 290 -> 245 us, 7,200 triangles x 64 hierarchical 1,420 ->
+// 1,355 us.
 template <int S>
-__global__ void __launch_bounds__(EW_THREADS, 12) k_ens_rhs(const EnsArgs *__restrict__ A)
+__global__ void __launch_bounds__(EW_THREADS, EW_BLOCKS) k_ens_stage(const EnsArgs *__restrict__ A)
 {
     __shared__ double sh[7 * EW_THREADS];
     const int gi = geom_of(A, blockIdx.x, false);
     const GeomDev &G = A->g[gi];
-    const int local = blockIdx.x - G.blk_e0;
-    const int i = local / G.epb_e;
-    const int e0 = (local % G.epb_e) * EW_THREADS;
-    if (i >= G.ninst) return;                        // uniform over the block
-    const InstCtl *c = G.ctl + i;
-    if (!inst_live(c, A->glob) || (S == 1 && !c->need_stage1)) return;
-    const int ne = min(EW_THREADS, G.np - e0);
-    const int el = e0 + threadIdx.x;
-    const bool valid = threadIdx.x < ne;
-    const double *ysrc = (S == 1) ? G.y : G.ys;
-    double *ks = G.k[S - 1];
-    const long base = (long)i * 7 * G.np + 7L * e0;
+    EwBlock b;
+    if (!ew_block(G, b)) return;                     // uniform over the block
+    InstCtl *c = G.ctl + b.i;
+    if (!inst_live(c, A->glob)) return;
+    const bool rate = S > 1 || c->need_stage1;       // a rejected attempt keeps its stage-1 rate
+    const double h = c->h;
+    const int n = 7 * b.ne;
+    // what the sums over the earlier stages come to, while the partial sums load
+    double y[7], r[7], er[S == 6 ? 7 : 1];
 #pragma unroll
     for (int u = 0; u < 7; u++) {
         const int f = threadIdx.x + u * EW_THREADS;
-        if (f < 7 * ne) sh[f] = ysrc[base + f];
+        y[u] = r[u] = 0.0;
+        if (f >= n) continue;
+        const long x = b.base + f;
+        y[u] = G.y[x];
+        if (S < 6) {
+            if (S > 1) r[u] = __dmul_rn(e_B[S < 6 ? S : 0][0], G.k[0][x]);
+#pragma unroll
+            for (int j = 1; j < S - 1; j++) r[u] = __dadd_rn(r[u], __dmul_rn(e_B[S < 6 ? S : 0][j], G.k[j][x]));
+        } else {
+            const double k1 = G.k[0][x], k3 = G.k[2][x], k4 = G.k[3][x], k5 = G.k[4][x];
+            double q = __dmul_rn(E_C1, k1);
+            q = __dadd_rn(q, __dmul_rn(E_C3, k3));
+            r[u] = __dadd_rn(q, __dmul_rn(E_C4, k4));
+            q = __dmul_rn(E_DC1, k1);
+            q = __dadd_rn(q, __dmul_rn(E_DC3, k3));
+            q = __dadd_rn(q, __dmul_rn(E_DC4, k4));
+            er[S == 6 ? u : 0] = __dadd_rn(q, __dmul_rn(E_DC5, k5));
+        }
     }
-    __syncthreads();
-    if (valid) {
-        const int e = el;
-        double t[3];
-        double *t1 = G.t1 + (long)i * 3 * G.np + 3L * e;
+    if (threadIdx.x < b.ne && rate) {
+        const int e = b.e0 + threadIdx.x;
+        double inc[3], t[3];
+        double *t1 = G.t1 + (long)b.i * 3 * G.np + 3L * e;
         // a hierarchical geometry's partial sums lie in the cluster order: the
         // element's permuted position finds them (a gather of a few floats per
         // row, while the state and the rate stay coalesced)
-        double inc[3];
         if (G.hier) {
-            traction_rows_h(A, G, i, G.hinv[e], inc);
+            traction_rows_h(A, G, b.i, G.hinv[e], inc);
         } else {
 #pragma unroll
-            for (int q = 0; q < 3; q++) inc[q] = traction_row(A, G, i, 3L * e + q, S > 1 && !A->glob->inc_full);
+            for (int q = 0; q < 3; q++) inc[q] = traction_row(A, G, b.i, 3L * e + q, S > 1 && !A->glob->inc_full);
         }
 #pragma unroll
         for (int q = 0; q < 3; q++) {
@@ -1705,72 +1744,47 @@ __global__ void __launch_bounds__(EW_THREADS, 12) k_ens_rhs(const EnsArgs *__res
                 t[q] = t1[q] + inc[q];
             }
         }
-        const long pe = (long)i * G.np + e;
+        const long pe = (long)b.i * G.np + e;
         double k[7];
-        ens_rate(sh + 7 * threadIdx.x, t, G.L[pe], G.b[pe], G.sig[pe], G.a[pe], G.damping[pe], k);
-        for (int q = 0; q < 7; q++) sh[7 * threadIdx.x + q] = k[q];   // each thread its own slots
+        ens_rate(G.vel[pe], G.cr[pe], G.sr[pe], G.eth[pe], t, G.L[pe], G.b[pe], G.sig[pe], G.a[pe], G.damping[pe], k);
+        for (int q = 0; q < 7; q++) sh[7 * threadIdx.x + q] = k[q];
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 7; u++) {
-        const int f = threadIdx.x + u * EW_THREADS;
-        if (f < 7 * ne) ks[base + f] = sh[f];
-    }
-}
-
-#define E_C1 (37.0 / 378.0)
-#define E_C3 (250.0 / 621.0)
-#define E_C4 (125.0 / 594.0)
-#define E_C6 (512.0 / 1771.0)
-#define E_DC1 (E_C1 - 2825.0 / 27648.0)
-#define E_DC3 (E_C3 - 18575.0 / 48384.0)
-#define E_DC4 (E_C4 - 13525.0 / 55296.0)
-#define E_DC5 (-277.0 / 14336.0)
-#define E_DC6 (E_C6 - 0.25)
-
-// candidate, error estimate and max |yerr/yscal| per instance (ode45.f90:184-200, 68-76)
-__global__ void k_ens_finish(const EnsArgs *__restrict__ A)
-{
-    const int gi = geom_of(A, blockIdx.x, true);
-    const GeomDev &G = A->g[gi];
-    const int local = blockIdx.x - G.blk_s0;
-    const int i = local / G.epb_s;
-    if (i >= G.ninst) return;
-    InstCtl *c = G.ctl + i;
-    if (!inst_live(c, A->glob)) return;        // uniform over the block
-    const long len = 7L * G.np;
-    const long j0 = (long)(local % G.epb_s) * ST_SPAN + threadIdx.x;
-    const double h = c->h;
+    double *ks = G.k[S < 6 ? S - 1 : 0];
     double mx = 0.0;
     bool bad = false;
 #pragma unroll
-    for (int u = 0; u < ST_PER; u++) {
-        const long j = j0 + (long)u * ST_THREADS;
-        if (j < len) {
-            const long x = (long)i * len + j;
-            const double k1 = G.k[0][x], k3 = G.k[2][x], k4 = G.k[3][x], k5 = G.k[4][x], k6 = G.k[5][x];
-            double r = __dmul_rn(E_C1, k1);
-            r = __dadd_rn(r, __dmul_rn(E_C3, k3));
-            r = __dadd_rn(r, __dmul_rn(E_C4, k4));
-            r = __dadd_rn(r, __dmul_rn(E_C6, k6));
-            const double yc = __dadd_rn(G.y[x], __dmul_rn(h, r));
-            double er = __dmul_rn(E_DC1, k1);
-            er = __dadd_rn(er, __dmul_rn(E_DC3, k3));
-            er = __dadd_rn(er, __dmul_rn(E_DC4, k4));
-            er = __dadd_rn(er, __dmul_rn(E_DC5, k5));
-            er = __dadd_rn(er, __dmul_rn(E_DC6, k6));
-            er = __dmul_rn(h, er);
+    for (int u = 0; u < 7; u++) {
+        const int f = threadIdx.x + u * EW_THREADS;
+        if (f >= n) break;
+        const long x = b.base + f;
+        const double k = rate ? sh[f] : ks[x];
+        if (S < 6) {
+            if (rate) ks[x] = k;
+            if (S == 1) {
+                if (rate) G.yscal[x] = fabs(y[u]) + fabs(h * k) + 1.0e-30;
+                sh[f] = __dadd_rn(y[u], __dmul_rn(__dmul_rn(h, e_B[1][0]), k));
+            } else {
+                sh[f] = __dadd_rn(y[u], __dmul_rn(h, __dadd_rn(r[u], __dmul_rn(e_B[S < 6 ? S : 0][S < 6 ? S - 1 : 0], k))));
+            }
+        } else {
+            const double yc = __dadd_rn(y[u], __dmul_rn(h, __dadd_rn(r[u], __dmul_rn(E_C6, k))));
+            const double ee = __dmul_rn(h, __dadd_rn(er[S == 6 ? u : 0], __dmul_rn(E_DC6, k)));
             G.ycand[x] = yc;
-            G.yerr[x] = er;
-            mx = fmax(mx, fabs(er / G.yscal[x]));
+            mx = fmax(mx, fabs(ee / G.yscal[x]));
             bad = bad || !isfinite(yc);
         }
     }
-    for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-    bad = __any_sync(0xffffffffu, bad);
-    if ((threadIdx.x & 31) == 0) {
-        if (mx > 0.0) atomicMax(&c->errbits, (unsigned long long)__double_as_longlong(mx));
-        if (bad) c->nonfinite = 1;
+    if (S < 6) {
+        __syncthreads();
+        ens_sources<S < 6 ? S + 1 : 6>(A, G, c, b, true, sh);
+    } else {
+        for (int off = 16; off > 0; off >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        bad = __any_sync(0xffffffffu, bad);
+        if ((threadIdx.x & 31) == 0) {
+            if (mx > 0.0) atomicMax(&c->errbits, (unsigned long long)__double_as_longlong(mx));
+            if (bad) c->nonfinite = 1;
+        }
     }
 }
 
@@ -1984,7 +1998,7 @@ struct EnsGeomHost {
     float *rscale = nullptr;
     float *kscale = nullptr;   // dense: K image scale per [mtile][kblock]
     float *vscale = nullptr;   // dense: V image scale per [ntile][kblock][ni]
-    double *state = nullptr;   // 12 vectors of ninst * 7 np
+    double *state = nullptr;   // STATE_VECS vectors of ninst * 7 np
     double *anchor = nullptr;  // v1 (ninst * 2 np) then t1 (ninst * 3 np)
     double *par = nullptr;     // 7 vectors of ninst * np
     InstCtl *ctl = nullptr;
@@ -2868,14 +2882,13 @@ int install_plan(ucg_ensemble *E, int ni, const Sched &s1, const Sched &s2)
         const long len = (long)g.ninst * 7 * g.np;
         double *v = g.state;
         d.y = v; v += len;
-        d.ys = v; v += len;
-        for (int j = 0; j < 6; j++) { d.k[j] = v; v += len; }
+        for (int j = 0; j < 5; j++) { d.k[j] = v; v += len; }
         d.ycand = v; v += len;
-        d.yerr = v; v += len;
         d.yscal = v; v += len;
         d.v1 = g.anchor;
         d.t1 = g.anchor + 2L * g.ninst * g.np;
         const long pl = (long)g.ninst * g.np;
+        d.vel = v; d.cr = v + pl; d.sr = v + 2 * pl; d.eth = v + 3 * pl;
         d.vpl_c = g.par; d.vpl_s = g.par + pl; d.a = g.par + 2 * pl; d.b = g.par + 3 * pl;
         d.sig = g.par + 4 * pl; d.L = g.par + 5 * pl; d.damping = g.par + 6 * pl;
         d.ctl = g.ctl;
@@ -2977,14 +2990,31 @@ int time_contract(ucg_ensemble *E, int reps, double *ms, bool klo = true)
     return UCG_OK;
 }
 
-// one Runge-Kutta stage for every instance
+// one Runge-Kutta stage for every instance: the contraction of the sources that
+// the kernel before it wrote, then the rest
 template <int S>
 cudaError_t enqueue_stage(ucg_ensemble *E, int be)
 {
-    k_ens_prologue<S><<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
     cudaError_t e = launch_all(E, S == 1 || E->inc_full);
     if (e != cudaSuccess) return e;
-    k_ens_rhs<S><<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
+    k_ens_stage<S><<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
+    E->launches += 1;
+    return cudaGetLastError();
+}
+
+// one attempt of every instance
+cudaError_t enqueue_attempt(ucg_ensemble *E, int be, cudaGraphConditionalHandle cond, int in_graph)
+{
+    k_ens_start<<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = enqueue_stage<1>(E, be);
+    if (e == cudaSuccess) e = enqueue_stage<2>(E, be);
+    if (e == cudaSuccess) e = enqueue_stage<3>(E, be);
+    if (e == cudaSuccess) e = enqueue_stage<4>(E, be);
+    if (e == cudaSuccess) e = enqueue_stage<5>(E, be);
+    if (e == cudaSuccess) e = enqueue_stage<6>(E, be);
+    if (e != cudaSuccess) return e;
+    k_ens_control<<<1, CTL_THREADS, 0, E->stream>>>(E->d_args, cond, in_graph);
     E->launches += 2;
     return cudaGetLastError();
 }
@@ -3024,15 +3054,7 @@ int build_graph(ucg_ensemble *E)
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         e = cudaStreamBeginCaptureToGraph(E->stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            cudaError_t le = enqueue_stage<1>(E, be);
-            if (le == cudaSuccess) le = enqueue_stage<2>(E, be);
-            if (le == cudaSuccess) le = enqueue_stage<3>(E, be);
-            if (le == cudaSuccess) le = enqueue_stage<4>(E, be);
-            if (le == cudaSuccess) le = enqueue_stage<5>(E, be);
-            if (le == cudaSuccess) le = enqueue_stage<6>(E, be);
-            k_ens_finish<<<bs, ST_THREADS, 0, E->stream>>>(E->d_args);
-            k_ens_control<<<1, CTL_THREADS, 0, E->stream>>>(E->d_args, cond, 1);
-            E->launches += 2;
+            const cudaError_t le = enqueue_attempt(E, be, cond, 1);
             cudaGraph_t tmp;
             e = cudaStreamEndCapture(E->stream, &tmp);
             if (e == cudaSuccess && le != cudaSuccess) e = le;
@@ -3163,11 +3185,11 @@ int ucg_ens_add_geometry(ucg_ensemble *E, ucg_ctx *c, int n_instances, int *geom
         if (e == cudaSuccess) e = cudaMalloc(&g.rscale, sizeof(float) * rows_pad);
         if (e == cudaSuccess) e = cudaMalloc(&g.kscale, sizeof(float) * (size_t)g.mtiles * g.kblocks);
     }
-    if (e == cudaSuccess) e = cudaMalloc(&g.state, sizeof(double) * 12 * len);
+    if (e == cudaSuccess) e = cudaMalloc(&g.state, sizeof(double) * STATE_VECS * len);
     if (e == cudaSuccess) e = cudaMalloc(&g.anchor, sizeof(double) * 5L * g.ninst * g.np);
     if (e == cudaSuccess) e = cudaMalloc(&g.par, sizeof(double) * 7L * g.ninst * g.np);
     if (e == cudaSuccess) e = cudaMalloc(&g.ctl, sizeof(InstCtl) * g.ninst);
-    if (e == cudaSuccess) e = cudaMemsetAsync(g.state, 0, sizeof(double) * 12 * len, E->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(g.state, 0, sizeof(double) * STATE_VECS * len, E->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.anchor, 0, sizeof(double) * 5L * g.ninst * g.np, E->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(g.par, 0, sizeof(double) * 7L * g.ninst * g.np, E->stream);
     if (e == cudaSuccess) {
@@ -3350,7 +3372,7 @@ int ucg_ens_put_states(ucg_ensemble *E, int gi, const double *y)
     EnsGeomHost &g = E->geoms[gi];
     ECUDA(cudaSetDevice(E->device));
     const long len = 7L * g.np, total = len * g.ninst;
-    double *staged = g.state + 8 * total;   // the candidate vector: free between launches
+    double *staged = g.state + STATE_CAND * total;   // the candidate vector: free between launches
     ECUDA(cudaMemcpyAsync(staged, y, sizeof(double) * total, cudaMemcpyHostToDevice, E->stream));
     const int blocks = (int)std::min<long>((total + 255) / 256, 4L * 148);
     ens::k_ens_put<<<blocks, 256, 0, E->stream>>>(g.state, staged, g.ctl, len, total);
@@ -3514,16 +3536,8 @@ int run_eager(ucg_ensemble *E)
     k_ens_begin<<<1, 256, 0, E->stream>>>(E->d_args);
     E->launches++;
     for (long a = 0; a < E->h_glob->budget; a++) {
-        cudaError_t le = enqueue_stage<1>(E, be);
-        if (le == cudaSuccess) le = enqueue_stage<2>(E, be);
-        if (le == cudaSuccess) le = enqueue_stage<3>(E, be);
-        if (le == cudaSuccess) le = enqueue_stage<4>(E, be);
-        if (le == cudaSuccess) le = enqueue_stage<5>(E, be);
-        if (le == cudaSuccess) le = enqueue_stage<6>(E, be);
+        const cudaError_t le = enqueue_attempt(E, be, 0, 0);
         if (le != cudaSuccess) return efail(E, le, "ensemble attempt");
-        k_ens_finish<<<bs, ST_THREADS, 0, E->stream>>>(E->d_args);
-        k_ens_control<<<1, CTL_THREADS, 0, E->stream>>>(E->d_args, 0, 0);
-        E->launches += 2;
         if ((a & 15) == 15 || a + 1 == E->h_glob->budget) {
             EnsGlobal g;
             ECUDA(cudaMemcpyAsync(&g, E->d_glob, sizeof g, cudaMemcpyDeviceToHost, E->stream));
