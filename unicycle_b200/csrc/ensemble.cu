@@ -406,7 +406,11 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
 
     if (warp == 0) {
         if (lane == 0) {
-            // producer: per k-block one copy of K per M-tile of the unit and one copy of V
+            // producer: per k-block one copy of K per M-tile of the unit and one copy of V.
+            // The first segment's K copies that fit the ring are under way before the
+            // kernel before this one has ended: K does not depend on it, V does (the
+            // first operands used to land 2.7 us after the launch; with the launches
+            // overlapped, 2,048 rectangles x 64: 250 -> 236 us an attempt)
             const uint64_t pol_a = l2_policy(false), pol_b = l2_policy(true);
             long issued = 0;
             // the next segments' descriptors are loaded ahead (segment two
@@ -414,6 +418,19 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
             GemmSeg s1 = q0 < q1 ? segs[q0] : GemmSeg{0, 0, 0, 0};
             GemmSeg s2 = q0 + 1 < q1 ? segs[q0 + 1] : s1;
             GemmTile t1 = q0 < q1 ? tiles[s1.tile] : GemmTile{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+            const int pre = hold ? 0 : min(s1.kb1 - s1.kb0, T::STAGES);
+            for (int j = 0; j < pre; j++) {
+                const bool two = MT == 2 && t1.a1 != nullptr;
+                uint8_t *st = smem + (size_t)j * T::STAGE;
+                bar_expect_tx(&full[j], (uint32_t)((two ? 2 : 1) * T::A_BYTES + T::B_IMG));
+                bulk_load_hint(st, t1.a + (size_t)(s1.kb0 + j) * A_IMG, T::A_BYTES, &full[j], pol_a);
+                if (two)
+                    bulk_load_hint(st + T::A_BYTES, t1.a1 + (size_t)(s1.kb0 + j) * A_IMG, T::A_BYTES, &full[j], pol_a);
+            }
+            pdl_wait();
+            for (; issued < pre; issued++)
+                bulk_load_hint(smem + (size_t)issued * T::STAGE + MT * T::A_BYTES,
+                               t1.b + (size_t)(s1.kb0 + issued) * T::B_IMG, T::B_IMG, &full[issued], pol_b);
             for (int q = q0; q < q1 && !abort_flag && !hold; q++) {
                 const GemmSeg sg = s1;
                 const GemmTile tl = t1;
@@ -422,7 +439,7 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
                 if (q + 2 < q1) s2 = segs[q + 2];
                 const bool two = MT == 2 && tl.a1 != nullptr;
                 const uint32_t bytes = (uint32_t)((two ? 2 : 1) * T::A_BYTES + T::B_IMG);
-                for (int kb = sg.kb0; kb < sg.kb1; kb++) {
+                for (int kb = sg.kb0 + (q == q0 ? pre : 0); kb < sg.kb1; kb++) {
                     const int s = (int)(issued % T::STAGES);
                     const uint32_t ph = (uint32_t)((issued / T::STAGES) & 1);
                     if (!bar_wait(&empty[s], ph ^ 1u, &abort_flag, lim)) {
@@ -442,7 +459,9 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
                 bar_wait(&full[i % T::STAGES], (uint32_t)((i / T::STAGES) & 1), nullptr);
         }
     } else if (warp == 1) {
+        pdl_wait();
         if (lane == 0) {
+            pdl_launch();
             long it = 0;
             int tc = 0;
             bool issued_any = false;
@@ -528,6 +547,7 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
         // Every k-block's partial sums (hi products + 2^-11 lo products, times
         // the K block and V block scales) are added in FP64 registers; a
         // segment's sums go to the workspace when its last k-block is in
+        pdl_wait();       // the sums' last readers are done, the V scales written
         const int quarter = warp & 3;
         const int grp = (warp - 2) >> 2;
         const int row = quarter * 32 + lane;
@@ -743,6 +763,11 @@ __device__ __forceinline__ uint64_t cm_desc(uint32_t saddr, uint32_t lbo, uint32
            ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1u << 46);
 }
 
+// Its operand images come before the kernel in front has ended; the kernel
+// behind starts when this one ends: started from within it (as the dense contraction
+// does), blocks that wait beside its CTAs cost more than they save (7,200
+// triangles x 64: 1,400 us an attempt against 1,320, 1,360 without any
+// programmatic launch)
 template <int NI, bool KLO, int PL>
 __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUnit *__restrict__ units,
         const HSeg *__restrict__ segs, const int *__restrict__ cta_seg, float *__restrict__ ws, int *err)
@@ -826,6 +851,7 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
                 for (int kg = sg.kg0; kg < sg.kg1; kg += T::KG) {
                     const int nk = min(T::KG, sg.kg1 - kg);
                     const int s = (int)(issued % T::SA);
+                    if (issued == T::SA) pdl_wait();    // the ring is full: what empties it waits for the kernel before
                     const uint32_t ph = (uint32_t)((issued / T::SA) & 1);
                     if (!bar_wait(&emptyA[s], ph ^ 1u, &abort_flag)) {
                         if (!abort_flag) fail();
@@ -852,6 +878,7 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
         // B: the whole warp loads the B K-groups of 32 stages at once (lane l:
         // stage l); lane 0 takes each stage's from its lane by shuffle and
         // issues one copy per run of consecutive B K-groups
+        pdl_wait();
         const uint64_t pol_b = l2_policy(true);
         long issued = 0;
         bool stop = false;
@@ -923,6 +950,7 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
             for (long i = issued - T::SB > 0 ? issued - T::SB : 0; i < issued; i++)
                 bar_wait(&fullB[i % T::SB], (uint32_t)((i / T::SB) & 1), nullptr);
     } else if (warp == 1) {
+        pdl_wait();
         if (lane == 0) {
             long it = 0;
             int tc = 0;
@@ -990,6 +1018,7 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
     } else {
         // drain: warp w reads tensor-memory lanes 32 (w mod 4) .. +31 = unit rows;
         // rows past the unit's 8-row groups are not written
+        pdl_wait();       // the sums' and Z's last readers are done
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;
         int tc = 0;
@@ -1241,6 +1270,8 @@ __global__ void k_hm_zconv(const HZUnit *__restrict__ zu, const long *__restrict
                            const float *__restrict__ ws, int ni)
 {
     const HZUnit U = zu[blockIdx.x];
+    pdl_wait();
+    pdl_launch();
     for (int w = threadIdx.x; w < U.g * ni; w += blockDim.x) {
         const int grp = w / ni, i = w % ni;
         double z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -1635,7 +1666,10 @@ __global__ void __launch_bounds__(EW_THREADS) k_ens_start(const EnsArgs *__restr
     const int gi = geom_of(A, blockIdx.x, false);
     const GeomDev &G = A->g[gi];
     EwBlock b;
-    if (!ew_block(G, b)) return;                     // uniform over the block
+    const bool any = ew_block(G, b);                 // uniform over the block
+    pdl_wait();
+    pdl_launch();
+    if (!any) return;
     InstCtl *c = G.ctl + b.i;
     const bool pend = c->pending;
     const bool work = inst_live(c, A->glob) && c->need_stage1;
@@ -1684,7 +1718,7 @@ __device__ __forceinline__ void ens_rate(double vel, double cr, double sr, doubl
 // sums are read, so that the two chains of loads overlap; 8 blocks of 64
 // registers an SM (a few spilled).  An attempt, contractions included: 2,048
 // rectangles x 64 290 -> 245 us, 7,200 triangles x 64 hierarchical 1,420 ->
-// 1,355 us.
+// 1,355 us.  Launched while the contraction runs (236 and 1,320).
 template <int S>
 __global__ void __launch_bounds__(EW_THREADS, EW_BLOCKS) k_ens_stage(const EnsArgs *__restrict__ A)
 {
@@ -1692,13 +1726,17 @@ __global__ void __launch_bounds__(EW_THREADS, EW_BLOCKS) k_ens_stage(const EnsAr
     const int gi = geom_of(A, blockIdx.x, false);
     const GeomDev &G = A->g[gi];
     EwBlock b;
-    if (!ew_block(G, b)) return;                     // uniform over the block
+    if (!ew_block(G, b)) {                           // uniform over the block
+        pdl_wait();
+        return;
+    }
     InstCtl *c = G.ctl + b.i;
-    if (!inst_live(c, A->glob)) return;
     const bool rate = S > 1 || c->need_stage1;       // a rejected attempt keeps its stage-1 rate
     const double h = c->h;
-    const int n = 7 * b.ne;
-    // what the sums over the earlier stages come to, while the partial sums load
+    const int n = c->active && c->status == 0 ? 7 * b.ne : 0;
+    // what the sums over the earlier stages come to, while the contraction still
+    // runs: all of it is from before that, whose blocks let this kernel start only
+    // once they had waited for the kernels before them
     double y[7], r[7], er[S == 6 ? 7 : 1];
 #pragma unroll
     for (int u = 0; u < 7; u++) {
@@ -1722,6 +1760,9 @@ __global__ void __launch_bounds__(EW_THREADS, EW_BLOCKS) k_ens_stage(const EnsAr
             er[S == 6 ? u : 0] = __dadd_rn(q, __dmul_rn(E_DC5, k5));
         }
     }
+    pdl_wait();
+    pdl_launch();
+    if (!inst_live(c, A->glob)) return;
     if (threadIdx.x < b.ne && rate) {
         const int e = b.e0 + threadIdx.x;
         double inc[3], t[3];
@@ -1797,6 +1838,7 @@ constexpr int CTL_THREADS = 512;    // 16 warps: up to 16 model evaluations in o
 __global__ void __launch_bounds__(CTL_THREADS) k_ens_control(const EnsArgs *__restrict__ A,
                                                                cudaGraphConditionalHandle cond, int in_graph)
 {
+    pdl_wait();
     EnsGlobal *gl = A->glob;
     const double SAFETY = 0.7, PGROW = -0.2, PSHRNK = -0.15, ERRCON = 1.89e-4;
     __shared__ mlp::Norm norm;
@@ -2626,10 +2668,9 @@ template <int NI, bool KLO, int PL>
 cudaError_t launch_hpass_t(ucg_ensemble *E, const HPlanBufs &P)
 {
     using T = HTile<NI, KLO, PL>;
-    k_hm_contract<NI, KLO, PL><<<T::CTAS * E->sms, 224, T::SMEM, E->stream>>>(P.units, P.segs, P.cta, P.ws,
-                                                                           &E->d_glob->err);
     E->launches++;
-    return cudaGetLastError();
+    return launch_pdl(k_hm_contract<NI, KLO, PL>, T::CTAS * E->sms, 224, T::SMEM, E->stream, P.units, P.segs, P.cta,
+                      P.ws, &E->d_glob->err);
 }
 
 // three planes: every stage in the one form (the increments' two-term option
@@ -2659,12 +2700,9 @@ cudaError_t launch_hier(ucg_ensemble *E, bool klo)
         e = launch_hpass(E, E->h1, klo);
         if (e != cudaSuccess) return e;
         if (E->h1.nzu > 0) {
-            if (E->hplanes == 3)
-                k_hm_zconv<3><<<E->h1.nzu, 256, 0, E->stream>>>(E->h1.zu, E->h1.pws, E->h1.ws, E->ni);
-            else
-                k_hm_zconv<2><<<E->h1.nzu, 256, 0, E->stream>>>(E->h1.zu, E->h1.pws, E->h1.ws, E->ni);
+            e = launch_pdl(E->hplanes == 3 ? k_hm_zconv<3> : k_hm_zconv<2>, E->h1.nzu, 256, 0, E->stream, E->h1.zu,
+                           E->h1.pws, E->h1.ws, E->ni);
             E->launches++;
-            e = cudaGetLastError();
             if (e != cudaSuccess) return e;
         }
     }
@@ -2703,10 +2741,9 @@ cudaError_t prepare_contract(int ni, int planes)
 template <int NI, bool KLO, int MT>
 cudaError_t launch_contract_t(ucg_ensemble *E, const PlanBufs &P)
 {
-    k_bf16x3_contract<NI, KLO, MT><<<E->sms, 320, Tile<NI, KLO, MT>::SMEM, E->stream>>>(P.tiles, P.segs, P.cta,
-                                                                                        P.ws, E->d_glob);
     E->launches++;
-    return cudaGetLastError();
+    return launch_pdl(k_bf16x3_contract<NI, KLO, MT>, E->sms, 320, Tile<NI, KLO, MT>::SMEM, E->stream, P.tiles, P.segs,
+                      P.cta, P.ws, E->d_glob);
 }
 
 // klo: the anchor's contraction (K hi and lo, single M-tiles); otherwise the
@@ -2997,16 +3034,14 @@ cudaError_t enqueue_stage(ucg_ensemble *E, int be)
 {
     cudaError_t e = launch_all(E, S == 1 || E->inc_full);
     if (e != cudaSuccess) return e;
-    k_ens_stage<S><<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
-    E->launches += 1;
-    return cudaGetLastError();
+    E->launches++;
+    return launch_pdl(k_ens_stage<S>, be, EW_THREADS, 0, E->stream, E->d_args);
 }
 
 // one attempt of every instance
 cudaError_t enqueue_attempt(ucg_ensemble *E, int be, cudaGraphConditionalHandle cond, int in_graph)
 {
-    k_ens_start<<<be, EW_THREADS, 0, E->stream>>>(E->d_args);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pdl(k_ens_start, be, EW_THREADS, 0, E->stream, E->d_args);
     if (e == cudaSuccess) e = enqueue_stage<1>(E, be);
     if (e == cudaSuccess) e = enqueue_stage<2>(E, be);
     if (e == cudaSuccess) e = enqueue_stage<3>(E, be);
@@ -3014,9 +3049,8 @@ cudaError_t enqueue_attempt(ucg_ensemble *E, int be, cudaGraphConditionalHandle 
     if (e == cudaSuccess) e = enqueue_stage<5>(E, be);
     if (e == cudaSuccess) e = enqueue_stage<6>(E, be);
     if (e != cudaSuccess) return e;
-    k_ens_control<<<1, CTL_THREADS, 0, E->stream>>>(E->d_args, cond, in_graph);
     E->launches += 2;
-    return cudaGetLastError();
+    return launch_pdl(k_ens_control, 1, CTL_THREADS, 0, E->stream, E->d_args, cond, in_graph);
 }
 
 int build_graph(ucg_ensemble *E)

@@ -509,25 +509,6 @@ int keep_blocks(ucg_ctx *c, const std::vector<KeepJob> &jobs)
 // be scheduled and waits for the ones before it itself, the row kernel only after
 // it has asked for its panel, which does not depend on them.
 
-__device__ __forceinline__ void hm_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void hm_pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-static cudaError_t hm_launch(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
-}
-
 // v in the permuted element order (so that every block's columns are a
 // contiguous range of xp)
 __global__ void k_hm_gather(const int *__restrict__ perm, int np, const double *__restrict__ v,
@@ -736,8 +717,8 @@ __global__ void __launch_bounds__(HM_THREADS) k_hm_rows(HmProduct P, int zblocks
         const bool z = slot < both ? !(slot & 1) : zblocks > P.n_dense;
         slot = slot < both ? slot >> 1 : slot - (both >> 1);
         if (z) {
-            hm_pdl_wait();
-            hm_pdl_launch();
+            pdl_wait();
+            pdl_launch();
             hm_z<SPLIT>(P, ((long)slot * blockDim.x + threadIdx.x) >> 5);
             return;
         }
@@ -760,8 +741,8 @@ __global__ void __launch_bounds__(HM_THREADS) k_hm_rows(HmProduct P, int zblocks
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                          ::"r"(hm_smem(sb + nel)), "l"(P.pl + ch.off), "r"(half), "r"(hm_smem(&bar)) : "memory");
     }
-    hm_pdl_wait();
-    hm_pdl_launch();
+    pdl_wait();
+    pdl_launch();
     double *part = P.part + (long)ch.id * P.rows_max + i;
     if (nel == 0) {
         if (i < rows) *part = 0.0;
@@ -1275,10 +1256,10 @@ static void launch_products(ucg_ctx *c)
     const size_t smem = (SPLIT ? HM_CHUNK_BYTES / 2 : HM_CHUNK_BYTES) + sizeof(double) * h->max_cols;
     const int thr = (3 * h->max_leaf + 31) & ~31;
     const int zb = (int)((h->n_items * 32 + thr - 1) / thr), lowrank = h->n_chunks - h->n_dense_chunks;
-    hm_launch(k_hm_rows<SPLIT, true>, dim3(zb + h->n_dense_chunks), dim3(thr), smem, c->stream, P, zb);
+    launch_pdl(k_hm_rows<SPLIT, true>, dim3(zb + h->n_dense_chunks), dim3(thr), smem, c->stream, P, zb);
     c->launches.count++;
     if (lowrank > 0) {
-        hm_launch(k_hm_rows<SPLIT, false>, dim3(lowrank), dim3(thr), smem, c->stream, P, 0);
+        launch_pdl(k_hm_rows<SPLIT, false>, dim3(lowrank), dim3(thr), smem, c->stream, P, 0);
         c->launches.count++;
     }
 }

@@ -90,29 +90,10 @@ __device__ __forceinline__ bool ctl_live(const Ctl *c) { return c->active && c->
 // its own successor be scheduled.  So the launch latency of every kernel of an
 // attempt overlaps the previous kernel instead of adding to it (it dominates
 // at small N).  Without a programmatic predecessor the wait returns at once.
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter()
 {
     pdl_wait();
     pdl_launch();
-}
-
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
 }
 
 __device__ __forceinline__ void atomic_max_pos(unsigned long long *p, double x)

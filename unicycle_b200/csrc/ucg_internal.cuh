@@ -298,4 +298,29 @@ int cuda_fail(ucg_ctx *c, cudaError_t e, const char *what);
         if (e_ != cudaSuccess) return ucg::cuda_fail(c, e_, #call); \
     } while (0)
 
+// Programmatic dependent launch: a kernel launched by launch_pdl may be scheduled
+// before its predecessor in the stream has ended, from the moment every block
+// of that has called pdl_launch or ended, and waits in pdl_wait until it has ended
+// and its writes are visible.  Every block of such a kernel waits, also one
+// with nothing to do: the kernels behind rely on it.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+
 }  // namespace ucg
