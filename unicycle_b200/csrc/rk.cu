@@ -1097,18 +1097,17 @@ __global__ void k_record(StageArgs a, const Ctl *ctl, Rec *rec)
     if (t == 0) rec->written = idx + 1;
 }
 
-__global__ void k_commit(StageArgs a, const Ctl *ctl)
+__global__ void k_commit(StageArgs a, Ctl *ctl)
 {
     pdl_enter();
-    if (!ctl->pending) return;
+    if (ctl_live(ctl) || !ctl->pending) return;      // the same in every block: the last one out clears it
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < a.len; i += (long)gridDim.x * blockDim.x)
         a.y[i] = a.ycand[i];
-}
-
-__global__ void k_clear_pending(Ctl *ctl)
-{
-    pdl_enter();
-    ctl->pending = 0;
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&ctl->committed, 1) == (int)gridDim.x - 1) {
+        ctl->committed = 0;
+        ctl->pending = 0;
+    }
 }
 
 // ---- host side -----------------------------------------------------------------
@@ -1319,8 +1318,7 @@ void rk_enqueue_commit(ucg_ctx *c)
 {
     StageArgs a = stage_args(c, 1, 0);
     launch_pdl(k_commit, dim3((unsigned)((c->state_len + 255) / 256)), dim3(256), 0, c->stream, a, c->ctl);
-    launch_pdl(k_clear_pending, dim3(1), dim3(1), 0, c->stream, c->ctl);
-    c->launches.count += 2;
+    c->launches.count += 1;
 }
 
 // Mean device time of the stage-2 traction launch (the dominant kernel), timed

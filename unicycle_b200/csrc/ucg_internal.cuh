@@ -48,6 +48,7 @@ struct Ctl {
     unsigned long long wait_ns;
     int test_hold;
     int ticket;        // CTAs of stage 6 that are done (the last one decides the attempt)
+    int committed;     // blocks of the commit that are done (the last one clears `pending`)
 };
 
 // Device-side output recorder (the reference's export/exportPoints,
