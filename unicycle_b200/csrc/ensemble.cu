@@ -1256,46 +1256,61 @@ __device__ __forceinline__ void put_x(uint8_t *Bt, int ni, int pl, int rr, int p
 }
 
 // pass 1's output into the B space for the units cut into several pieces (the
-// drain writes the others directly): one thread per (unit, 8-row group,
-// instance) adds the unit's partial sums in k order (FP64) and writes 8 rank
-// entries of Z as hi and lo
+// drain writes the others directly): a block per (unit, 8-row group), a thread per
+// instance, adds the unit's partial sums in k order (FP64) and writes 8 rank
+// entries of Z as its planes.  Latency bound: a stack over many sources has
+// some 60 pieces, whose loads are issued HZ_AHEAD pieces at a time (a block per
+// unit that walked them one by one took 18 us at 7,200 triangles x 64; now
+// 9.5)
 struct HZUnit {
     uint8_t *b;                 // the instance tile's B space
     const int *zdst;            // per 8-row group of the unit: its K-group in the B space
     int g, rows, p0, np, pad;
 };
 
+constexpr int HZ_AHEAD = 8;
+
 template <int PL>
-__global__ void k_hm_zconv(const HZUnit *__restrict__ zu, const long *__restrict__ pws,
-                           const float *__restrict__ ws, int ni)
+__global__ void __launch_bounds__(128) k_hm_zconv(const HZUnit *__restrict__ zu, const long *__restrict__ pws,
+                                                  const float *__restrict__ ws, int ni)
 {
     const HZUnit U = zu[blockIdx.x];
+    const int grp = blockIdx.y, i = threadIdx.x;
     pdl_wait();
     pdl_launch();
-    for (int w = threadIdx.x; w < U.g * ni; w += blockDim.x) {
-        const int grp = w / ni, i = w % ni;
-        double z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int p = 0; p < U.np; p++) {
-            const float4 *src = reinterpret_cast<const float4 *>(ws + pws[U.p0 + p] + (long)i * U.rows + grp * 8);
-            const float4 a = src[0], b = src[1];
-            z[0] += a.x; z[1] += a.y; z[2] += a.z; z[3] += a.w;
-            z[4] += b.x; z[5] += b.y; z[6] += b.z; z[7] += b.w;
-        }
-        uint32_t wd[PL][4];
+    if (grp >= U.g) return;
+    const float *src = ws + (long)i * U.rows + grp * 8;
+    double z[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int p0 = 0; p0 < U.np; p0 += HZ_AHEAD) {
+        float4 x[HZ_AHEAD][2];
 #pragma unroll
-        for (int k = 0; k < 8; k += 2) {
-            __nv_bfloat16 a[PL], b[PL];
-            split_planes<PL>(z[k], a);
-            split_planes<PL>(z[k + 1], b);
-#pragma unroll
-            for (int p = 0; p < PL; p++)
-                wd[p][k / 2] = (uint32_t)__bfloat16_as_ushort(a[p]) | ((uint32_t)__bfloat16_as_ushort(b[p]) << 16);
+        for (int j = 0; j < HZ_AHEAD; j++) {
+            if (p0 + j >= U.np) break;
+            const float4 *q = reinterpret_cast<const float4 *>(src + pws[U.p0 + p0 + j]);
+            x[j][0] = q[0];
+            x[j][1] = q[1];
         }
-        uint8_t *q = U.b + (size_t)U.zdst[grp] * (PL * ni * 16) + (size_t)(i >> 3) * 128 + (size_t)(i & 7) * 16;
+#pragma unroll
+        for (int j = 0; j < HZ_AHEAD; j++) {
+            if (p0 + j >= U.np) break;
+            z[0] += x[j][0].x; z[1] += x[j][0].y; z[2] += x[j][0].z; z[3] += x[j][0].w;
+            z[4] += x[j][1].x; z[5] += x[j][1].y; z[6] += x[j][1].z; z[7] += x[j][1].w;
+        }
+    }
+    uint32_t wd[PL][4];
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        __nv_bfloat16 a[PL], b[PL];
+        split_planes<PL>(z[k], a);
+        split_planes<PL>(z[k + 1], b);
 #pragma unroll
         for (int p = 0; p < PL; p++)
-            *reinterpret_cast<uint4 *>(q + (size_t)p * ni * 16) = make_uint4(wd[p][0], wd[p][1], wd[p][2], wd[p][3]);
+            wd[p][k / 2] = (uint32_t)__bfloat16_as_ushort(a[p]) | ((uint32_t)__bfloat16_as_ushort(b[p]) << 16);
     }
+    uint8_t *q = U.b + (size_t)U.zdst[grp] * (PL * ni * 16) + (size_t)(i >> 3) * 128 + (size_t)(i & 7) * 16;
+#pragma unroll
+    for (int p = 0; p < PL; p++)
+        *reinterpret_cast<uint4 *>(q + (size_t)p * ni * 16) = make_uint4(wd[p][0], wd[p][1], wd[p][2], wd[p][3]);
 }
 
 // ---- K images ----------------------------------------------------------------------
@@ -2585,7 +2600,14 @@ int upload_hplan(ucg_ensemble *E, HPlanBufs &P, int ni, int pass)
     std::vector<int> steps, w;
     for (const HUnit &u : units) {
         steps.push_back(u.nkg / 2);
-        w.push_back(u.g + 4);      // a K-step's bytes grow with the row groups; its MMAs do not
+        // what a K-step takes of shared memory, which bounds the kernel: its MMAs
+        // read 128 rows of the operand whatever the unit has, 32 KB with B
+        // (three planes, 64 instances), the copies write 6 KB of B and 0.75 KB a
+        // row group.  (Weighed by bytes of K, g + 4, a CTA with a stack of two row
+        // groups took 71,000 cycles beside the others' 25,000; both passes at
+        // 7,200 triangles x 64 148 -> 132 us, x 32 134 -> 115, two planes 84 -> 80.
+        // The line is flat: g + 16, 134 us, g + 200, 133.)
+        w.push_back(u.g + 49);
     }
     Sched s = sched_weighted(steps, w, hm_ctas(ni, E->hplanes) * E->sms);   // HTile<ni, *, planes>::CTAS per SM
     // 512 K-steps (8,192 K entries) per FP32 partial sum (three planes: of
@@ -2700,7 +2722,7 @@ cudaError_t launch_hier(ucg_ensemble *E, bool klo)
         e = launch_hpass(E, E->h1, klo);
         if (e != cudaSuccess) return e;
         if (E->h1.nzu > 0) {
-            e = launch_pdl(E->hplanes == 3 ? k_hm_zconv<3> : k_hm_zconv<2>, E->h1.nzu, 256, 0, E->stream, E->h1.zu,
+            e = launch_pdl(E->hplanes == 3 ? k_hm_zconv<3> : k_hm_zconv<2>, dim3(E->h1.nzu, 16), E->ni, 0, E->stream, E->h1.zu,
                            E->h1.pws, E->h1.ws, E->ni);
             E->launches++;
             if (e != cudaSuccess) return e;
