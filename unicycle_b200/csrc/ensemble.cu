@@ -686,9 +686,16 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
 constexpr int HSUB_KG3 = 8;                  // three planes: K-groups per fresh accumulator (64 entries)
 constexpr int HKG_STAGE = 8;                  // K-groups per stage (four K-steps of 16); see HTile::KG
 
-// tensor-memory columns of a hierarchical CTA: two accumulators of two NI-column
-// parts (every plane count), a power of two as tcgen05.alloc takes
-constexpr int hm_cols(int ni, int) { return 4 * ni; }
+// an accumulator's NI-column parts and a CTA's tensor-memory columns: two
+// accumulators, a power of two as tcgen05.alloc takes.  Three planes have three
+// parts where two CTAs per SM still have room for them (HTile::PARTS)
+constexpr int hm_parts(int ni, int pl) { return pl == 3 && ni <= 32 ? 3 : 2; }
+constexpr int hm_cols(int ni, int pl)
+{
+    int c = 32;
+    while (c < 2 * hm_parts(ni, pl) * ni) c *= 2;
+    return c;
+}
 // CTAs per SM: two when their tensor memory fits the SM's 512 columns; two
 // independent pipelines per SM hide the per-stage issue latency that bounds
 // one (measured: 20 % less time per launch)
@@ -718,15 +725,21 @@ struct HTile {
     static constexpr int SA = SA_FIT < 12 ? SA_FIT : 12;
     static constexpr int SMEM = SA * A_STAGE + SB * B_STAGE + 1024;   // + 1024 for the alignment
     static_assert(SA >= 2 && SB >= 1 && SMEM * CTAS <= 227 * 1024, "hierarchical contraction rings");
-    // an accumulator has two NI-column parts, which the drain adds.  Two
+    // an accumulator has two or three NI-column parts, which the drain adds.  Two
     // planes: one MMA of N = 2 NI per K-step reads the hi and lo planes of the
     // B K-groups together (consecutive 8-row groups): Ahi [Bhi; Blo], then Alo
     // Bhi into part 0.  Three planes: the six products of weight 2^-16 and above
-    // (the three left out are below 2^-24 of the value), Ahi [Bhi; Bmid] with
-    // N = 2 NI, then Ahi Blo, Amid Bhi, Amid Bmid and Alo Bhi into part 1, so
-    // that part 0 takes one tensor-core addition per K-step and part 1, 2^-8 of
-    // it, keeps the small products to 2^-31 of the value
-    static constexpr int ACC = 2 * NI;                     // columns of one accumulator
+    // (the three left out are below 2^-24 of the value).  In three parts, Ahi
+    // [Bhi; Bmid; Blo], Amid [Bhi; Bmid] into parts 1 and 2 and Alo Bhi into part
+    // 2; in two, Ahi [Bhi; Bmid], then Ahi Blo, Amid Bhi, Amid Bmid and Alo Bhi
+    // into part 1.  Either way part 0 takes one tensor-core addition per K-step,
+    // and the small products keep to 2^-31 of the value.  Shared memory bounds
+    // the K-step, and three MMAs read the operand three times where five do
+    // five times: 7,200 triangles x 32, both passes, 114 -> 101 us.  64 instances
+    // keep two parts: three leave half an SM's columns room for one accumulator
+    // (128 -> 137 us), a lone CTA with two of them 142
+    static constexpr int PARTS = hm_parts(NI, PL);
+    static constexpr int ACC = PARTS * NI;                 // columns of one accumulator
     // three planes: a fresh accumulator every SUB_KG K-groups (64 entries),
     // which the drain adds into FP32 register sums with round-to-nearest; the
     // tensor core's own accumulation truncates at each K-step, a bias that
@@ -737,6 +750,7 @@ struct HTile {
     static constexpr uint32_t TMEM_COLS = hm_cols(NI, PL);
     static constexpr uint32_t IDESC = Tile<NI, false, 1>::idesc(NI, true);
     static constexpr uint32_t IDESC2 = Tile<NI, false, 1>::idesc(2 * NI, true);
+    static constexpr uint32_t IDESC_P = Tile<NI, false, 1>::idesc(PARTS * NI, true);
 };
 
 struct HUnit {                  // one M-tile of one pass for one instance tile
@@ -988,8 +1002,12 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
                             const uint64_t ahi = cm_desc(a + ao, plane, 128u);
                             const uint64_t bhl = cm_desc(b + bo, T::B_KG, 128u);   // hi rows, then the other planes'
                             const uint32_t acc = (kg > k0 || j > 0) ? 1u : 0u;
-                            mma_bf16(d, ahi, bhl, T::IDESC2, acc);
-                            if (PL == 3) {
+                            mma_bf16(d, ahi, bhl, T::IDESC_P, acc);
+                            if (T::PARTS == 3) {
+                                mma_bf16(d + (uint32_t)NI, cm_desc(a + T::A_PLANE + ao, plane, 128u), bhl, T::IDESC2, 1u);
+                                mma_bf16(d + (uint32_t)(2 * NI), cm_desc(a + 2 * T::A_PLANE + ao, plane, 128u), bhl,
+                                         T::IDESC, 1u);
+                            } else if (PL == 3) {
                                 const uint32_t d1 = d + (uint32_t)NI;
                                 const uint64_t amid = cm_desc(a + T::A_PLANE + ao, plane, 128u);
                                 const uint64_t bmid = cm_desc(b + bo + NI * 16, T::B_KG, 128u);
@@ -1115,11 +1133,10 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
                         for (int i = 0; i < 16; i++) dst[(size_t)(c0 + i) * rows] = z[i];
                     }
                 };
-                const int span = T::SUB_KG ? T::SUB_KG : sg.kg1 - sg.kg0;
-                const int nsub = span > 0 ? (sg.kg1 - sg.kg0 + span - 1) / span : 0;
-                float sum[T::SUB_KG ? NI : 1];
+                const int nsub = (sg.kg1 - sg.kg0 + T::SUB_KG - 1) / T::SUB_KG;
+                float sum[NI];
 #pragma unroll
-                for (int c = 0; c < (T::SUB_KG ? NI : 1); c++) sum[c] = 0.0f;
+                for (int c = 0; c < NI; c++) sum[c] = 0.0f;
                 bool ok = true;
 #pragma unroll 1
                 for (int sub = 0; sub < nsub; sub++, tc++) {
@@ -1135,47 +1152,31 @@ __global__ void __launch_bounds__(224, hm_ctas(NI, PL)) k_hm_contract(const HUni
                     }
                     tc_fence_after();
                     const uint32_t tbase = tmem + (uint32_t)(buf * T::ACC) + ((uint32_t)(quarter * 32) << 16);
-                    // the sum of the accumulator's PL parts for 16 instances, the
-                    // small parts first
-                    auto load16 = [&](int c0, float *z) {
-                        uint32_t r[16], r2[16];
-                        tmem_ld16(tbase + (uint32_t)c0, r);
-                        tmem_ld16(tbase + (uint32_t)(c0 + NI), r2);
+                    // the sum of the accumulator's parts for 16 instances at a time,
+                    // the small parts first; the accumulator goes back once the last
+                    // 16 are in registers
 #pragma unroll
-                        for (int i = 0; i < 16; i++) z[i] = __uint_as_float(r[i]) + __uint_as_float(r2[i]);
-                    };
-                    if constexpr (T::SUB_KG > 0) {
-#pragma unroll
-                        for (int c0 = 0; c0 < NI; c0 += 16) {
-                            float z[16];
-                            load16(c0, z);
-#pragma unroll
-                            for (int i = 0; i < 16; i++) sum[c0 + i] += z[i];
+                    for (int c0 = 0; c0 < NI; c0 += 16) {
+                        uint32_t r[16], r2[16], r3[16];
+                        tmem_ld16_async(tbase + (uint32_t)c0, r);
+                        tmem_ld16_async(tbase + (uint32_t)(c0 + NI), r2);
+                        if (T::PARTS == 3) tmem_ld16_async(tbase + (uint32_t)(c0 + 2 * NI), r3);
+                        tmem_wait_ld();
+                        if (c0 + 16 >= NI) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(&acc_empty[buf]);
                         }
-                    } else if (sg.direct) {
 #pragma unroll
-                        for (int c0 = 0; c0 < NI; c0 += 16) {
-                            float z[16];
-                            load16(c0, z);
-                            put16(c0, z);
-                        }
-                    } else {
-#pragma unroll
-                        for (int c0 = 0; c0 < NI; c0 += 16) {
-                            float z[16];
-                            load16(c0, z);
-                            put16(c0, z);
-                        }
+                        for (int i = 0; i < 16; i++)
+                            sum[c0 + i] += __uint_as_float(r[i]) +
+                                           (T::PARTS == 3 ? __uint_as_float(r2[i]) + __uint_as_float(r3[i])
+                                                          : __uint_as_float(r2[i]));
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(&acc_empty[buf]);
                 }
                 if (!ok) break;
-                if constexpr (T::SUB_KG > 0) {
 #pragma unroll
-                    for (int c0 = 0; c0 < NI; c0 += 16) put16(c0, sum + c0);
-                }
+                for (int c0 = 0; c0 < NI; c0 += 16) put16(c0, sum + c0);
             }
         }
     }
@@ -2605,7 +2606,7 @@ int upload_hplan(ucg_ensemble *E, HPlanBufs &P, int ni, int pass)
         // (three planes, 64 instances), the copies write 6 KB of B and 0.75 KB a
         // row group.  (Weighed by bytes of K, g + 4, a CTA with a stack of two row
         // groups took 71,000 cycles beside the others' 25,000; both passes at
-        // 7,200 triangles x 64 148 -> 132 us, x 32 134 -> 115, two planes 84 -> 80.
+        // 7,200 triangles x 64 148 -> 132 us, x 32 134 -> 115 (100 with three parts), two planes 84 -> 80.
         // The line is flat: g + 16, 134 us, g + 200, 133.)
         w.push_back(u.g + 49);
     }
