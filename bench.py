@@ -878,7 +878,7 @@ def hmatrix_leg(args, local, sim, cfg, plain):
             "speedup_vs_plain_fp64_steps": steps / el / plain["value"],
             "sim_years_per_hour": (t_t - t_w) / YEAR / (el / 3600.0),
             "split": split,
-            "roofline": {"bound": "hbm", "kernel": "hierarchical product (k_hm_gather, k_hm_z, k_hm_rows, "
+            "roofline": {"bound": "hbm", "kernel": "hierarchical product (k_hm_gather, k_hm_rows, "
                                                    "k_hm_reduce)", "ms_per_launch": ms, "bytes_per_launch": alg,
                          "achieved": alg / (ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": alg / (ms / 1e3) / 1e9 / peak, "peak_source": peak_kind}}
@@ -1201,7 +1201,7 @@ def run_hmatrix(args, world, rank, local):
             "sim_years_per_hour": (t_t - t_w) / YEAR / (el / 3600.0),
             "hmatrix": {"build_seconds": build_s, "eta": args.hm_eta, "eps": args.hm_eps, "leaf": args.hm_leaf,
                         **{k: info[k] for k in ("n_dense", "n_lowrank", "max_rank", "bytes", "compression")}},
-            "roofline": {"bound": "hbm", "kernel": "hierarchical product (k_hm_gather, k_hm_z, k_hm_rows, "
+            "roofline": {"bound": "hbm", "kernel": "hierarchical product (k_hm_gather, k_hm_rows, "
                                                    "k_hm_reduce)", "ms_per_launch": ms, "bytes_per_launch": alg,
                          "achieved": alg / (ms / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                          "frac": alg / (ms / 1e3) / 1e9 / peak, "peak_source": peak_kind, "traffic": None},

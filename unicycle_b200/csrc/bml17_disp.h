@@ -5,10 +5,9 @@
 // (fortran/3d/src/strainvolume.f90:215-991).  The integrals are the published
 // closed forms and therefore have to be the same expressions; they are grouped
 // here by their recurring sub-terms (d1 = x1'-y1, d2 = x2'-y2, dm = x3-y3,
-// dp = x3+y3, r1, r2) and templated on the scalar type, so that evaluating them
-// on dual numbers seeded with the observation point gives the exact
-// displacement gradient (the reference evaluates hand-derived derivative
-// integrals instead, strainvolume.f90:1042-4640).
+// dp = x3+y3, r1, r2) and templated on the scalar type.  The observation points'
+// displacements use them; the strains have their own corner sums
+// (strainvolume.cuh).
 //
 // Requirements on T: arithmetic with T and double, and the free functions
 // sv_sqrt, sv_log, sv_atan, sv_atan2 and sv_val (value as double).
