@@ -38,7 +38,7 @@
 // 2^11), rows of 128 bytes in the 128-byte swizzle (16-byte chunk c of row r at
 // chunk c ^ (r mod 8)), with a power-of-two scale per row and per 128 x 64
 // block.  One 32 KB cp.async.bulk moves a whole k-block of a tile.  V is written
-// by the stage prologue directly in the same image form (instances are the rows
+// by the stage kernels directly in the same image form (instances are the rows
 // of the B operand), with a power-of-two scale per instance and k-block.  No
 // tensor map is needed and nothing is re-laid out per stage.
 //
@@ -55,17 +55,17 @@
 // packing), so geometries of uneven sizes balance across the SMs; every segment
 // is then cut to at most 256 k-blocks.
 // The partial sums of a tile are added in k order, in FP64, by the stage
-// epilogue kernel: results are deterministic for a given schedule and an
+// kernel behind: results are deterministic for a given schedule and an
 // instance's column never depends on the other instances.
 //
 // Every mbarrier wait is bounded (about 4 s of %globaltimer); one that runs out
 // records UCG_E_TIMEOUT, the CTA stops issuing, waits (bounded) for its copies
 // and MMAs in flight, frees its tensor memory and returns.
 //
-// One attempt of all instances is 6 x (prologue, contraction, epilogue) plus a
-// finish and a control kernel; the attempt is the body of a CUDA-graph while
-// loop whose condition the control kernel sets, so a whole run of many
-// attempts is ONE graph launch.
+// One attempt of all instances is a start kernel, 6 x (contraction, stage) and a
+// control kernel; the attempt is the body of a CUDA-graph while loop whose
+// condition the control kernel sets, so a whole run of many attempts is ONE
+// graph launch.
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
