@@ -363,7 +363,7 @@ def run_ours(args, world, rank, local, keep_sim=False, plain_steps=None):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": load_traffic("k_traction"),
                          "kernel": "k_traction (FP64 K.v + rate-state epilogue)" if args.precision == "fp64"
-                         else "k_traction<S,bf16> (hi plane x velocity increments + rate-state epilogue)",
+                         else "k_traction<bf16> (hi plane x velocity increments + rate-state epilogue)",
                          "ms_per_launch": ms_mv, "peak_source": peak_kind,
                          "bytes_per_launch": alg_bytes},
             "e2e": {"value": world * e2e_steps / e2e_elapsed, "unit": "steps/s",
@@ -616,8 +616,8 @@ def run_cfg3(args, world, rank, local):
                       "roofline": {"bound": "hbm", "ms_per_launch": ms_mv, "bytes_per_launch": alg,
                                    "achieved": alg / (ms_mv / 1e3) / 1e9, "peak": peak, "unit": "GB/s",
                                    "frac": alg / (ms_mv / 1e3) / 1e9 / peak, "peak_source": peak_kind,
-                                   "kernel": "k_traction<S,double>" if prec == "fp64" else
-                                   "k_traction<S,bf16> (hi plane x increments)"},
+                                   "kernel": "k_traction<double>" if prec == "fp64" else
+                                   "k_traction<__half> (fp16 plane x increments)"},
                       "clocks": clk.summary(), "final_state_finite": bool(np.all(np.isfinite(y)))}
     # split product error against FP64 on the preloaded state
     sim.set_precision("fp64")
@@ -920,10 +920,10 @@ def split_leg(args, local, sim, cfg, plain):
         ms_mv = sim.profile_traction(reps=10)   # a stage-2 launch: the increment plane (bf16) or the pair plane
         if form == "split_bf16":
             alg = 2.0 * (3 * n) * (2 * n) + 4.0 * 3 * n + 8.0 * (2 * n + 3 * n)
-            kern = "k_traction<S,__half> (fp16 increment plane x FP32 velocity increments, 8-term FP32 sums added in FP64)"
+            kern = "k_traction<__half> (fp16 increment plane x FP32 velocity increments, 8-term FP32 sums added in FP64)"
         else:
             alg = 4.0 * (3 * n) * (2 * n) + 4.0 * 3 * n + 8.0 * (2 * n + 3 * n)
-            kern = "k_traction<S,float> (FP32 pair plane, FP64 sums)"
+            kern = "k_traction<float> (FP32 pair plane, FP64 sums)"
         syh = (t_t - t_w) / YEAR / (el / 3600.0)
         out[form] = {"steps_per_s": steps / el, "ms_per_step": 1e3 * el / steps, "steps": steps,
                      "sim_years_per_hour": syh, "rejected_attempts": rej_t - rej_w,
