@@ -141,7 +141,8 @@ int ucg_keep_fp64(ucg_ctx *ctx, int keep);
    held (models beyond what a dense K fits in HBM).  The reference's MATLAB
    toolbox does this with the hmmvp library
    (matlab/+unicycle/+ode/+hmmvp/rateandstate.m:71-143).  Selected for the
-   traction product with ucg_set_precision(ctx, UCG_PREC_HMATRIX). */
+   traction product with ucg_set_precision(ctx, UCG_PREC_HMATRIX).  leaf: 4 or
+   more, with no upper limit (ensembles: at most 42). */
 int ucg_build_hmatrix(ucg_ctx *ctx, int okada_mode, double eta, double eps, int leaf);
 /* blocks stored dense (including low-rank candidates that failed their check)
    and low-rank, bytes stored, the largest rank, device time of the build */

@@ -2165,11 +2165,11 @@ int build_hgeom(ucg_ensemble *E, const ucg::HLayout &L, EnsGeomHost &g)
 {
     const int np = L.np, NL = L.n_leaves;
     std::vector<int> xkg0(NL + 1, 0), leaf_of_pos(np), kg_leaf;
+    if (3 * L.tree_leaf > BM)
+        return ebad(E, UCG_E_UNSUPPORTED,
+                    "hierarchical ensemble: row leaves of at most 42 patches (build the matrix with leaf <= 42)");
     for (int l = 0; l < NL; l++) {
         const int sz = L.leaf_e0[l + 1] - L.leaf_e0[l];
-        if (3 * sz > BM)
-            return ebad(E, UCG_E_UNSUPPORTED,
-                        "hierarchical ensemble: row leaves of at most 42 patches (build the matrix with leaf <= 42)");
         xkg0[l + 1] = xkg0[l] + (2 * sz + 7) / 8;
         for (int p = L.leaf_e0[l]; p < L.leaf_e0[l + 1]; p++) leaf_of_pos[p] = l;
         for (int q = xkg0[l]; q < xkg0[l + 1]; q++) kg_leaf.push_back(l);

@@ -97,6 +97,7 @@ struct HMat {
     int n_chunks = 0, n_dense_chunks = 0;
     int *leaf_e0_d = nullptr;            // row leaves: element ranges (permuted)
     int n_leaves = 0, max_leaf = 0;
+    int tree_leaf = 0;                   // patches of the cluster tree's largest leaf
     int max_cols = 0;                    // columns of the widest chunk
     double *z_d = nullptr;               // low-rank workspace
     long nz = 0;
@@ -541,6 +542,7 @@ __global__ void k_hm_gather(const int *__restrict__ perm, int np, const double *
 // 5 % for FP64 (fewer CTAs an SM).  Before these kernels a stage took 150 / 120 / 46.
 constexpr long HM_CHUNK_BYTES = 24 * 1024;
 constexpr int HM_THREADS = 128;   // at most; the launch takes a leaf's rows rounded up to warps
+constexpr int HM_LEAF = HM_THREADS / 3;   // patches of a row leaf: a thread a row
 constexpr int HM_ZR = 2, HM_ZU = 2;
 constexpr unsigned long long HM_TIMEOUT_NS = 4000000000ull;
 
@@ -885,9 +887,15 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     const size_t bound = std::min<size_t>((size_t)8 << 30, free_b / 4);   // of the build scratch
     std::vector<HBlock> blocks;
     block_tree(tb.nodes, 0, 0, eta, 0.4 * (double)bound / sizeof(double), blocks);
+    // row leaves of the product: the tree's, those of more patches than a CTA of the
+    // row kernel has threads for cut into equal parts
     std::vector<int> leaf_e0;
-    for (const Node &nd : tb.nodes)
-        if (nd.c[0] < 0) leaf_e0.push_back(nd.e0);
+    for (const Node &nd : tb.nodes) {
+        if (nd.c[0] >= 0) continue;
+        const int sz = nd.e1 - nd.e0, parts = (sz + HM_LEAF - 1) / HM_LEAF;
+        for (int k = 0; k < parts; k++) leaf_e0.push_back(nd.e0 + (int)((long)sz * k / parts));
+        h->tree_leaf = std::max(h->tree_leaf, sz);
+    }
     std::sort(leaf_e0.begin(), leaf_e0.end());
     h->n_leaves = (int)leaf_e0.size();
     leaf_e0.push_back(np);
@@ -1329,6 +1337,7 @@ bool hmatrix_layout(const ucg_ctx *c, HLayout *out)
     if (!h) return false;
     out->np = h->np;
     out->n_leaves = h->n_leaves;
+    out->tree_leaf = h->tree_leaf;
     out->perm = h->perm;
     out->leaf_e0 = h->leaf_e0_h;
     out->leaf_term0 = h->leaf_term0_h;

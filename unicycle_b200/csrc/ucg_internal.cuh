@@ -276,6 +276,7 @@ struct HLayout {
         int r0, m;               // first receiver element (permuted), rows
     };
     int np = 0, n_leaves = 0;
+    int tree_leaf = 0;           // patches of the cluster tree's largest leaf (the row leaves may be parts of one)
     std::vector<int> perm;       // permuted position -> element
     std::vector<int> leaf_e0;    // n_leaves + 1 element offsets of the row (and column) leaves
     std::vector<int> leaf_term0; // n_leaves + 1 offsets into terms
