@@ -1256,7 +1256,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
 // the chunks' partial row sums of H xp (split: of its FP32 planes), enqueued on
 // the context stream
 template <bool SPLIT>
-static void launch_products(ucg_ctx *c)
+static cudaError_t launch_products(ucg_ctx *c)
 {
     HMat *h = c->hm;
     const HmProduct P{h->lr_d, h->items_d, h->n_items, h->terms_d, h->chunks_d, h->n_dense_chunks, h->panel,
@@ -1264,18 +1264,18 @@ static void launch_products(ucg_ctx *c)
     const size_t smem = (SPLIT ? HM_CHUNK_BYTES / 2 : HM_CHUNK_BYTES) + sizeof(double) * h->max_cols;
     const int thr = (3 * h->max_leaf + 31) & ~31;
     const int zb = (int)((h->n_items * 32 + thr - 1) / thr), lowrank = h->n_chunks - h->n_dense_chunks;
-    launch_pdl(k_hm_rows<SPLIT, true>, dim3(zb + h->n_dense_chunks), dim3(thr), smem, c->stream, P, zb);
+    cudaError_t e = launch_pdl(k_hm_rows<SPLIT, true>, dim3(zb + h->n_dense_chunks), dim3(thr), smem, c->stream, P, zb);
     c->launches.count++;
-    if (lowrank > 0) {
-        launch_pdl(k_hm_rows<SPLIT, false>, dim3(lowrank), dim3(thr), smem, c->stream, P, 0);
+    if (e == cudaSuccess && lowrank > 0) {
+        e = launch_pdl(k_hm_rows<SPLIT, false>, dim3(lowrank), dim3(thr), smem, c->stream, P, 0);
         c->launches.count++;
     }
+    return e;
 }
 
-void hmatrix_products(ucg_ctx *c, bool split)
+cudaError_t hmatrix_products(ucg_ctx *c, bool split)
 {
-    if (split) launch_products<true>(c);
-    else launch_products<false>(c);
+    return split ? launch_products<true>(c) : launch_products<false>(c);
 }
 
 HmParts hmatrix_parts(const ucg_ctx *c)
@@ -1285,15 +1285,17 @@ HmParts hmatrix_parts(const ucg_ctx *c)
 }
 
 // t = H v (K's row order), enqueued on the context stream
-void hmatrix_apply(ucg_ctx *c, const double *v, double *t)
+cudaError_t hmatrix_apply(ucg_ctx *c, const double *v, double *t)
 {
     HMat *h = c->hm;
     k_hm_gather<<<(h->np + 255) / 256, 256, 0, c->stream>>>(h->perm_d, h->np, v, h->xp_d);
-    hmatrix_products(c, false);
+    const cudaError_t e = hmatrix_products(c, false);
+    if (e != cudaSuccess) return e;
     const int rows = 3 * h->max_leaf, gs = ((rows + 31) / 32) * 32, nthr = std::max(gs, (1024 / gs) * gs);
     k_hm_reduce<<<h->n_leaves, nthr, sizeof(double) * nthr, c->stream>>>(h->leaf_e0_d, h->leaf_chunk_d, h->perm_d,
                                                                          h->part_d, rows, t, gs);
     c->launches.count += 2;
+    return cudaGetLastError();
 }
 
 // hi / lo planes of the FP32 copies of the panels and of V (once; kept with the matrix)

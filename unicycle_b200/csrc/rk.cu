@@ -1225,80 +1225,76 @@ void rk_free(ucg_ctx *c)
 }
 
 template <class KT>
-static void launch_traction_t(ucg_ctx *c, int S, const StageArgs &a, const KT *K, long ldk, const float *scale)
+static cudaError_t launch_traction_t(ucg_ctx *c, int S, const StageArgs &a, const KT *K, long ldk, const float *scale)
 {
     const int ne = a.np + a.nvol, grid = ne < c->sms ? ne : c->sms;
     const size_t smem = tm_smem_bytes<KT>();
     auto kfn = k_traction<KT>;
-    cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    launch_pdl(kfn, dim3(grid), dim3(TM_THREADS), smem, c->stream, S, K, c->n, ldk, scale, a, c->ctl);
+    const cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(kfn, dim3(grid), dim3(TM_THREADS), smem, c->stream, S, K, c->n, ldk, scale, a, c->ctl);
 }
 
-static void launch_traction(ucg_ctx *c, int S, const StageArgs &a)
+static cudaError_t launch_traction(ucg_ctx *c, int S, const StageArgs &a)
 {
     if (S > 1 && c->precision == UCG_PREC_SPLIT_BF16 && rk_anchored(c) && c->Khi_plane) {
         // anchored stages multiply the increments by the fp16 plane
-        launch_traction_t<__half>(c, S, a, c->Khi_plane, c->ldk_split, c->Kscale);
+        return launch_traction_t<__half>(c, S, a, c->Khi_plane, c->ldk_split, c->Kscale);
     } else if ((c->precision == UCG_PREC_SPLIT_BF16 || c->precision == UCG_PREC_SPLIT_PAIR) && c->Ksp) {
-        launch_traction_t<float>(c, S, a, c->Ksp, c->ldk_split, c->Kscale);
-    } else {
-        launch_traction_t<double>(c, S, a, c->K, c->n, nullptr);
+        return launch_traction_t<float>(c, S, a, c->Ksp, c->ldk_split, c->Kscale);
     }
+    return launch_traction_t<double>(c, S, a, c->K, c->n, nullptr);
 }
 
-static void enqueue_stage(ucg_ctx *c, int S, int next)
+static cudaError_t enqueue_stage(ucg_ctx *c, int S, int next)
 {
     const StageArgs a = stage_args(c, S, next);
-    if (rk_hierarchical(c)) {
-        hmatrix_products(c, c->precision == UCG_PREC_HMATRIX_SPLIT);
-        const HmParts hp = hmatrix_parts(c);
-        launch_pdl(k_hm_stage, dim3(hp.n_leaves, (hp.rows_max + HS_ROWS - 1) / HS_ROWS), dim3(HS_THREADS), 0, c->stream,
-                   S, a, c->ctl, hp);
-    } else {
-        launch_traction(c, S, a);
-    }
     c->launches.count += 1;
+    if (!rk_hierarchical(c)) return launch_traction(c, S, a);
+    const cudaError_t e = hmatrix_products(c, c->precision == UCG_PREC_HMATRIX_SPLIT);
+    if (e != cudaSuccess) return e;
+    const HmParts hp = hmatrix_parts(c);
+    return launch_pdl(k_hm_stage, dim3(hp.n_leaves, (hp.rows_max + HS_ROWS - 1) / HS_ROWS), dim3(HS_THREADS), 0,
+                      c->stream, S, a, c->ctl, hp);
 }
 
 // source rates of the state y, before a run's first attempt
-static void enqueue_begin(ucg_ctx *c)
+cudaError_t rk_enqueue_begin(ucg_ctx *c)
 {
     const StageArgs a = stage_args(c, 1, 0);
     const int ne = a.np + a.nvol;
-    launch_pdl(k_begin, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl,
-               a.perm ? a.vn : c->st.v[1]);
     c->launches.count += 1;
+    return launch_pdl(k_begin, dim3((ne + 127) / 128), dim3(128), 0, c->stream, a, c->ctl,
+                      a.perm ? a.vn : c->st.v[1]);
 }
 
-static void enqueue_attempt_raw(ucg_ctx *c)
+static cudaError_t enqueue_attempt_raw(ucg_ctx *c)
 {
-    enqueue_stage(c, 1, 1);
+    cudaError_t e = enqueue_stage(c, 1, 1);
     // the recorder joins the attempt (and its graph) only while recording is on
-    if (c->rec_host.enabled) {
-        launch_pdl(k_record, dim3(c->sms), dim3(256), 0, c->stream, stage_args(c, 1, 0), c->ctl, c->rec);
+    if (e == cudaSuccess && c->rec_host.enabled) {
+        e = launch_pdl(k_record, dim3(c->sms), dim3(256), 0, c->stream, stage_args(c, 1, 0), c->ctl, c->rec);
         c->launches.count += 1;
     }
-    enqueue_stage(c, 2, 1);
-    enqueue_stage(c, 3, 1);
-    enqueue_stage(c, 4, 1);
-    enqueue_stage(c, 5, 1);
-    enqueue_stage(c, 6, 1);
+    for (int s = 2; s <= 6 && e == cudaSuccess; s++) e = enqueue_stage(c, s, 1);
+    return e;
 }
 
-void rk_enqueue_begin(ucg_ctx *c) { enqueue_begin(c); }
-
-void rk_enqueue_attempt(ucg_ctx *c)
+cudaError_t rk_enqueue_attempt(ucg_ctx *c)
 {
     if (!c->attempt_graph || c->graph_precision != c->precision) {
         if (c->attempt_graph) cudaGraphExecDestroy(c->attempt_graph);
         c->attempt_graph = nullptr;
         cudaGraph_t g;
         long before = c->launches.count;
+        cudaError_t refused = cudaSuccess;
         if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-            enqueue_attempt_raw(c);
+            refused = enqueue_attempt_raw(c);
             c->graph_launches = c->launches.count - before;
             if (cudaStreamEndCapture(c->stream, &g) == cudaSuccess) {
-                if (cudaGraphInstantiate(&c->attempt_graph, g, 0) != cudaSuccess) c->attempt_graph = nullptr;
+                // (an attempt without one of its kernels is no attempt)
+                if (refused != cudaSuccess || cudaGraphInstantiate(&c->attempt_graph, g, 0) != cudaSuccess)
+                    c->attempt_graph = nullptr;
                 cudaGraphDestroy(g);
             }
         }
@@ -1306,19 +1302,17 @@ void rk_enqueue_attempt(ucg_ctx *c)
         c->graph_precision = c->precision;
         cudaGetLastError();
     }
-    if (c->attempt_graph) {
-        cudaGraphLaunch(c->attempt_graph, c->stream);
-        c->launches.count += c->graph_launches;
-    } else {
-        enqueue_attempt_raw(c);
-    }
+    // without a graph the attempt is launched kernel by kernel, and says what refuses it
+    if (!c->attempt_graph) return enqueue_attempt_raw(c);
+    c->launches.count += c->graph_launches;
+    return cudaGraphLaunch(c->attempt_graph, c->stream);
 }
 
-void rk_enqueue_commit(ucg_ctx *c)
+cudaError_t rk_enqueue_commit(ucg_ctx *c)
 {
-    StageArgs a = stage_args(c, 1, 0);
-    launch_pdl(k_commit, dim3((unsigned)((c->state_len + 255) / 256)), dim3(256), 0, c->stream, a, c->ctl);
+    const StageArgs a = stage_args(c, 1, 0);
     c->launches.count += 1;
+    return launch_pdl(k_commit, dim3((unsigned)((c->state_len + 255) / 256)), dim3(256), 0, c->stream, a, c->ctl);
 }
 
 // Mean device time of the stage-2 traction launch (the dominant kernel), timed
@@ -1338,9 +1332,8 @@ int rk_profile_traction(ucg_ctx *c, int reps, double *ms)
     UCG_CUDA(cudaEventCreate(&e0));
     UCG_CUDA(cudaEventCreate(&e1));
     UCG_CUDA(cudaEventRecord(e0, c->stream));
-    for (int r = 0; r < reps; r++) {
-        launch_traction(c, 2, a);
-    }
+    cudaError_t le = cudaSuccess;
+    for (int r = 0; r < reps && le == cudaSuccess; r++) le = launch_traction(c, 2, a);
     c->launches.count += reps;
     UCG_CUDA(cudaEventRecord(e1, c->stream));
     UCG_CUDA(cudaEventSynchronize(e1));
@@ -1352,7 +1345,7 @@ int rk_profile_traction(ucg_ctx *c, int reps, double *ms)
     *h = saved;
     UCG_CUDA(cudaMemcpyAsync(c->ctl, h, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
     UCG_CUDA(cudaStreamSynchronize(c->stream));
-    return UCG_OK;
+    return le == cudaSuccess ? UCG_OK : cuda_fail(c, le, "traction launch");
 }
 
 // A coseismic perturbation of the state: slip (2 per patch) and eigenstrain
@@ -1399,7 +1392,7 @@ int rk_perturb(ucg_ctx *c, const double *u)
         k_perturb<<<blocks, 256, 0, c->stream>>>(c->K, c->m, c->n, c->nr + c->nt, c->pert, c->st.y);
     } else {
         double *t = hmatrix_t(c);
-        hmatrix_apply(c, c->pert, t);
+        UCG_CUDA(hmatrix_apply(c, c->pert, t));
         k_perturb_t<<<blocks, 256, 0, c->stream>>>(c->m, c->n, c->nr + c->nt, t, c->pert, c->st.y);
     }
     c->launches.count++;
@@ -1422,8 +1415,8 @@ int rk_odefun(ucg_ctx *c)
     h->nonfinite = 0;
     h->ticket = 0;
     UCG_CUDA(cudaMemcpyAsync(c->ctl, h, sizeof(Ctl), cudaMemcpyHostToDevice, c->stream));
-    enqueue_begin(c);
-    enqueue_stage(c, 1, 0);
+    UCG_CUDA(rk_enqueue_begin(c));
+    UCG_CUDA(enqueue_stage(c, 1, 0));
     UCG_CUDA(cudaGetLastError());
     UCG_CUDA(cudaMemcpyAsync(h, c->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, c->stream));
     UCG_CUDA(cudaStreamSynchronize(c->stream));

@@ -678,8 +678,7 @@ int ucg_hmatrix_matvec(ucg_ctx *c, const double *x, double *y)
     cudaError_t e = cudaMemcpyAsync(xd, x, sizeof(double) * c->n, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
         double *t = hmatrix_t(c);
-        hmatrix_apply(c, xd, t);
-        e = cudaGetLastError();
+        e = hmatrix_apply(c, xd, t);
         if (e == cudaSuccess) e = cudaMemcpyAsync(y, t, sizeof(double) * c->m, cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     }
@@ -700,9 +699,9 @@ int ucg_hmatrix_profile(ucg_ctx *c, int reps, double *ms)
     UCG_CUDA(cudaEventCreate(&e0));
     UCG_CUDA(cudaEventCreate(&e1));
     double *t = hmatrix_t(c);
-    hmatrix_apply(c, xd, t);   // warm-up
+    cudaError_t le = hmatrix_apply(c, xd, t);   // warm-up
     UCG_CUDA(cudaEventRecord(e0, c->stream));
-    for (int r = 0; r < reps; r++) hmatrix_apply(c, xd, t);
+    for (int r = 0; r < reps && le == cudaSuccess; r++) le = hmatrix_apply(c, xd, t);
     UCG_CUDA(cudaEventRecord(e1, c->stream));
     UCG_CUDA(cudaEventSynchronize(e1));
     float f = 0.0f;
@@ -711,7 +710,7 @@ int ucg_hmatrix_profile(ucg_ctx *c, int reps, double *ms)
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFree(xd);
-    return UCG_OK;
+    return le == cudaSuccess ? UCG_OK : cuda_fail(c, le, "ucg_hmatrix_profile");
 }
 
 int ucg_odefun(ucg_ctx *c, double t, const double *y, double *dydt, double *vmax)
@@ -754,10 +753,10 @@ int ucg_set_tolerance(ucg_ctx *c, double epsilon, double max_step)
 static int drive(ucg_ctx *c, int batch, bool out = false)
 {
     const size_t bytes = sizeof(double) * c->state_len;
-    rk_enqueue_begin(c);
+    UCG_CUDA(rk_enqueue_begin(c));
     for (;;) {
-        for (int i = 0; i < batch; i++) rk_enqueue_attempt(c);
-        rk_enqueue_commit(c);
+        for (int i = 0; i < batch; i++) UCG_CUDA(rk_enqueue_attempt(c));
+        UCG_CUDA(rk_enqueue_commit(c));
         if (out) {
             UCG_CUDA(cudaMemcpyAsync(c->pin, c->st.y, bytes, cudaMemcpyDeviceToHost, c->stream));
             UCG_CUDA(cudaMemcpyAsync(c->pin + c->state_len, c->st.k[0], bytes, cudaMemcpyDeviceToHost, c->stream));

@@ -230,9 +230,10 @@ void rk_free(ucg_ctx *c);
 int rk_odefun(ucg_ctx *c);                  // k[0] = f(y) on device, sets vmax
 int rk_test_wait_timeout(ucg_ctx *c, unsigned long long wait_ns, int hold);
 int rk_profile_traction(ucg_ctx *c, int reps, double *ms);
-void rk_enqueue_begin(ucg_ctx *c);          // source rates of the state, before a run's first attempt
-void rk_enqueue_attempt(ucg_ctx *c);        // one Cash-Karp attempt + control
-void rk_enqueue_commit(ucg_ctx *c);         // copy a pending candidate into y
+// these return the first launch that was refused
+cudaError_t rk_enqueue_begin(ucg_ctx *c);   // source rates of the state, before a run's first attempt
+cudaError_t rk_enqueue_attempt(ucg_ctx *c); // one Cash-Karp attempt + control
+cudaError_t rk_enqueue_commit(ucg_ctx *c);  // copy a pending candidate into y
 bool rk_anchored(const ucg_ctx *c);         // stages contract increments over the stage-1 anchor
 int rk_perturb(ucg_ctx *c, const double *u); // y += slip/strain u and the stress change K u (host u)
 void rk_drop_graph(ucg_ctx *c);             // before freeing anything the attempt graph reads
@@ -241,7 +242,7 @@ void split_bf16_free(ucg_ctx *c);
 // hmatrix.cu
 int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf);
 void hmatrix_free(ucg_ctx *c);
-void hmatrix_apply(ucg_ctx *c, const double *v, double *t);   // t = H v, K's row order
+cudaError_t hmatrix_apply(ucg_ctx *c, const double *v, double *t);   // t = H v, K's row order
 int hmatrix_split_build(ucg_ctx *c);                          // bf16 hi / lo copies (UCG_PREC_HMATRIX_SPLIT)
 // The product inside an attempt: partial row sums of H xp per chunk of a row leaf
 // (split: on the FP32 planes), added up by the stage kernel (rk.cu), which also
@@ -254,7 +255,7 @@ struct HmParts {
     double *xp;
     int rows_max, n_leaves;
 };
-void hmatrix_products(ucg_ctx *c, bool split);
+cudaError_t hmatrix_products(ucg_ctx *c, bool split);
 HmParts hmatrix_parts(const ucg_ctx *c);
 double *hmatrix_t(ucg_ctx *c);                                 // the product's output buffer
 void hmatrix_info(const ucg_ctx *c, long *n_dense, long *n_lowrank, long *n_fallback, size_t *bytes,
