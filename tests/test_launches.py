@@ -28,3 +28,12 @@ def test_every_launch_status_is_used():
             line = text[:m.end()].count("\n") + 1
             raise AssertionError(f"{name}:{line}: the launch's status is dropped")
     assert found > 20
+
+
+def test_no_read_only_loads_in_the_stage_kernels():
+    """The launches of rk.cu overlap: one starts while the one in front still writes
+    the rates and partial sums that it reads after its wait.  A load on the read-only
+    path may return an older value."""
+    text = dict(_sources())["rk.cu"]
+    assert "launch_pdl(" in text
+    assert not re.findall(r"__ldg\s*\(|ld\.global\.nc", text)

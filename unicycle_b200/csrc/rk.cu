@@ -660,13 +660,15 @@ __device__ __forceinline__ void tm_load_v<double>(const double *v, long c, long 
     vr.x = *reinterpret_cast<const double2 *>(v + c);
 }
 // c is a multiple of the values per thread (4 or 8), so away from the ragged
-// end the thread's values are 16-byte aligned pairs
+// end the thread's values are 16-byte aligned pairs.  Plain loads: the launch in
+// front may still be writing v when this one starts, and the read-only path asks for
+// memory that nobody writes while the kernel runs (same time)
 template <>
 __device__ __forceinline__ void tm_load_v<float>(const double *v, long c, long n, TmV<float> &vr)
 {
     if (c + 4 <= n) {
-        const double2 a = __ldg(reinterpret_cast<const double2 *>(v + c));
-        const double2 b = __ldg(reinterpret_cast<const double2 *>(v + c + 2));
+        const double2 a = *reinterpret_cast<const double2 *>(v + c);
+        const double2 b = *reinterpret_cast<const double2 *>(v + c + 2);
         vr.x[0] = a.x; vr.x[1] = a.y; vr.x[2] = b.x; vr.x[3] = b.y;
         return;
     }
@@ -685,7 +687,7 @@ __device__ __forceinline__ void tm_load_raw<__half>(const double *v, long c, lon
     if (c + 8 <= n) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            const double2 a = __ldg(reinterpret_cast<const double2 *>(v + c + 2 * q));
+            const double2 a = *reinterpret_cast<const double2 *>(v + c + 2 * q);
             raw.x[2 * q] = a.x;
             raw.x[2 * q + 1] = a.y;
         }
