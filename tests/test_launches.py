@@ -37,3 +37,23 @@ def test_no_read_only_loads_in_the_stage_kernels():
     text = dict(_sources())["rk.cu"]
     assert "launch_pdl(" in text
     assert not re.findall(r"__ldg\s*\(|ld\.global\.nc", text)
+
+
+def test_overlapping_kernels_promise_read_only_memory_for_tables_alone():
+    """Kernels launched programmatically start while the one in front runs.  What they
+    read through `const ... __restrict__` (which lets the compiler take the read-only
+    path) or __ldg has to be laid out once: K, its scales, plans and index tables."""
+    tables = {"K", "scale", "tiles", "segs", "cta_seg", "units", "zu", "pws", "A"}
+    kernels, text = set(), ""
+    for _, t in _sources():
+        kernels |= {k for m in re.finditer(r"\blaunch_pdl\(([^;]*)", t) for k in re.findall(r"\bk_\w+", m.group(1))}
+        text += t
+    kernels |= {"k_traction"}    # launched through a variable
+    assert len(kernels) == 12
+    for k in kernels:
+        m = re.search(rf"__global__[^;{{}}]*?\b{k}\s*\(([^{{}}]*?)\)\s*{{", text)
+        assert m, k
+        named = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s+(\w+)", m.group(1)))
+        assert named <= tables, (k, named - tables)
+    ens = dict(_sources())["ensemble.cu"]
+    assert set(re.findall(r"__ldg\(\s*(\w+)", ens)) <= {"ubidx"}

@@ -575,7 +575,8 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
             // k-block ahead and multiplied only when used (a product formed at
             // the load would wait out the L2 latency in every k-block once the
             // drain is the busy side), the lane's product broadcast to the warp
-            // by shuffles
+            // by shuffles.  (V's scales by plain loads: the kernel in front may still
+            // be writing them when this one starts)
             constexpr int NL = (NC + 31) / 32;       // instance columns per lane
             const float *ksu = u == 0 ? tl.ks : tl.ks1;
             float nk = 0.0f, nv[NL];
@@ -583,7 +584,7 @@ __global__ void __launch_bounds__(320, 1) k_bf16x3_contract(const GemmTile *__re
                 nk = ksu[k];
 #pragma unroll
                 for (int j = 0; j < NL; j++)
-                    nv[j] = (32 * j + lane < NC) ? __ldg(tl.vs + (size_t)k * NI + cbase + 32 * j + lane) : 0.0f;
+                    nv[j] = (32 * j + lane < NC) ? tl.vs[(size_t)k * NI + cbase + 32 * j + lane] : 0.0f;
             };
 #pragma unroll
             for (int j = 0; j < NL; j++) nv[j] = 0.0f;
@@ -1273,7 +1274,7 @@ constexpr int HZ_AHEAD = 8;
 
 template <int PL>
 __global__ void __launch_bounds__(128) k_hm_zconv(const HZUnit *__restrict__ zu, const long *__restrict__ pws,
-                                                  const float *__restrict__ ws, int ni)
+                                                  const float *ws, int ni)
 {
     const HZUnit U = zu[blockIdx.x];
     const int grp = blockIdx.y, i = threadIdx.x;
