@@ -57,3 +57,14 @@ def test_overlapping_kernels_promise_read_only_memory_for_tables_alone():
         assert named <= tables, (k, named - tables)
     ens = dict(_sources())["ensemble.cu"]
     assert set(re.findall(r"__ldg\(\s*(\w+)", ens)) <= {"ubidx"}
+
+
+def test_traction_kernel_reads_the_control_block_once():
+    """The warps of a CTA wait for one another at named barriers, without a limit: they
+    have to agree on whether there is anything to do, so one thread reads the control
+    block for all of them (another CTA may change it between two reads)."""
+    text = dict(_sources())["rk.cu"]
+    m = re.search(r"__global__[^;{}]*?\bk_traction\b.*?\n}\n", text, flags=re.S)
+    body = m.group()
+    assert not re.findall(r"\bctl_live\(|ctl->(?:active|need_stage1|wait_ns|h)\b", body)
+    assert body.count("tm_head(") == 2 and "&head_read" in body

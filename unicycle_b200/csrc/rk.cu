@@ -843,6 +843,27 @@ constexpr int TM_THREADS = (MV_WARPS + 2) * 32;   // consumers, producer, epilog
 __device__ __forceinline__ void bar_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(MV_WARPS * 32 + 32) : "memory"); }
 __device__ __forceinline__ void bar_wait(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(MV_WARPS * 32 + 32) : "memory"); }
 
+// What a CTA of k_traction takes from the control block, read once and handed to all
+// its warps: another CTA may end the run (a wait that ran out) between two reads, and
+// a warp that left by itself would keep the others waiting at the barriers above.  The
+// consumers and the epilogue warp meet at a barrier, the producer's one lane waits for
+// `read` (a producer warp kept whole for the barrier took 1.5 % of 8 steps of 7,200
+// triangles, split pair: 10.13 ms against 9.95).
+struct TmHead {
+    double h;
+    unsigned long long wait_ns;
+    int live, first;       // first: the product is wanted (stage 1 of a rejected attempt repeats nothing)
+};
+__device__ __forceinline__ TmHead tm_head(int S, const Ctl *ctl, TmHead &sh, uint64_t *read, bool reader)
+{
+    if (reader) {
+        sh = TmHead{ctl->h, ctl->wait_ns, ctl_live(ctl), S > 1 || ctl->need_stage1};
+        mbar_arrive(read);
+    }
+    asm volatile("bar.sync 5, %0;" ::"n"(MV_WARPS * 32 + 32) : "memory");
+    return sh;
+}
+
 // The stage number is an argument: the six launches of an attempt run the same
 // code, which then stays in the instruction caches.
 template <class KT>
@@ -854,9 +875,10 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
     constexpr int CH = Tr::CH, PER = Tr::PER, ROWS = Tr::ROWS, stages = Tr::STAGES;
     extern __shared__ __align__(128) unsigned char tm_smem[];
     KT *stage = reinterpret_cast<KT *>(tm_smem);
-    __shared__ __align__(8) uint64_t full[Tr::STAGES], empty[Tr::STAGES];
+    __shared__ __align__(8) uint64_t full[Tr::STAGES], empty[Tr::STAGES], head_read;
     __shared__ double red[2][MV_WARPS][ROWS];
     __shared__ int abort_flag;
+    __shared__ TmHead head;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // the next launch may come as soon as there is room: before its own wait it only
     // reads K and the friction, which no launch changes
@@ -869,6 +891,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], MV_WARPS);
         }
+        mbar_init(&head_read, 1);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -900,7 +923,8 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
         if (!hold)
             while (item < total && item < stages) issue();
         pdl_wait();
-        if (!hold && ctl_live(ctl) && !(S == 1 && !ctl->need_stage1)) {
+        const bool go = mbar_wait(&head_read, 0, nullptr) && head.live && head.first;
+        if (!hold && go) {
             while (item < total && !*(volatile int *)&abort_flag) {
                 if (!mbar_wait(&empty[s], ph ^ 1, &abort_flag)) {
                     abort_flag = 1;
@@ -929,9 +953,10 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
                 fr = patch_friction(a, e0 + (lane >> 3), lane & 7, (lane >> 3) < nel && (lane & 7) < 7);
         }
         pdl_wait();
-        if (!ctl_live(ctl)) return;
-        const double h = ctl->h;
-        const bool first = S > 1 || ctl->need_stage1;
+        const TmHead hd = tm_head(S, ctl, head, &head_read, lane == 0);
+        if (!hd.live) return;
+        const double h = hd.h;
+        const bool first = hd.first;
         double mx = 0.0;
         bool bad = false;
         for (int b = 0; b < nblk; b++) {
@@ -998,14 +1023,14 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
         return;
     }
 
-    // consumers.  The first v values are asked for together with the control block.
+    // consumers.  The first v values are on their way while the control block is read.
     const int t = threadIdx.x, cl = PER * t;
     pdl_wait();
     TmVRaw<KT> vn;
     if (cl < n) tm_load_raw<KT>(a.v, cl, n, vn);
-    const unsigned long long wait_ns = ctl->wait_ns;   // (looked at only where a wait has to be timed)
-    if (!ctl_live(ctl)) return;
-    if (S == 1 && !ctl->need_stage1) return;
+    const TmHead hd = tm_head(S, ctl, head, &head_read, false);
+    if (!hd.live || !hd.first) return;
+    const unsigned long long wait_ns = hd.wait_ns;
     int s = 0, ph = 0;
     for (int b = 0; b < nblk; b++) {
         long row0;
