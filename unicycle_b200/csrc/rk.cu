@@ -82,6 +82,8 @@ struct StageArgs {
 };
 
 __device__ __forceinline__ bool ctl_live(const Ctl *c) { return c->active && c->status == 0; }
+// the same while the launch in front may still change it: a hint, nothing to decide by
+__device__ __forceinline__ bool ctl_hint(const Ctl *c) { return *(const volatile int *)&c->active != 0; }
 
 // Programmatic dependent launch.  The kernels of an attempt are launched with
 // programmatic stream serialization: each may be scheduled while its
@@ -927,7 +929,7 @@ __global__ void __launch_bounds__(TM_THREADS, 1) k_traction(int S, const KT *__r
         const bool hold = blockIdx.x == 0 && *(volatile int *)&ctl->test_hold;
         if (!hold && total > 0) {
             issue();
-            if (*(volatile int *)&ctl->active)
+            if (ctl_hint(ctl))
                 while (item < total && item < stages) issue();
         }
         pdl_wait();
