@@ -130,11 +130,20 @@ __device__ __forceinline__ double stage_comb(int S, const LaneState &st, double 
 
 // x / d where rd = 1 / d is at hand before x: the quotient's residual corrects it
 // once (Markstein, IBM J. Res. Dev. 34, 1990), which rounds like the division for
-// normal quotients; three dependent operations instead of a division's sequence
+// normal quotients; three dependent operations instead of a division's sequence.
+// (x, d and the quotient finite)
 __device__ __forceinline__ double div_by(double x, double d, double rd)
 {
     const double q = x * rd;
     return fma(fma(-d, q, x), rd, q);
+}
+
+// where one of them may be infinite the correction is NaN, and the product x rd (or a
+// chain of them) is already the quotient (an infinite L is a fault without state
+// evolution)
+__device__ __forceinline__ double or_product(double quotient, double product)
+{
+    return isnan(quotient) ? product : quotient;
 }
 
 constexpr double INV_LG10 = 0.434294481903251827651128918916605082;   // 1 / ln 10
@@ -272,7 +281,8 @@ __device__ __forceinline__ PatchTerms patch_terms(int S, Ctl *ctl, const PatchFr
     patch_slip(ts, td, lv, p.vel, p.cr, p.sr);
     p.den = f.a * f.sig + f.eta * p.vel;
     p.rden = 1.0 / p.den;
-    p.dth = div_by(exp(-th * LG10) - div_by(p.vel, f.L, f.iL), LG10, INV_LG10);
+    const double rate = exp(-th * LG10) - or_product(div_by(p.vel, f.L, f.iL), p.vel * f.iL);
+    p.dth = or_product(div_by(rate, LG10, INV_LG10), rate * INV_LG10);
     p.q = f.b * f.sig * p.dth * LG10;
     p.ev = f.eta * p.vel;
     p.vpl = f.vpl;
@@ -288,7 +298,8 @@ __device__ __forceinline__ void patch_finish(int S, const StageArgs &a, Ctl *ctl
                                              const LaneState &st, const PatchTerms &p, double t0, double t1,
                                              double t2, double &mx, bool &bad)
 {
-    const double dv = div_by(div_by(t0 * p.cr + t1 * p.sr - p.q, p.den, p.rden), LG10, INV_LG10);
+    const double dtau = t0 * p.cr + t1 * p.sr - p.q;
+    const double dv = or_product(div_by(div_by(dtau, p.den, p.rden), LG10, INV_LG10), dtau * p.rden * INV_LG10);
     const double corr = p.ev * dv * LG10;
     const double vs = p.vel * (c == 0 ? p.cr : p.sr);
     const double ks = c < 2 ? vs : c == 2 ? t0 - corr * p.cr : c == 3 ? t1 - corr * p.sr : c == 4 ? t2
