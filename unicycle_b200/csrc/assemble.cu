@@ -659,6 +659,7 @@ int assemble_matrix(ucg_ctx *c, int okada_mode)
     const long m = 3L * np + 6L * c->nv;
     if (ne == 0) return UCG_E_BADARG;
     UCG_CUDA(cudaSetDevice(c->device));
+    c->assembled = false;   // until all of K is
     if (c->K && (c->n != n || c->m != m)) {
         cudaFree(c->K);
         c->K = nullptr;

@@ -854,7 +854,8 @@ void hmatrix_free(ucg_ctx *c)
     c->hm = nullptr;
 }
 
-int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
+// temp_allocs: storage of the build alone, the caller's to free when it fails
+static int build_matrix(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf, std::vector<void *> &temp_allocs)
 {
     hmatrix_free(c);
     const int np = c->nr + c->nt;
@@ -934,7 +935,6 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     const size_t CHUNK = (size_t)256 << 20;
     size_t chunk_left[2] = {0, 0};
     char *chunk_ptr[2] = {nullptr, nullptr};
-    std::vector<void *> temp_allocs;
     auto store = [&](int pool, size_t bytes, double **out) -> int {
         bytes = (bytes + 255) & ~(size_t)255;
         if (bytes > chunk_left[pool]) {
@@ -1204,6 +1204,7 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
             cudaFree(pk_d);
         }
         for (void *p : temp_allocs) cudaFree(p);
+        temp_allocs.clear();
         for (HLowRank &b : lr) b.U = nullptr;   // the product reads U from the panels
         for (HLeafTerm &T : terms) T.A = nullptr;
         h->terms_h = terms;
@@ -1251,6 +1252,20 @@ int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
     return UCG_OK;
+}
+
+// A build that fails leaves no matrix: its parts would be taken for one.
+int hmatrix_build(ucg_ctx *c, int okada_mode, double eta, double eps, int leaf)
+{
+    std::vector<void *> temp_allocs;
+    int rc = build_matrix(c, okada_mode, eta, eps, leaf, temp_allocs);
+    // the split planes belong to the matrix that a run in the split form reads
+    if (!rc && c->precision == UCG_PREC_HMATRIX_SPLIT) rc = hmatrix_split_build(c);
+    if (!rc) return UCG_OK;
+    cudaStreamSynchronize(c->stream);
+    for (void *p : temp_allocs) cudaFree(p);
+    hmatrix_free(c);
+    return rc;
 }
 
 // the chunks' partial row sums of H xp (split: of its FP32 planes), enqueued on

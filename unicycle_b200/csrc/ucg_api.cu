@@ -916,9 +916,10 @@ int ucg_run(ucg_ctx *c, double t_end, long max_steps, long *steps)
 {
     if (!c || max_steps < 0) return UCG_E_BADARG;
     if (!c->state_ready) return set_err(c, UCG_E_STATE, "call ucg_set_state first");
-    UCG_CUDA(cudaSetDevice(c->device));
-    int rc = pull_ctl(c);
+    int rc = ensure_state(c);   // the matrix may have gone since
     if (rc) return rc;
+    UCG_CUDA(cudaSetDevice(c->device));
+    if ((rc = pull_ctl(c))) return rc;
     Ctl *h = c->ctl_host;
     const long acc0 = h->accepted;
     if (max_steps == 0 || h->time >= t_end) {
@@ -1006,6 +1007,8 @@ int ucg_profile_traction(ucg_ctx *c, int reps, double *ms)
 {
     if (!c || reps <= 0 || !ms) return UCG_E_BADARG;
     if (!c->state_ready) return set_err(c, UCG_E_STATE, "no device state");
+    const bool split = (c->precision == UCG_PREC_SPLIT_BF16 || c->precision == UCG_PREC_SPLIT_PAIR) && c->Ksp;
+    if (!split && !c->K) return set_err(c, UCG_E_STATE, "no dense matrix");
     UCG_CUDA(cudaSetDevice(c->device));
     return rk_profile_traction(c, reps, ms);
 }
