@@ -109,7 +109,10 @@ int ucg_set_rheology(ucg_ctx *ctx, const double *e_bg, const double *gammadot0m,
 
 /* Assemble the stress-interaction matrix on the device, FP64, one thread per
    (receiver, source) pair.  Replaces buildG (fortran/3d/src/greens.f90:73-275).
-   okada_mode: UCG_OKADA_*. */
+   okada_mode: UCG_OKADA_*.
+   K, and workspaces of some 1.2 KB a triangle and at most 96 MB, stay with the
+   context until it is destroyed, so that an assembly after the first allocates
+   nothing.  A call that fails leaves no matrix. */
 int ucg_assemble(ucg_ctx *ctx, int okada_mode);
 
 /* Device time (ms) of the last ucg_assemble per source family: the columns of
@@ -142,7 +145,8 @@ int ucg_keep_fp64(ucg_ctx *ctx, int keep);
    toolbox does this with the hmmvp library
    (matlab/+unicycle/+ode/+hmmvp/rateandstate.m:71-143).  Selected for the
    traction product with ucg_set_precision(ctx, UCG_PREC_HMATRIX).  leaf: 4 or
-   more, with no upper limit (ensembles: at most 42). */
+   more, with no upper limit (ensembles: at most 42).  Building keeps the
+   assembly workspaces of ucg_assemble with the context. */
 int ucg_build_hmatrix(ucg_ctx *ctx, int okada_mode, double eta, double eps, int leaf);
 /* blocks stored dense (including low-rank candidates that failed their check)
    and low-rank, bytes stored, the largest rank, device time of the build */

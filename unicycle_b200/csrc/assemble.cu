@@ -11,9 +11,10 @@
 // One thread per (receiver, source) pair computes every unit component of the
 // source at once, sharing the pair geometry, and writes them as contiguous
 // columns: a warp covers 32 consecutive sources of one receiver, so each of its
-// row stores is one coalesced 512-byte (patches) segment.  Per-source constants
-// (frames, the REAL*4-rounded DC3D inputs, the Nikkhoo-Walter records) are built
-// once on the host and read through the read-only path.
+// row stores is one coalesced 512-byte (patches) segment.  Per-source constants are
+// formed once and read through the read-only path: the rectangles' (frames, the
+// REAL*4-rounded DC3D inputs) and the cuboids' on the host, the triangles' records and
+// their mesh edges' by a kernel from the vertices.
 #include <algorithm>
 #include <cmath>
 #include <cstring>

@@ -24,16 +24,21 @@
 //              vector; a block that fails the check, or whose factors would not
 //              be smaller, is kept dense.
 //   storage    FP64.  V is stored rank-major (k x n); the rows of U and of the
-//              dense blocks are repacked into panels, one per row leaf and chunk
-//              of at most 16 KB, each a column-major (rows x columns) slab.
-//   product    t = H v: v is gathered into the permuted order (every block's
-//              columns become a contiguous slice); z_b = V_b^T v_sigma for every
-//              low-rank block (one warp per rank vector); one CTA per chunk
-//              copies its panel into shared memory with one bulk copy and one
-//              thread per row multiplies it by the matching slices of v or z;
-//              a last kernel adds a leaf's chunks in order and writes K's row
-//              order.  Every stored byte is read once per product and the
-//              summation order is fixed (deterministic).
+//              dense blocks are repacked into panels, one per row leaf (of at most 42
+//              patches: a tree leaf or a part of one) and chunk of at most 24 KB,
+//              each a column-major (rows x columns) slab of one kind, dense or U.
+//   product    t = H v on v in the permuted order (every block's columns are a
+//              contiguous slice), two launches of k_hm_rows: the first forms
+//              z_b = V_b^T v_sigma of the low-rank blocks (one warp per two rank
+//              vectors) and, in CTAs between them, the dense chunks; the second
+//              the chunks of U.  A CTA copies its chunk's panel into shared memory
+//              with one bulk copy (two in the split form) and one thread per row
+//              multiplies it by the matching entries of v or z.  Inside an attempt
+//              the stage kernel (rk.cu) adds a leaf's chunks in order and writes the
+//              next v permuted; by itself, k_hm_gather permutes v before and
+//              k_hm_reduce adds up and writes K's row order after.  Every stored
+//              byte is read once per product and the summation order is fixed
+//              (deterministic).
 #include <algorithm>
 #include <cmath>
 #include <cstdint>

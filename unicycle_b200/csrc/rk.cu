@@ -3,7 +3,8 @@
 // One attempt of RKQSm (fortran/3d/src/ode45.f90:51-108) is six launches, one per
 // stage, captured once into a CUDA graph.  The launch of stage s
 //
-//   multiplies    t = K v_s (k_traction; hierarchical K: its product, then k_rhs_t)
+//   multiplies    t = K v_s (k_traction; hierarchical K: its two product launches
+//                 leave partial sums, which k_hm_stage adds up)
 //   and then, element by element as the row sums arrive,
 //   evaluates     k_s = f(y_s) (rate-state / Maxwell epilogue),
 //   and forms     s < 6: y_{s+1} = y + h sum_j b_sj k_j (BLAS-1 order of RKCKm) and
@@ -16,11 +17,14 @@
 // alternates between two buffers.  Stage 1 of the next attempt commits an accepted
 // candidate into y; after a rejection it only forms y_2 again for the new h.
 //
-// Every kernel reads the control block first and returns at once when the
-// integration is inactive, so the same graph serves accepted and rejected attempts
-// and many attempts can be queued without host round trips.  Separate kernels for
-// the stage state, the error norm and the decision (14 launches an attempt) cost
-// 67 us a step at N = 512, where each launch is latency alone.
+// Every kernel of this file looks at the control block and does nothing when the
+// integration is inactive (k_traction has asked for its first block of K by then), so
+// the same graph serves accepted and rejected attempts and many attempts can be
+// queued without host round trips.  The hierarchical product does not look: an idle
+// attempt moves its matrix six times all the same (tens of thousands of CTAs that
+// read one word: one reading each took 1.5 % of a live attempt at 7,200 triangles).
+// Separate kernels for the stage state, the error norm and the decision (14 launches
+// an attempt) cost 67 us a step at N = 512, where each launch is latency alone.
 //
 // The stage combinations, yout and yerr follow the reference's operation order
 // with explicit round-to-nearest multiplies and adds (no FMA contraction), so
