@@ -115,7 +115,7 @@ __device__ __forceinline__ void sv_log_factor(bool plus, double r, double d, dou
 // faces: 1e-14 of the stress 1 m and 1 um from the line, where the sum over the
 // corners had 1e-7 and 1e5.
 //
-// Per pair: 112 reciprocals, 32 square roots and about 5,300 other FP64
+// Per pair: 112 reciprocals, 32 square roots and about 5,200 other FP64
 // instructions, against 130,174 flops on duals of the 27 integrals.
 __device__ __forceinline__ void sv_strain(double x1, double x2, double x3, double q3, double L, double T, double W,
                                           double nu, double E[6][6])
